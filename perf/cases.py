@@ -375,9 +375,12 @@ def exact(case, seed):
     s = _inputs(case, seed)
     if kind in ('fq', 'fq_grad', 'grad_fq'):
         pos = torch.as_tensor(s['pos'])
+        # the gradient costs about ten times F(Q): minutes beyond this size
+        grad = kind != 'fq' and case['n'] ** 2 * s['tab'].shape[1] <= 3e10
+        if kind == 'grad_fq' and not grad:
+            return None
         fq, g = _exact_pairs(pos, s['sp'], s['tab'], s['qbin'], s['kb'],
-                             grad=kind != 'fq',
-                             need_f=kind == 'fq_grad')
+                             grad=grad, need_f=kind == 'fq_grad')
         return fq if kind == 'fq' else g if kind == 'grad_fq' else (fq, g)
     if kind == 'batch_fq':
         off = s['off']
