@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "../../include/pyiid_gb300.h"
+#include "adjoint_grid.cuh"
 #include "debye_kernels.cuh"
 #include "move_kernels.cuh"
 #include "spring_kernels.cuh"
@@ -37,6 +38,7 @@ namespace {
 constexpr int kVersion = 10000;  // 1.0.0
 constexpr int kJMax = kJMaxTiles;  // max J tiles per F(Q) work item
 constexpr int kAdjRS = 128;      // adjoint re-seed period (bins)
+constexpr size_t kAdjTabSmem = 108 * 1024;  // pair-force table of one key
 
 // ---------------------------------------------------------------- variants
 // Launch shapes of the two pair kernels; pyiid_tune selects one per context.
@@ -709,6 +711,9 @@ int set_attrs(pyiid_ctx *ctx) {
   CUDA_TRY(ctx, cudaFuncSetAttribute(adjoint_kernel<kAdjRS>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      160 * 1024));
+  CUDA_TRY(ctx, cudaFuncSetAttribute(adjoint_grid_kernel<true>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kAdjTabSmem));
   CUDA_TRY(ctx, cudaFuncSetAttribute(move_gram_kernel,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      2 * kGramCH * 3200 * (int)sizeof(float)));
@@ -722,6 +727,32 @@ int set_attrs(pyiid_ctx *ctx) {
                     umma::PersistShape<128, 3>::kSmem));
   ctx->attrs_set = true;
   return PYIID_OK;
+}
+
+GridScale grid_scale(double qstep, int m) {
+  GridScale g;
+  split_double((double)m * qstep / (2.0 * M_PI), g.hi, g.lo);
+  g.m = (float)m;
+  g.inv_m = 1.0f / (float)m;
+  return g;
+}
+
+// Whether the position gradient goes through the pair-force table
+// (adjoint_grid.cuh) or through the bins of each pair (adjoint_kernel,
+// adjoint_sym_kernel).  A table costs 4 n_bins cells x n_bins bins per key,
+// whatever the atoms; a pair costs about n_bins on the direct path and next
+// to nothing with the table.  Up to about 8 tables are built side by side in
+// the time of one; beyond that they take turns, and the pairs must pay for
+// them.  Whole evaluations, direct against table: 64 x 80 atoms at 330 bins
+// 165 / 169 us, 64 x 120 192 / 180, 64 x 300 536 / 321, 64 x 1,000
+// 4,048 / 1,859; 64 x 160 of two elements (192 keys) 265 / 275, 64 x 220
+// 365 / 313; one configuration of 10 atoms 79 / 77, of 300 102 / 100.  A few
+// pairs per key are not worth the launch (10 atoms of two elements 81 / 83).
+bool grid_adjoint(const Layout *L, int n_bins) {
+  double pairs = 0;
+  for (double p : L->pair_counts) pairs += p;
+  const double keys = (double)L->n_configs * L->n_spairs;
+  return pairs >= 100.0 * keys && pairs >= 24.0 * n_bins * (keys - 8.0);
 }
 
 // A pointer the device can write for the output `what`: device or managed
@@ -1457,6 +1488,41 @@ int pyiid_batch_potential_grad(pyiid_ctx *ctx, const float *positions,
   wvec_kernel<<<(nwarps * 32 + 255) / 256, 256, 0, ctx->stream>>>(
       T->d_T, cvec, n_bins, n_r, kmin, n_configs, w);
   LAUNCH_CHECK(ctx);
+  if (grid_adjoint(L, n_bins)) {
+    const int m = kAdjCellsPerBin * n_bins, n_cells = m / 2 + 1;
+    const size_t n_keys = (size_t)n_configs * L->n_spairs;
+    TRY(ensure(ctx, "b_wk", n_keys * n_bins * 2 * sizeof(float4), &p));
+    float4 *wk = static_cast<float4 *>(p);
+    TRY(ensure(ctx, "b_gtab", n_keys * n_cells * 2 * sizeof(float4), &p));
+    float4 *gtab = static_cast<float4 *>(p);
+    adjoint_grid_weights_kernel<<<256, 256, 0, ctx->stream>>>(
+        w, d_na, d_ftab, L->d_spair, L->n_spairs, n_bins, kmin, n_configs,
+        (float)(2.0 * M_PI / m), wk);
+    LAUNCH_CHECK(ctx);
+    // keys in grid.y: at most 65,535 per launch
+    for (size_t key0 = 0; key0 < n_keys; key0 += 32768) {
+      const dim3 g((n_cells + 31) / 32,
+                   (unsigned)std::min<size_t>(32768, n_keys - key0));
+      adjoint_grid_table_kernel<<<g, kAdjBlock, 0, ctx->stream>>>(
+          wk + key0 * n_bins * 2, n_bins, kmin, m, 1.0f / (float)m,
+          gtab + key0 * n_cells * 2);
+      LAUNCH_CHECK(ctx);
+    }
+    const GridScale gs = grid_scale(qstep, m);
+    const size_t smem = (size_t)n_cells * 2 * sizeof(float4);
+    if (smem <= kAdjTabSmem)
+      adjoint_grid_kernel<true>
+          <<<(unsigned)L->tiles.size(), kAdjBlock, smem, ctx->stream>>>(
+              positions, L->d_perm, L->d_tiles, L->d_cfg_tiles, gs, n_cells,
+              gtab, L->n_spairs, grad);
+    else
+      adjoint_grid_kernel<false>
+          <<<(unsigned)L->tiles.size(), kAdjBlock, 0, ctx->stream>>>(
+              positions, L->d_perm, L->d_tiles, L->d_cfg_tiles, gs, n_cells,
+              gtab, L->n_spairs, grad);
+    LAUNCH_CHECK(ctx);
+    return PYIID_OK;
+  }
   const int kb0 = kmin & ~1;
   // table length: bins [kb0, n_bins) rounded up to a multiple of 4 (two
   // packed steps); the kernel runs full re-seed blocks, then the remainder

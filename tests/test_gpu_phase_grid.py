@@ -1,0 +1,103 @@
+"""GPU parity of the phase-grid kernels (phase_grid.cuh) against the FP64
+oracle, at the edges of their tiles, grids and dispatch rules.
+
+Tolerances are the suite's (norm-wise relative): F(Q) and potentials 1e-5,
+gradients 1e-4.
+"""
+import numpy as np
+import pytest
+
+from oracle import debye_np as O
+from pyiid_gb300.scatter_factors import form_factor_array
+from pyiid_gb300 import structures as S
+
+pytestmark = pytest.mark.gpu
+
+TOL_F = 1e-5
+TOL_G = 1e-4
+
+
+def rel(a, b):
+    a = np.asarray(a, dtype=np.float64)
+    b = np.asarray(b, dtype=np.float64)
+    nb = np.linalg.norm(b)
+    return np.linalg.norm(a - b) / (nb if nb > 0 else 1.0)
+
+
+@pytest.fixture(scope='module')
+def D():
+    from pyiid_gb300 import debye
+    return debye
+
+
+def cluster(n, seed, species=1, shift=0.0):
+    rng = np.random.default_rng(seed)
+    pos = S.displaced(S.fcc_nearest(4.08, n), 0.05, seed) + np.float32(shift)
+    nums = rng.choice([46, 78, 79][:species], n) if species > 1 \
+        else np.full(n, 79)
+    return pos[rng.permutation(n)], nums
+
+
+def tables(numbers, qb, nb):
+    uniq, sp = np.unique(numbers, return_inverse=True)
+    tab = np.stack([form_factor_array(z, np.arange(nb) * qb) for z in uniq])
+    return sp.reshape(-1).astype(np.int32), tab.astype(np.float32)
+
+
+# tile edges (31, 32, 33, 65 atoms); one to three elements; a period of Q
+# shorter than the cluster (rmax 3: distances beyond half a period fold);
+# qmin above some bins; a table too large for shared memory (rmax 110: 887
+# bins); a cluster away from the origin; chi^2
+@pytest.mark.parametrize('sizes,species,exp,shift,kind', [
+    ([31], 1, {}, 0.0, 'rw'),
+    ([32], 1, {'rmax': 20.0}, 0.0, 'chi_sq'),
+    ([33, 65], 2, {'rmax': 17.3, 'qmin': 0.9}, 0.0, 'rw'),
+    ([97], 3, {'rmax': 3.0}, 0.0, 'rw'),
+    ([64], 2, {'rmax': 110.0, 'rstep': 0.05}, 0.0, 'rw'),
+    ([120], 1, {'rmax': 12.0, 'qmax': 7.0}, 150.0, 'rw'),
+    ([300, 1, 0, 280], 2, {'rmax': 20.0}, -60.0, 'chi_sq'),
+])
+def test_pair_force_table_matches_oracle(D, sizes, species, exp, shift, kind):
+    import torch
+    e = O.update_experiment(dict({'rstep': 0.02}, **exp))
+    qb, rg = O.pdf_qbin(e), O.r_grid(e)
+    nb = int(np.floor(e['qmax'] / qb))
+    parts = [cluster(n, 7 + n, species, shift) for n in sizes]
+    pos = np.concatenate([p for p, _ in parts]).astype(np.float32)
+    sp, tab = tables(np.concatenate([z for _, z in parts]), qb, nb)
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    ref = S.fcc_nearest(4.0, 50).astype(np.float32)
+    gobs = O.pdf_fft(O.fq(ref, np.repeat(tab[:1], 50, 0), qb), e['rstep'], qb,
+                     rg, e['qmin'])
+    out = D.batch_potential_grad(pos, sp, off, tab, qb, e['rstep'], rg,
+                                 e['qmin'], torch.as_tensor(gobs), kind)
+    g = out['grad'].cpu().numpy()
+    for i, n in enumerate(sizes):
+        if n < 2:
+            continue
+        a, b = off[i], off[i + 1]
+        val, tg = O.true_grad_potential(pos[a:b], tab[sp[a:b]], e, gobs, kind)
+        assert abs(out['energy'][i, 0].item() - val) <= TOL_F * abs(val)
+        assert rel(g[a:b], tg) <= TOL_G, (i, rel(g[a:b], tg))
+
+
+def test_pair_force_table_close_and_coincident_pairs(D):
+    """Pairs nearer than the split coordinates resolve (0.1 A) take the
+    general distance; coincident atoms give NaN rows, the others' stay."""
+    import torch
+    e = O.update_experiment({'rmax': 20.0, 'rstep': 0.02})
+    qb, rg = O.pdf_qbin(e), O.r_grid(e)
+    nb = int(np.floor(e['qmax'] / qb))
+    pos, nums = cluster(80, 5)
+    pos[11] = pos[40] + np.float32([0.03, -0.02, 0.01])
+    sp, tab = tables(nums, qb, nb)
+    gobs = O.pdf_fft(O.fq(S.fcc_nearest(4.0, 50), np.repeat(tab, 50, 0), qb),
+                     e['rstep'], qb, rg, e['qmin'])
+    args = (sp, np.array([0, 80]), tab, qb, e['rstep'], rg, e['qmin'],
+            torch.as_tensor(gobs))
+    g = D.batch_potential_grad(pos, *args)['grad'].cpu().numpy()
+    _, tg = O.true_grad_potential(pos, tab[sp], e, gobs)
+    assert rel(g, tg) <= TOL_G
+    pos[11] = pos[40]
+    g = D.batch_potential_grad(pos, *args)['grad'].cpu().numpy()
+    assert np.all(np.isnan(g[[11, 40]]))
