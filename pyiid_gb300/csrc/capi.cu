@@ -26,6 +26,7 @@
 #include "../../include/pyiid_gb300.h"
 #include "adjoint_grid.cuh"
 #include "debye_kernels.cuh"
+#include "fq_grid.cuh"
 #include "move_kernels.cuh"
 #include "spring_kernels.cuh"
 #include "transform_kernels.cuh"
@@ -38,6 +39,13 @@ namespace {
 constexpr int kVersion = 10000;  // 1.0.0
 constexpr int kJMax = kJMaxTiles;  // max J tiles per F(Q) work item
 constexpr int kAdjRS = 128;      // adjoint re-seed period (bins)
+// one warp's histogram of half a period fits the spreading kernel's memory
+constexpr int kFqGridMaxBins = 2816;
+static_assert(kSpreadStage + 4 * kSpreadSlots *
+                      grid_words(kFqCellsPerBin * kFqGridMaxBins / 2 + 2) <=
+                  kSpreadSmem,
+              "");
+
 constexpr size_t kAdjTabSmem = 108 * 1024;  // pair-force table of one key
 
 // ---------------------------------------------------------------- variants
@@ -186,6 +194,23 @@ struct DevBuf {
   size_t bytes = 0;
 };
 
+// Work of the F(Q) grid path for one layout and bin count: the rows of
+// columns of the configurations that take it, and what is left to the direct
+// kernels.
+struct FqGridWork {
+  int n_bins = 0;
+  int n_segs = 0, total = 0, n_keys = 0, n_cfgs = 0;  // n_cfgs 0: no work
+  int max_cols = 0;  // most columns of one key
+  int n_direct = 0;  // work items of the other configurations
+  GridSeg *d_segs = nullptr;
+  int *d_seg_begin = nullptr;
+  int2 *d_key_cols = nullptr;
+  int *d_key_spair = nullptr;
+  int4 *d_cfg_keys = nullptr;
+  int *d_direct_order = nullptr;
+  unsigned char *d_skip = nullptr;
+};
+
 struct Layout {
   uint64_t key = 0;
   int total = 0, n_configs = 0, n_species = 0, n_spairs = 0;
@@ -223,6 +248,15 @@ struct Layout {
   int *d_item_order = nullptr;
   int *d_key_item_begin = nullptr;
   int2 *d_spair = nullptr;
+  std::vector<std::unique_ptr<FqGridWork>> fq_grid;  // by n_bins, newest first
+};
+
+// Phase grid of n_bins bins (independent of their step): the window's
+// polynomials and what its spectrum takes off each bin.
+struct PhaseGrid {
+  int n_bins = 0, m = 0;
+  float *d_taps = nullptr;      // [kTaps][kTapCoef]
+  double *d_inv_phi = nullptr;  // [n_bins]
 };
 
 struct TMatrix {
@@ -267,6 +301,7 @@ struct pyiid_ctx {
   std::vector<std::unique_ptr<Layout>> layouts;  // small LRU (front = newest)
   std::vector<std::unique_ptr<TMatrix>> tmats;
   std::vector<std::unique_ptr<NaTable>> nas;
+  std::vector<std::unique_ptr<PhaseGrid>> grids;
   uint64_t ftab_key = 0;
   int ftab_species = 0, ftab_bins = 0;
   bool attrs_set = false;
@@ -355,7 +390,18 @@ int upload(pyiid_ctx *ctx, T **dst, const std::vector<T> &src) {
   return PYIID_OK;
 }
 
+void free_fq_grid(FqGridWork *W) {
+  cudaFree(W->d_segs);
+  cudaFree(W->d_seg_begin);
+  cudaFree(W->d_key_cols);
+  cudaFree(W->d_key_spair);
+  cudaFree(W->d_cfg_keys);
+  cudaFree(W->d_direct_order);
+  cudaFree(W->d_skip);
+}
+
 void free_layout(Layout *L) {
+  for (auto &W : L->fq_grid) free_fq_grid(W.get());
   cudaFree(L->d_perm);
   cudaFree(L->d_tiles);
   cudaFree(L->d_cfg_tiles);
@@ -711,6 +757,15 @@ int set_attrs(pyiid_ctx *ctx) {
   CUDA_TRY(ctx, cudaFuncSetAttribute(adjoint_kernel<kAdjRS>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      160 * 1024));
+  CUDA_TRY(ctx, cudaFuncSetAttribute(
+                    fq_spread_kernel,
+                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                    kSpreadSmem));
+  CUDA_TRY(ctx, cudaFuncSetAttribute(
+                    fq_grid_finish_kernel,
+                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                    (int)(fq_dft_floats(kFqCellsPerBin * kFqGridMaxBins) *
+                          sizeof(float))));
   CUDA_TRY(ctx, cudaFuncSetAttribute(adjoint_grid_kernel<true>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kAdjTabSmem));
@@ -735,6 +790,221 @@ GridScale grid_scale(double qstep, int m) {
   g.m = (float)m;
   g.inv_m = 1.0f / (float)m;
   return g;
+}
+
+// ------------------------------------------------------ spreading window
+// Kaiser-Bessel window of kTaps cells, I0(beta sqrt(1 - (2 x / kTaps)^2)),
+// as one polynomial of degree kTapCoef - 1 per tap in t = u - floor(u) - 1/2
+// (Chebyshev interpolation: 2e-8 of the peak).  beta = 0.98 pi kTaps
+// (1 - 1/(2 sigma)) for sigma = M / (2 n_bins) is where the spectrum left
+// out of the bins is smallest, found by scanning beta.
+void window_taps(double sigma, float *taps) {
+  const double beta = 0.98 * M_PI * kTaps * (1.0 - 1.0 / (2.0 * sigma));
+  constexpr int N = kTapCoef;
+  for (int p = 0; p < kTaps; ++p) {
+    double y[N], x[N];
+    for (int i = 0; i < N; ++i) {
+      x[i] = std::cos(M_PI * (i + 0.5) / N) / 2;
+      const double d = 2.0 * (p - (kTaps - 1) / 2.0 - x[i]) / kTaps;
+      y[i] = std::cyl_bessel_i(0.0, beta * std::sqrt(std::max(0.0, 1 - d * d))) /
+             std::cyl_bessel_i(0.0, beta);
+    }
+    // Newton's divided differences, then expanded in powers of t
+    for (int j = 1; j < N; ++j)
+      for (int i = N - 1; i >= j; --i) y[i] = (y[i] - y[i - 1]) / (x[i] - x[i - j]);
+    double c[N] = {y[N - 1]};
+    for (int i = N - 2; i >= 0; --i) {
+      for (int j = N - 1; j >= 1; --j) c[j] = c[j - 1] - x[i] * c[j];
+      c[0] = y[i] - x[i] * c[0];
+    }
+    for (int j = 0; j < N; ++j) taps[p * N + j] = (float)c[j];
+  }
+}
+
+// Spectrum of the window as the kernels evaluate it (the float polynomials,
+// integrated exactly enough by 16 Gauss points per tap): phi_k = integral
+// phi(x) cos(theta_k x) dx, theta_k = 2 pi k / m, and dphi_k = d phi/d theta.
+void window_spectrum(const float *taps, int m, int n_bins, double *phi,
+                     double *dphi) {
+  constexpr int G = 16;
+  double gx[G], gw[G];
+  for (int i = 0; i < G; ++i) {  // Gauss-Legendre nodes by Newton
+    double z = std::cos(M_PI * (i + 0.75) / (G + 0.5)), dp = 0;
+    for (int it = 0; it < 60; ++it) {
+      double p0 = 1, p1 = z;
+      for (int n = 2; n <= G; ++n) {
+        const double p2 = ((2 * n - 1) * z * p1 - (n - 1) * p0) / n;
+        p0 = p1;
+        p1 = p2;
+      }
+      dp = G * (z * p1 - p0) / (z * z - 1);
+      const double dz = p1 / dp;
+      z -= dz;
+      if (std::fabs(dz) < 1e-15) break;
+    }
+    gx[i] = z / 2;
+    gw[i] = 1.0 / ((1 - z * z) * dp * dp);
+  }
+  std::vector<double> xs, ws;
+  for (int p = 0; p < kTaps; ++p)
+    for (int i = 0; i < G; ++i) {
+      double f = 0;
+      for (int j = kTapCoef - 1; j >= 0; --j)
+        f = f * gx[i] + (double)taps[p * kTapCoef + j];
+      xs.push_back(p - (kTaps - 1) / 2.0 - gx[i]);
+      ws.push_back(f * gw[i]);
+    }
+  for (int k = 0; k < n_bins; ++k) {
+    const double th = 2.0 * M_PI * k / m;
+    double s = 0, d = 0;
+    for (size_t i = 0; i < xs.size(); ++i) {
+      s += ws[i] * std::cos(th * xs[i]);
+      d -= ws[i] * xs[i] * std::sin(th * xs[i]);
+    }
+    phi[k] = s;
+    if (dphi) dphi[k] = d;
+  }
+}
+
+int get_fq_phase_grid(pyiid_ctx *ctx, int n_bins, PhaseGrid **out) {
+  for (auto &G : ctx->grids)
+    if (G->n_bins == n_bins) {
+      *out = G.get();
+      return PYIID_OK;
+    }
+  auto G = std::make_unique<PhaseGrid>();
+  G->n_bins = n_bins;
+  G->m = (kFqCellsPerBin * n_bins + 3) & ~3;
+  std::vector<float> taps(kTaps * kTapCoef);
+  window_taps((double)G->m / (2.0 * n_bins), taps.data());
+  std::vector<double> phi(n_bins);
+  window_spectrum(taps.data(), G->m, n_bins, phi.data(), nullptr);
+  for (double &v : phi) v = 1.0 / v;
+  TRY(upload(ctx, &G->d_taps, taps));
+  TRY(upload(ctx, &G->d_inv_phi, phi));
+  ctx->grids.insert(ctx->grids.begin(), std::move(G));
+  while (ctx->grids.size() > 16) {
+    cudaFree(ctx->grids.back()->d_taps);
+    cudaFree(ctx->grids.back()->d_inv_phi);
+    ctx->grids.pop_back();
+  }
+  *out = ctx->grids[0].get();
+  return PYIID_OK;
+}
+
+// Which configurations of a layout take the F(Q) grid path (empty: none).
+// Times in us of both paths, fitted to single configurations of 60 to 2,000
+// atoms and batches of 16 to 256 x 40 to 320 atoms, each of one to three
+// elements at 250, 500 and 1,500 bins: the grid path spends four launches,
+// and on each (configuration, species pair) a transform of 2.8e-4 n_bins,
+// but 1.5e-5 per pair where the direct kernels spend 1.3e-7 n_bins (2e-7
+// while the pairs do not fill the GPU).  A configuration takes it if its own
+// pairs pay for its transforms, and all of those do if together they pay for
+// the launches.  Either side of the line, direct / grid: 300 atoms at 500
+// bins 22.3 / 23.5, 420 26.6 / 26.0, 1,000 91.6 / 44.1; 420 of three elements
+// at 1,500 bins 49 / 67, 600 80 / 69; 64 x 80 of two elements at 500 bins
+// 28 / 54, 64 x 160 70 / 61, 256 x 320 859 / 234.
+std::vector<int> fq_grid_configs(const Layout *L, int n_bins) {
+  std::vector<int> on;
+  if (n_bins < 64 || n_bins > kFqGridMaxBins) return on;
+  const double k = n_bins;
+  double pairs = 0, keys = 0, most_keys = 0;
+  for (int c = 0; c < L->n_configs; ++c) {
+    double p = 0, n = 0;
+    for (int s = 0; s < L->n_spairs; ++s) {
+      const double ps = L->pair_counts[(size_t)c * L->n_spairs + s];
+      p += ps;
+      n += ps > 0;
+    }
+    if (p * (1.3e-7 * k - 1.5e-5) <= 2.8e-4 * k * n) continue;
+    on.push_back(c);
+    pairs += p;
+    keys += n;
+    most_keys = std::max(most_keys, n);
+  }
+  const double pk = pairs * k;
+  const double direct =
+      10 + k / 60 + (pk < 3e8 ? 2e-7 * pk : 18 + 1.4e-7 * pk);
+  const double grid = 19.5 + most_keys * (2 + k / 250) + 2.8e-4 * k * keys +
+                      1.5e-5 * pairs;
+  if (grid >= direct) on.clear();
+  return on;
+}
+
+// The grid path's share of a layout (n_cfgs == 0: none of it).
+int get_fq_grid_work(pyiid_ctx *ctx, Layout *L, int n_bins,
+                     FqGridWork **out) {
+  for (auto &W : L->fq_grid)
+    if (W->n_bins == n_bins) {
+      *out = W.get();
+      return PYIID_OK;
+    }
+  auto W = std::make_unique<FqGridWork>();
+  W->n_bins = n_bins;
+  std::vector<GridSeg> segs;
+  std::vector<int> begin, key_spair, direct;
+  std::vector<int4> cfg_keys;
+  std::vector<int2> cols;  // columns [x, y) of each key
+  std::vector<unsigned char> skip(L->n_configs, 0);
+  long long total = 0;
+  for (int c : fq_grid_configs(L, n_bins)) {
+    skip[c] = 1;
+    const int first_key = (int)key_spair.size();
+    const int t0 = L->cfg_tiles[c].x, t1 = L->cfg_tiles[c].y;
+    // start of each species' atoms in the sorted order
+    std::vector<int> start(L->n_species + 1, -1), count(L->n_species, 0);
+    for (int t = t0; t < t1; ++t) {
+      const int4 ti = L->tiles[t];
+      if (start[ti.w] < 0) start[ti.w] = ti.x;
+      count[ti.w] += ti.y;
+    }
+    for (int sp = 0; sp < L->n_spairs; ++sp) {
+      if (L->pair_counts[(size_t)c * L->n_spairs + sp] == 0) continue;
+      const int sa = L->spair_species[sp].x, sb = L->spair_species[sp].y;
+      const int x = (int)total;
+      for (int t = t0; t < t1; ++t) {
+        const int4 ti = L->tiles[t];
+        if (ti.w != sa) continue;
+        // b < a only: the tile's last atom sees ti.x + ti.y - 1 of them
+        const int nb = sa == sb ? ti.x + ti.y - 1 - start[sb] : count[sb];
+        if (nb <= 0) continue;
+        segs.push_back(GridSeg{ti.x, ti.y, start[sb], (int)key_spair.size()});
+        begin.push_back((int)total);
+        total += nb;
+      }
+      cols.push_back(make_int2(x, (int)total));
+      key_spair.push_back(sp);
+    }
+    cfg_keys.push_back(
+        make_int4(c, first_key, (int)key_spair.size() - first_key, 0));
+  }
+  begin.push_back((int)total);
+  W->n_segs = (int)segs.size();
+  W->total = (int)total;
+  W->n_keys = (int)key_spair.size();
+  // (grid.y of the launches; columns are counted in int)
+  if (W->n_keys <= 65535 && total < INT32_MAX / 2)
+    W->n_cfgs = (int)cfg_keys.size();
+  if (W->n_cfgs > 0) {
+    for (const int2 &k : cols) W->max_cols = std::max(W->max_cols, k.y - k.x);
+    for (int i : L->item_order)
+      if (!skip[L->items[i].w / L->n_spairs]) direct.push_back(i);
+    W->n_direct = (int)direct.size();
+    TRY(upload(ctx, &W->d_segs, segs));
+    TRY(upload(ctx, &W->d_seg_begin, begin));
+    TRY(upload(ctx, &W->d_key_cols, cols));
+    TRY(upload(ctx, &W->d_key_spair, key_spair));
+    TRY(upload(ctx, &W->d_cfg_keys, cfg_keys));
+    TRY(upload(ctx, &W->d_direct_order, direct));
+    TRY(upload(ctx, &W->d_skip, skip));
+  }
+  L->fq_grid.insert(L->fq_grid.begin(), std::move(W));
+  while (L->fq_grid.size() > 4) {
+    free_fq_grid(L->fq_grid.back().get());
+    L->fq_grid.pop_back();
+  }
+  *out = L->fq_grid[0].get();
+  return PYIID_OK;
 }
 
 // Whether the position gradient goes through the pair-force table
@@ -844,15 +1114,77 @@ int check_common(pyiid_ctx *ctx, int n_configs, const int32_t *offsets,
   return PYIID_OK;
 }
 
+// F(Q) of the configurations of W (fq_grid.cuh): spread, sum, transform.
+int run_fq_grid(pyiid_ctx *ctx, const Layout *L, const FqGridWork *W,
+                const float *positions, const float *d_ftab,
+                const double *d_na, int n_bins, double qbin, int kb_out,
+                float *fq, double *fq_raw) {
+  PhaseGrid *G;
+  TRY(get_fq_phase_grid(ctx, n_bins, &G));
+  const int m = G->m, quarter = m / 4;
+  const int row_words = grid_words(m / 2), n_ctas = ctx->n_sms;
+  void *p;
+  TRY(ensure(ctx, "fqg_rows",
+             ((size_t)kSpreadWarps * n_ctas + W->n_keys) * row_words *
+                 sizeof(float),
+             &p));
+  float *rows = static_cast<float *>(p);
+  TRY(ensure(ctx, "fqg_sum",
+             (size_t)W->n_keys * (2 * (quarter + 1) + 8) * sizeof(float), &p));
+  float *hsum = static_cast<float *>(p);
+  TRY(ensure(ctx, "fqg_ext", (size_t)W->n_cfgs * sizeof(int), &p));
+  int *ext = static_cast<int *>(p);
+  const GridScale gs = grid_scale(qbin, m);
+  grid_extent_kernel<<<W->n_cfgs, 256, 0, ctx->stream>>>(
+      positions, L->d_offsets, W->d_cfg_keys, gs.hi, m / 2, ext);
+  LAUNCH_CHECK(ctx);
+  fq_spread_kernel<<<n_ctas, 32 * kSpreadWarps, kSpreadSmem, ctx->stream>>>(
+      positions, L->d_perm, W->d_segs, W->d_seg_begin, W->n_segs, W->total,
+      ext, W->n_cfgs, gs, (float)(kNearPhase / (n_bins * qbin)),
+      (float)(n_bins * qbin), G->d_taps, row_words, rows);
+  LAUNCH_CHECK(ctx);
+  // a share of about eight slots per thread row, at most 32 rows
+  const double most =
+      (double)W->max_cols / W->total * kSpreadWarps * n_ctas + 2;
+  const int ny = std::max(1, std::min(32, (int)(most / 8)));
+  fq_grid_reduce_kernel<<<dim3((quarter + kNearTerms) / 32 + 1, W->n_keys),
+                          dim3(32, ny), 4 * ny * 32 * sizeof(float),
+                          ctx->stream>>>(rows, W->d_key_cols, ext, W->n_cfgs,
+                                         n_ctas, W->total, m, row_words, hsum);
+  LAUNCH_CHECK(ctx);
+  fq_grid_finish_kernel<<<dim3((n_bins + 31) / 32, W->n_cfgs),
+                          32 * kFqDftWarps, fq_dft_floats(m) * sizeof(float),
+                          ctx->stream>>>(
+      hsum, W->d_cfg_keys, W->d_key_spair, L->d_spair, d_ftab, d_na,
+      G->d_inv_phi, m, 1.0f / (float)m, n_bins, kb_out, qbin,
+      1.0f / (float)n_bins, fq, fq_raw);
+  LAUNCH_CHECK(ctx);
+  return PYIID_OK;
+}
+
 // Pair sums + finishing: fq[c][k] for k in [k_begin, n_bins) (zero below).
-int run_fq(pyiid_ctx *ctx, const Layout *L, const float *positions,
+int run_fq(pyiid_ctx *ctx, Layout *L, const float *positions,
            const float *d_ftab, const double *d_na, int n_bins, double qbin,
            int k_begin, float *fq, double *fq_raw) {
   float dq_hi, dq_lo;
   split_double(qbin, dq_hi, dq_lo);
   const int kb0 = std::min(k_begin, n_bins) & ~1;
-  const int n_items = (int)L->items.size();
+  int n_items = (int)L->items.size();
+  const int *order = L->d_item_order;
+  const unsigned char *skip = nullptr;
   double *partial = nullptr;
+  if (n_items > 0 && kb0 < n_bins) {
+    FqGridWork *W;
+    TRY(get_fq_grid_work(ctx, L, n_bins, &W));
+    if (W->n_cfgs > 0) {
+      TRY(run_fq_grid(ctx, L, W, positions, d_ftab, d_na, n_bins, qbin,
+                      std::min(k_begin, n_bins), fq, fq_raw));
+      if (W->n_cfgs == L->n_configs) return PYIID_OK;
+      n_items = W->n_direct;
+      order = W->d_direct_order;
+      skip = W->d_skip;
+    }
+  }
   if (n_items > 0 && kb0 < n_bins) {
     const FqEntry &E = kFqTable[ctx->fq_variant];
     const int Lb = E.v.L;
@@ -864,7 +1196,8 @@ int run_fq(pyiid_ctx *ctx, const Layout *L, const float *positions,
     const int n_chunks = (chunks_total + n_cb - 1) / n_cb;
     const int n_groups = kBlock / n_chunks;
     void *p;
-    TRY(ensure(ctx, "fq_partial", (size_t)n_items * n_bins * sizeof(double), &p));
+    TRY(ensure(ctx, "fq_partial",
+               L->items.size() * (size_t)n_bins * sizeof(double), &p));
     partial = static_cast<double *>(p);
     const size_t smem = fq_smem(E.v, n_chunks);
     if (E.kp) {
@@ -880,14 +1213,14 @@ int run_fq(pyiid_ctx *ctx, const Layout *L, const float *positions,
       const int grid = std::max(
           1, std::min(n_units, std::max(per_sm, 1) * ctx->n_sms));
       E.kp<<<grid, kBlock, smem, ctx->stream>>>(
-          positions, L->d_perm, L->d_tiles, L->d_items, L->d_item_order,
-          dq_hi, dq_lo, kb0, n_chunks, n_groups, n_bins, n_cb, n_units,
+          positions, L->d_perm, L->d_tiles, L->d_items, order, dq_hi,
+          dq_lo, kb0, n_chunks, n_groups, n_bins, n_cb, n_units,
           static_cast<int *>(ctr), partial);
     } else {
       dim3 grid(n_items, n_cb);
       E.k<<<grid, kBlock, smem, ctx->stream>>>(
-          positions, L->d_perm, L->d_tiles, L->d_items, L->d_item_order,
-          dq_hi, dq_lo, kb0, n_chunks, n_groups, n_bins, partial);
+          positions, L->d_perm, L->d_tiles, L->d_items, order, dq_hi, dq_lo,
+          kb0, n_chunks, n_groups, n_bins, partial);
     }
     LAUNCH_CHECK(ctx);
   }
@@ -895,7 +1228,7 @@ int run_fq(pyiid_ctx *ctx, const Layout *L, const float *positions,
   const int kb_out = (n_items > 0) ? std::min(k_begin, n_bins) : n_bins;
   fq_finish_kernel<<<g2, 128, 0, ctx->stream>>>(
       partial, L->d_key_item_begin, d_ftab, L->d_spair, d_na, L->n_spairs,
-      n_bins, kb_out, fq, fq_raw);
+      n_bins, kb_out, fq, fq_raw, skip);
   LAUNCH_CHECK(ctx);
   return PYIID_OK;
 }
@@ -977,6 +1310,10 @@ int pyiid_destroy(pyiid_ctx *ctx) {
   for (auto &L : ctx->layouts) free_layout(L.get());
   for (auto &T : ctx->tmats) free_tmatrix(T.get());
   for (auto &N : ctx->nas) cudaFree(N->d_na);
+  for (auto &G : ctx->grids) {
+    cudaFree(G->d_taps);
+    cudaFree(G->d_inv_phi);
+  }
   cudaFree(ctx->d_status);
   delete ctx;
   return PYIID_OK;
@@ -2203,7 +2540,8 @@ extern "C" int pyiid_fq_noalloc(pyiid_ctx *ctx, const float *positions,
   dim3 g2((n_bins + 127) / 128, 1);
   const int kb_out = (n_items > 0) ? std::min(k_begin, n_bins) : n_bins;
   fq_finish_kernel<<<g2, 128, 0, st>>>(d_part, d_keys, d_ftab, d_spair, d_na,
-                                       n_spairs, n_bins, kb_out, fq, nullptr);
+                                       n_spairs, n_bins, kb_out, fq, nullptr,
+                                       nullptr);
   LAUNCH_CHECK(ctx);
   // the host vectors are released on return: wait for the copies only
   CUDA_TRY(ctx, cudaStreamSynchronize(st));

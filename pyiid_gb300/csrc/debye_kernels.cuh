@@ -237,17 +237,19 @@ __device__ __forceinline__ float fq_value(double s, double na) {
 // as wrap_fq does (cpu_wrappers/flat_multi_cpu_wrap.py:44-60: FP64 sum of the
 // FP32 pair terms, na = N mean_{i>j} f_i f_j, factor 2, nan_to_num).
 // na is precomputed per (config, bin) on the host in FP64 (it depends only on
-// species counts and form factors).  Configurations with < 2 atoms give 0.
+// species counts and form factors).  Configurations with < 2 atoms give 0;
+// those marked in skip (nullptr: none) are left to another kernel.
 __global__ void fq_finish_kernel(const double *__restrict__ partial,
                                  const int *__restrict__ key_item_begin,
                                  const float *__restrict__ ftab,
                                  const int2 *__restrict__ spair_species,
                                  const double *__restrict__ na, int n_spairs,
                                  int n_bins, int kb_out, float *__restrict__ fq,
-                                 double *__restrict__ fq_raw) {
+                                 double *__restrict__ fq_raw,
+                                 const unsigned char *__restrict__ skip) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
-  if (k >= n_bins) return;
+  if (k >= n_bins || (skip && skip[b])) return;
   float outv = 0.f;
   double sraw = 0.0;
   if (k >= kb_out) {

@@ -1,0 +1,505 @@
+// fq_grid.cuh -- F(Q) of a configuration by spreading its pairs on a phase
+// grid.
+//
+// sum over pairs of sin(Q_k r)/r (cpu_flat.py:79-114, gpu_flat.py:73-112 of
+// pyiid/experiments/elasticscatter/kernels) is a sine transform of weights
+// 1/r at the points u = r M dq / (2 pi) of a period of M cells.  Every pair
+// is spread on its eight nearest cells with a Kaiser-Bessel window phi,
+//   H_j = sum_pairs phi(j - u) / r,
+// and the sums follow from one transform per (configuration, species pair),
+//   D_k = (1 / phihat_k) sum_j H_j sin(2 pi k j / M),
+// the usual non-uniform transform (Kaiser-Bessel gridding; Fessler and
+// Sutton, IEEE Trans. Signal Process. 51, 2003).  What is left out is the
+// window's spectrum beyond the period: 2e-8 rms of a term at M = 5 n_bins,
+// against 2e-7 for the seeds and the recurrence of the direct kernels.
+#pragma once
+
+#include "debye_kernels.cuh"
+#include "phase_grid.cuh"
+
+namespace pyiid {
+
+constexpr int kTaps = 8;        // cells a pair is spread on
+constexpr int kTapCoef = 8;     // polynomial coefficients of a tap
+constexpr int kFqCellsPerBin = 5;
+constexpr int kNearTerms = 5;   // power sums of pairs at tiny distances
+constexpr float kNearPhase = 0.6f;  // ... with Q_max r below this
+
+// A histogram in memory: 8 words of power sums, then cells -3 .. used + 4.
+constexpr int kGridCell0 = 8 + 3;  // word of cell 0
+__host__ __device__ constexpr int grid_words(int used) {
+  return kGridCell0 + used + 5;
+}
+
+// One row of work: tile I (atoms [a0, a0 + na) in sorted order) against the
+// atoms [b0, b0 + nb) of one species; only b < a counts.  key: rank of the
+// (configuration, species pair) among those on the grid.
+struct GridSeg {
+  int a0, na, b0, key;
+};
+
+// Cells that the distances of a configuration can reach: ext[c] = the cell
+// of twice the largest distance from the centre of the atoms' box (at most
+// M/2, where the period folds).  One CTA per configuration.
+__global__ void __launch_bounds__(256)
+    grid_extent_kernel(const float *__restrict__ pos,
+                       const int *__restrict__ offsets,
+                       const int4 *__restrict__ cfg_keys, float scale, int half,
+                       int *__restrict__ ext) {
+  __shared__ float red[8][6];
+  __shared__ float mx[8];
+  const int c = cfg_keys[blockIdx.x].x;
+  const int i0 = offsets[c], i1 = offsets[c + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float lo[3], hi[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) lo[d] = 3e38f, hi[d] = -3e38f;
+  for (int i = i0 + threadIdx.x; i < i1; i += 256) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const float x = pos[3 * (size_t)i + d];
+      lo[d] = fminf(lo[d], x);
+      hi[d] = fmaxf(hi[d], x);
+    }
+  }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    for (int o = 16; o > 0; o >>= 1) {
+      lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+      hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+    }
+    if (lane == 0) red[warp][d] = lo[d], red[warp][3 + d] = hi[d];
+  }
+  __syncthreads();
+  float mid[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    float l = red[0][d], h = red[0][3 + d];
+    for (int w = 1; w < 8; ++w)
+      l = fminf(l, red[w][d]), h = fmaxf(h, red[w][3 + d]);
+    mid[d] = 0.5f * l + 0.5f * h;
+  }
+  float r2 = 0.f;
+  for (int i = i0 + threadIdx.x; i < i1; i += 256) {
+    const float x = pos[3 * (size_t)i] - mid[0];
+    const float y = pos[3 * (size_t)i + 1] - mid[1];
+    const float z = pos[3 * (size_t)i + 2] - mid[2];
+    r2 = fmaxf(r2, fmaf(x, x, fmaf(y, y, z * z)));
+  }
+  for (int o = 16; o > 0; o >>= 1)
+    r2 = fmaxf(r2, __shfl_xor_sync(0xffffffffu, r2, o));
+  if (lane == 0) mx[warp] = r2;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) r2 = fmaxf(r2, mx[w]);
+    // a millionth more for the roundings here; cells are floor(u)
+    const float u = 2.000002f * sqrtf(r2) * scale + 2.0f;
+    const bool fin = fabsf(mid[0] + mid[1] + mid[2]) < 3e38f;
+    ext[blockIdx.x] = fin && u < (float)half ? (int)u : half;
+  }
+}
+
+// How the spreading kernel's warps share the columns, which depends on the
+// cells in use and so is known on the device only: CTA b's first `per_cta`
+// warps work, warp i = b per_cta + w takes columns [i T / n, (i + 1) T / n).
+struct SpreadPlan {
+  int used, per_cta, n;
+};
+
+// (all threads of a CTA call this; s: shared scratch of 32 ints)
+__device__ __forceinline__ SpreadPlan spread_plan(const int *__restrict__ ext,
+                                                  int n_cfgs, int n_ctas,
+                                                  int max_warps, int warp_bytes,
+                                                  int cell_bytes, int smem,
+                                                  int total, int *s) {
+  int u = 0;
+  for (int i = threadIdx.y * blockDim.x + threadIdx.x; i < n_cfgs;
+       i += blockDim.x * blockDim.y)
+    u = max(u, ext[i]);
+  const int t = threadIdx.y * blockDim.x + threadIdx.x;
+  u = __reduce_max_sync(0xffffffffu, u);
+  if ((t & 31) == 0) s[t >> 5] = u;
+  __syncthreads();
+  const int nw = (blockDim.x * blockDim.y + 31) >> 5;
+  for (int w = 0; w < nw; ++w) u = max(u, s[w]);
+  SpreadPlan p;
+  p.used = u;
+  // as many warps as have room for a histogram, each with at least eight
+  // columns (its flush costs about four)
+  p.per_cta = min(max_warps, smem / (warp_bytes + cell_bytes * grid_words(u)));
+  // the four schedulers of the SM get equal numbers of warps
+  if (p.per_cta > 4) p.per_cta &= ~3;
+  p.per_cta = max(1, min(p.per_cta, (total + 8 * n_ctas - 1) / (8 * n_ctas)));
+  p.n = p.per_cta * n_ctas;
+  return p;
+}
+
+// One CTA per SM.  Each warp has a private histogram (no atomics, a fixed
+// order of additions: the result is the same bits on every run), and the
+// columns of all rows, in order, are dealt out evenly to the warps: warp i
+// writes one partial histogram per key it meets, at slot i + key.
+//
+// A column is 32 pairs, one per lane (lane = atom a of the tile, one b):
+// distance, cell and weight take about 60 instructions.  They are then
+// spread eight pairs at a time: lane = (slot, tap pair), each slot keeping
+// its own copy of the histogram, interleaved by cell ([cell][slot]), so that
+// the 32 lanes of a read or write fall on 32 different banks whatever the
+// cells are, and no two lanes touch the same word.  The lane's two taps of
+// the window are polynomials of degree 7 in the pair's position within its
+// cell, evaluated together by packed FMAs (coefficients in registers): 19
+// instructions per eight pairs.  Bound by instruction issue and the latency
+// of its dependent chains (0.60 issued per cycle and scheduler): two columns
+// go side by side, and as many warps run as have room for a histogram, 8 per
+// SM at 650 cells.  163 instructions per column; four slots of one tap per
+// lane, at half the memory per warp, took 248.
+// 64 x 1,000 atoms at 330 bins: 253 us (fq_pair3_kernel 1,451); 256 alloys of
+// 55 to 2,000 atoms at 500 bins 1.45 ms (11.5); 10,007 atoms at 1,500 bins
+// 0.60 ms (9.5).
+constexpr int kSpreadWarps = 16;
+constexpr int kSpreadSlots = 8;
+constexpr int kSpreadCols = 2;
+constexpr int kSpreadSmem = 224 * 1024;
+constexpr int kSpreadStage = 32 * 32;  // bytes of 32 staged atoms
+__global__ void __launch_bounds__(32 * kSpreadWarps)
+    fq_spread_kernel(const float *__restrict__ pos,
+                     const int *__restrict__ perm,
+                     const GridSeg *__restrict__ segs,
+                     const int *__restrict__ seg_begin, int n_segs, int total,
+                     const int *__restrict__ ext, int n_cfgs, GridScale gs,
+                     float near_r, float near_scale,
+                     const float *__restrict__ taps, int row_words,
+                     float *__restrict__ rows) {
+  extern __shared__ float4 smem4[];
+  __shared__ int splan[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const SpreadPlan plan =
+      spread_plan(ext, n_cfgs, gridDim.x, kSpreadWarps, kSpreadStage,
+                  4 * kSpreadSlots, kSpreadSmem, total, splan);
+  const int wi = blockIdx.x * plan.per_cta + warp;
+  const int c0 = (int)((long long)wi * total / plan.n);
+  const int c1 = (int)((long long)(wi + 1) * total / plan.n);
+  if (warp >= plan.per_cta || c0 >= c1) return;
+  const int words = grid_words(plan.used);
+  float4 *stage = smem4 + warp * (kSpreadStage / 16 + 2 * words);
+  float4 *hist4 = stage + kSpreadStage / 16;  // [word][slot]
+  float *hist = reinterpret_cast<float *>(hist4);
+  const int slot = lane >> 2, tp = lane & 3;  // taps tp and tp + 4
+  float2 cf[kTapCoef];
+#pragma unroll
+  for (int i = 0; i < kTapCoef; ++i)
+    cf[i] = make_float2(taps[tp * kTapCoef + i], taps[(tp + 4) * kTapCoef + i]);
+  for (int i = lane; i < 2 * words; i += 32)
+    hist4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncwarp();
+  // the row that holds column c0
+  int lo = 0, hi = n_segs;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (seg_begin[mid] <= c0)
+      lo = mid;
+    else
+      hi = mid;
+  }
+  // tap p of cell j is cell j - 3 + p
+  float *const base = hist + (8 + tp) * kSpreadSlots + slot;
+  auto flush = [&](int key) {
+    __syncwarp();
+    float *out = rows + (size_t)(wi + key) * row_words;
+    for (int i = lane; i < words; i += 32) {
+      const float4 v = hist4[2 * i], w = hist4[2 * i + 1];
+      out[i] = ((v.x + v.y) + (v.z + v.w)) + ((w.x + w.y) + (w.z + w.w));
+      hist4[2 * i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      hist4[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncwarp();
+  };
+  int cur = -1;
+  int c = c0;
+  for (int sgi = lo; c < c1; ++sgi) {
+    const GridSeg sg = segs[sgi];
+    const int begin = seg_begin[sgi], end = min(seg_begin[sgi + 1], c1);
+    if (sg.key != cur) {
+      if (cur >= 0) flush(cur);
+      cur = sg.key;
+    }
+    // (lanes past the tile count no pair: no b is below 0)
+    const int ia = lane < sg.na ? sg.a0 + lane : 0;
+    const float4 pa = load_atom(pos, perm, sg.a0 + min(lane, sg.na - 1));
+    const SplitAtom a = split_atom(pa.x, pa.y, pa.z);
+    for (; c < end; c += 32) {
+      // the next 32 (or fewer) b's, staged by one lane each
+      const int nb = min(32, end - c);
+      const int ib0 = sg.b0 + (c - begin);
+      const float4 q = load_atom(pos, perm, ib0 + min(lane, nb - 1));
+      const SplitAtom mine = split_atom(q.x, q.y, q.z);
+      __syncwarp();
+      stage[2 * lane] = make_float4(mine.hx, mine.hy, mine.hz, mine.lx);
+      stage[2 * lane + 1] = make_float4(mine.ly, mine.lz, 0.f, 0.f);
+      __syncwarp();
+      for (int i = 0; i < nb; i += kSpreadCols) {
+        // kSpreadCols columns side by side: their chains overlap
+        SplitAtom b[kSpreadCols];
+        bool on[kSpreadCols], ok[kSpreadCols];
+        float t[kSpreadCols], w[kSpreadCols];
+        int off[kSpreadCols];
+#pragma unroll
+        for (int q = 0; q < kSpreadCols; ++q) {
+          const int iq = min(i + q, nb - 1);
+          const float4 q0 = stage[2 * iq];
+          const float2 q1 =
+              *reinterpret_cast<const float2 *>(&stage[2 * iq + 1]);
+          b[q] = SplitAtom{q0.x, q0.y, q0.z, q0.w, q1.x, q1.y};
+          on[q] = ib0 + i + q < ia && i + q < nb;
+          PairDist p;
+          ok[q] = pair_dist_fast(a, b[q], p) && on[q];
+          float uh, ul;
+          grid_pos(gs, p.r, p.rl, uh, ul);
+          // sin is odd: the half [-M/2, 0] of the period folds on the other
+          w[q] = ok[q] ? (uh < 0.f ? -p.inv_r : p.inv_r) : 0.f;
+          ul = uh < 0.f ? -ul : ul;
+          uh = fabsf(uh);
+          const float fj = floorf(uh);
+          t[q] = ok[q] ? (uh - fj) + (ul - 0.5f) : 0.f;
+          off[q] = ok[q] ? min((int)fj, plan.used) * kSpreadSlots : 0;
+        }
+        int o[4 * kSpreadCols];
+        float2 v[4 * kSpreadCols];
+#pragma unroll
+        for (int it = 0; it < 4 * kSpreadCols; ++it) {
+          const int src = (it & 3) * 8 + slot;
+          o[it] = __shfl_sync(0xffffffffu, off[it >> 2], src);
+          const float2 tt = f2(__shfl_sync(0xffffffffu, t[it >> 2], src));
+          const float2 ww = f2(__shfl_sync(0xffffffffu, w[it >> 2], src));
+          float2 f = cf[7];
+#pragma unroll
+          for (int n = 6; n >= 0; --n) f = __ffma2_rn(f, tt, cf[n]);
+          v[it] = __fmul2_rn(ww, f);
+        }
+#pragma unroll
+        for (int it = 0; it < 4 * kSpreadCols; ++it) {
+          float *h = base + o[it];
+          const float x = h[0], y = h[4 * kSpreadSlots];
+          h[0] = x + v[it].x;
+          h[4 * kSpreadSlots] = y + v[it].y;
+          __syncwarp();
+        }
+        bool left = false;
+#pragma unroll
+        for (int q = 0; q < kSpreadCols; ++q) left |= on[q] && !ok[q];
+        if (!__any_sync(0xffffffffu, left)) continue;
+        // pairs that the fast distance does not cover, one at a time
+        for (int l = 0; l < 32; ++l) {
+          for (int q = 0; q < kSpreadCols; ++q) {
+            if (lane != l || !on[q] || ok[q]) continue;
+            const PairDist g = pair_dist_general(
+                a.hx + a.lx, a.hy + a.ly, a.hz + a.lz, b[q].hx + b[q].lx,
+                b[q].hy + b[q].ly, b[q].hz + b[q].lz);
+            if (g.r > 0.f && g.r < near_r) {
+              // far below the resolution of Q (Q_max r < 0.6): the power
+              // sums of r^2 give sin(Q r)/r, which the window would only
+              // give to 1e-7 / r
+              const float z = (g.r * near_scale) * (g.r * near_scale);
+              float x = 1.f;
+              for (int n = 0; n < kNearTerms; ++n, x *= z)
+                hist[n * kSpreadSlots] += x;
+            } else {
+              float uh, ul;
+              grid_pos(gs, g.r, g.rl, uh, ul);
+              float wg = uh < 0.f ? -g.inv_r : g.inv_r;
+              ul = uh < 0.f ? -ul : ul;
+              uh = fabsf(uh);
+              // r = 0, infinite or NaN: NaN for every bin, as sin(Q r)/r is
+              if (!(g.r > 0.f && g.r < 3e38f)) wg = __int_as_float(0x7fffffff);
+              const float fg = floorf(uh);
+              const float tg =
+                  fminf(fmaxf((uh - fg) + (ul - 0.5f), -0.5f), 0.5f);
+              const int j = min(max((int)fg, 0), plan.used);
+              for (int n = 0; n < kTaps; ++n) {
+                float f = taps[n * kTapCoef + 7];
+                for (int m = 6; m >= 0; --m)
+                  f = fmaf(f, tg, taps[n * kTapCoef + m]);
+                hist[(8 + j + n) * kSpreadSlots] += wg * f;
+              }
+            }
+          }
+          __syncwarp();
+        }
+      }
+    }
+    c = end;
+  }
+  flush(cur);
+}
+
+// Sums the partial histograms of a key and folds them for the transform.
+// With j' = M/2 - j, sin(2 pi k j'/M) is -(-1)^k sin(2 pi k j/M), so even
+// bins need G-_j = H_j - H_j' and odd bins G+_j = H_j + H_j' for j <= M/4
+// only: out[key][j] = (G-_j, G+_j), then the power sums.  The slots follow
+// from the plan of the spreading kernel, made again here from its arguments.
+// Threads (x: cell, y: a share of the slots) add in float pairs.
+__global__ void fq_grid_reduce_kernel(const float *__restrict__ rows,
+                                      const int2 *__restrict__ key_cols,
+                                      const int *__restrict__ ext, int n_cfgs,
+                                      int n_ctas, int total, int m,
+                                      int row_words, float *__restrict__ out) {
+  extern __shared__ float sred[];  // [4][blockDim.y][32]
+  __shared__ int splan[32];
+  const SpreadPlan plan =
+      spread_plan(ext, n_cfgs, n_ctas, kSpreadWarps, kSpreadStage,
+                  4 * kSpreadSlots, kSpreadSmem, total, splan);
+  const int2 kc = key_cols[blockIdx.y];  // columns [x, y) of the key
+  // warps of column x and of column y - 1
+  auto warp_of = [&](long long col) {
+    long long i = col * plan.n / total;
+    while (i > 0 && i * total / plan.n > col) --i;
+    while ((i + 1) * total / plan.n <= col) ++i;
+    return (int)i;
+  };
+  const int w0 = warp_of(kc.x), n_rows = warp_of(kc.y - 1) - w0 + 1;
+  const int quarter = m / 4, half = m / 2;
+  const int j = blockIdx.x * 32 + threadIdx.x;
+  // the cells that meet in (G-_j, G+_j): j, its mirror images at 0 and M/2
+  float hs = 0.f, hc = 0.f, ms = 0.f, mc = 0.f;
+  const bool on = j <= quarter, near = j > quarter && j <= quarter + kNearTerms;
+  auto add = [](float x, float &s, float &c) {
+    const float y = __fadd_rn(x, c);
+    const float t = __fadd_rn(s, y);
+    c = __fsub_rn(y, __fsub_rn(t, s));
+    s = t;
+  };
+  if (on || near) {
+    const int j1 = half - j, last = plan.used + 4;
+    for (int i = threadIdx.y; i < n_rows; i += blockDim.y) {
+      const float *r = rows + (size_t)(w0 + blockIdx.y + i) * row_words;
+      if (near) {
+        add(r[j - quarter - 1], hs, hc);
+      } else {
+        // cells below 0 and above M/2 are images with the opposite sign
+        r += kGridCell0;
+        float x = j <= last ? r[j] : 0.f, y = j1 <= last ? r[j1] : 0.f;
+        if (j >= 1 && j <= 3) x -= r[-j];
+        if (j >= 1 && half + j <= last) y -= r[half + j];
+        add(x, hs, hc);
+        add(y, ms, mc);
+      }
+    }
+  }
+  float *sh = sred + threadIdx.y * 32 + threadIdx.x;
+  const int st = blockDim.y * 32;
+  sh[0] = hs;
+  sh[st] = hc;
+  sh[2 * st] = ms;
+  sh[3 * st] = mc;
+  __syncthreads();
+  if (threadIdx.y != 0 || !(on || near)) return;
+  for (int y = 1; y < (int)blockDim.y; ++y) {
+    add(sh[y * 32], hs, hc);
+    hc += sh[st + y * 32];
+    add(sh[2 * st + y * 32], ms, mc);
+    mc += sh[3 * st + y * 32];
+  }
+  float *o = out + (size_t)blockIdx.y * (2 * (quarter + 1) + 8);
+  if (near) {
+    o[2 * (quarter + 1) + (j - quarter - 1)] = hs + hc;
+  } else {
+    const bool mid = j == quarter;  // its own mirror image
+    o[2 * j] = j == 0 || mid ? 0.f : (hs - ms) + (hc - mc);
+    o[2 * j + 1] = j == 0 ? 0.f : mid ? hs + hc : (hs + ms) + (hc + mc);
+  }
+}
+
+// F(Q) of the configurations on the grid.  CTA = (32 bins, configuration),
+// lane = bin k; the warps share the cells j in blocks of 17 around an
+// accurate centre sin(theta_k jc), from which the others are one rotation by
+// n theta_k, n <= 8.  About 6 instructions per (bin, cell), FP32 issue bound;
+// block sums are added in float pairs, the rest is FP64 per bin.
+constexpr int kFqDftWarps = 8;
+constexpr int kFqDftReach = 8;
+// floats of shared memory: (G-, G+) up to a whole round of blocks past M/4
+__host__ __device__ constexpr int fq_dft_floats(int m) {
+  return 2 * (m / 4 + 2 + kFqDftWarps * (2 * kFqDftReach + 1)) + 8;
+}
+__global__ void __launch_bounds__(32 * kFqDftWarps)
+    fq_grid_finish_kernel(const float *__restrict__ hsum,
+                          const int4 *__restrict__ cfg_keys,
+                          const int *__restrict__ key_spair,
+                          const int2 *__restrict__ spair_species,
+                          const float *__restrict__ ftab,
+                          const double *__restrict__ na,
+                          const double *__restrict__ inv_phi, int m,
+                          float inv_m, int n_bins, int kb_out, double dq, float near_unit,
+                          float *__restrict__ fq, double *__restrict__ fq_raw) {
+  constexpr int R = kFqDftReach;
+  extern __shared__ float sh[];  // the key's folded histogram, zero-padded
+  __shared__ float red[2][kFqDftWarps][32];
+  const int4 ck = cfg_keys[blockIdx.y];  // configuration, first key, keys
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int k = min((int)(blockIdx.x * 32 + lane), n_bins - 1);
+  const int quarter = m / 4;
+  float sn[R], cn[R];
+#pragma unroll
+  for (int n = 0; n < R; ++n)
+    sincos_turn((int)((unsigned)(n + 1) * (unsigned)k % (unsigned)m), m, inv_m,
+                sn[n], cn[n]);
+  double sum = 0.0;
+  for (int q = 0; q < ck.z; ++q) {
+    const float *h = hsum + (size_t)(ck.y + q) * (2 * (quarter + 1) + 8);
+    __syncthreads();
+    for (int i = threadIdx.x; i < fq_dft_floats(m) - 8; i += blockDim.x)
+      sh[i] = i < 2 * (quarter + 1) ? h[i] : 0.f;
+    __syncthreads();
+    const float *hk = sh + (k & 1);
+    float s = 0.f, c = 0.f;
+    for (int j0 = 1 + warp * (2 * R + 1); j0 <= quarter;
+         j0 += kFqDftWarps * (2 * R + 1)) {
+      float sc, cc;
+      sincos_turn((int)((unsigned)k * (unsigned)(j0 + R) % (unsigned)m), m,
+                  inv_m, sc, cc);
+      const float *hj = hk + 2 * (j0 + R);
+      float blk = sc * hj[0];
+#pragma unroll
+      for (int n = 1; n <= R; ++n) {
+        const float u = sc * cn[n - 1], v = cc * sn[n - 1];
+        blk = fmaf(u + v, hj[2 * n], blk);
+        blk = fmaf(u - v, hj[-2 * n], blk);
+      }
+      const float y = __fadd_rn(blk, c);
+      const float t = __fadd_rn(s, y);
+      c = __fsub_rn(y, __fsub_rn(t, s));
+      s = t;
+    }
+    __syncthreads();
+    red[0][warp][lane] = s;
+    red[1][warp][lane] = c;
+    __syncthreads();
+    if (warp == 0) {
+      double d = 0.0;
+      for (int w = 0; w < kFqDftWarps; ++w)
+        d += (double)red[0][w][lane] + (double)red[1][w][lane];
+      d *= inv_phi[k];
+      const float *nr = h + 2 * (quarter + 1);
+      if (nr[0] != 0.f) {
+        // sum over near pairs of sin(Q r)/r = Q sum_n (-1)^n (Q r)^2n /
+        // (2n + 1)!; nr[n] = sum (Q_max r)^2n
+        const float z = -(k * near_unit) * (k * near_unit);
+        const float v =
+            nr[0] +
+            z * (nr[1] / 6.f +
+                 z * (nr[2] / 120.f +
+                      z * (nr[3] / 5040.f + z * (nr[4] / 362880.f))));
+        d += (double)k * dq * (double)v;
+      }
+      const int2 ss = spair_species[key_spair[ck.y + q]];
+      sum += (double)ftab[ss.x * n_bins + k] * (double)ftab[ss.y * n_bins + k] *
+             d;
+    }
+  }
+  const int kk = blockIdx.x * 32 + lane;
+  if (warp != 0 || kk >= n_bins) return;
+  const size_t o = (size_t)ck.x * n_bins + kk;
+  const bool on = kk >= kb_out;
+  if (fq) fq[o] = on ? fq_value(sum, na[o]) : 0.f;
+  if (fq_raw) fq_raw[o] = on ? sum : 0.0;
+}
+
+}  // namespace pyiid

@@ -78,20 +78,17 @@ static __device__ __noinline__ PairDist pair_dist_general(float ax, float ay,
 // and so is the sum n of their squares up to 128 A (24 bits); what the rest
 // adds, c = sum dl (2 dh + dl), carries an absolute error of 2^-24 c, which
 // is under 1e-8 A in r.  That is half the operations of the error-free form
-// (27 against 58).  Pairs nearer than 0.1 A or further than 128 A, where the
-// argument fails, and NaN take the general form.
-__device__ __forceinline__ PairDist pair_dist(const SplitAtom &a,
-                                              const SplitAtom &b) {
-  PairDist p;
+// (27 against 58).  False for pairs nearer than 0.1 A or further than 128 A,
+// where the argument fails, and for NaN: they take the general form.
+__device__ __forceinline__ bool pair_dist_fast(const SplitAtom &a,
+                                               const SplitAtom &b,
+                                               PairDist &p) {
   const float hx = a.hx - b.hx, hy = a.hy - b.hy, hz = a.hz - b.hz;
   const float lx = a.lx - b.lx, ly = a.ly - b.ly, lz = a.lz - b.lz;
   const float n = fmaf(hx, hx, fmaf(hy, hy, hz * hz));
   const float c = fmaf(lx, fmaf(2.0f, hx, lx),
                        fmaf(ly, fmaf(2.0f, hy, ly), lz * fmaf(2.0f, hz, lz)));
   const float s = __fadd_rn(n, c);
-  if (!(s > 0.01f && n < 16384.0f))
-    return pair_dist_general(a.hx + a.lx, a.hy + a.ly, a.hz + a.lz,
-                             b.hx + b.lx, b.hy + b.ly, b.hz + b.lz);
   const float e = __fadd_rn(__fsub_rn(n, s), c);
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
@@ -103,6 +100,15 @@ __device__ __forceinline__ PairDist pair_dist(const SplitAtom &a,
   p.dx = hx + lx;
   p.dy = hy + ly;
   p.dz = hz + lz;
+  return s > 0.01f && n < 16384.0f;
+}
+
+__device__ __forceinline__ PairDist pair_dist(const SplitAtom &a,
+                                              const SplitAtom &b) {
+  PairDist p;
+  if (!pair_dist_fast(a, b, p))
+    p = pair_dist_general(a.hx + a.lx, a.hy + a.ly, a.hz + a.lz, b.hx + b.lx,
+                          b.hy + b.ly, b.hz + b.lz);
   return p;
 }
 

@@ -101,3 +101,90 @@ def test_pair_force_table_close_and_coincident_pairs(D):
     pos[11] = pos[40]
     g = D.batch_potential_grad(pos, *args)['grad'].cpu().numpy()
     assert np.all(np.isnan(g[[11, 40]]))
+
+
+def fq64(pos, sp, tab, qb):
+    return O.fq(np.asarray(pos, np.float32), tab[sp], qb)
+
+
+# sizes either side of the rule that takes a call to the grid; odd bin counts
+# (M is rounded up to a multiple of 4); two and three elements; k_begin odd;
+# a period shorter than the cluster; a cluster away from the origin
+@pytest.mark.parametrize('n,species,qb,nb,kb,shift', [
+    (380, 1, 0.05, 500, 2, 0.0),
+    (421, 1, 0.05, 501, 3, 25.0),
+    (600, 2, 0.05, 499, 0, 0.0),
+    (260, 1, 0.02, 1475, 25, -70.0),
+    (700, 1, 0.4, 250, 1, 0.0),
+    (640, 3, 0.02, 1502, 0, 0.0),
+])
+def test_fq_on_the_grid_matches_oracle(D, n, species, qb, nb, kb, shift):
+    pos, nums = cluster(n, n, species, shift)
+    sp, tab = tables(nums, qb, nb)
+    f = D.fq(pos, sp, tab, qb, k_begin=kb).cpu().numpy()
+    f2 = D.fq(pos, sp, tab, qb, k_begin=kb).cpu().numpy()
+    assert np.array_equal(f, f2) and np.all(f[:kb] == 0)
+    idx = np.unique(np.concatenate([np.arange(kb, nb, 7), [nb - 1]]))
+    x = pos.astype(np.float64)
+    fi = tab[sp][:, idx].astype(np.float64)
+    s = np.zeros(len(idx))
+    for a in range(1, n):
+        d = np.sqrt(((x[a] - x[:a]) ** 2).sum(1))[:, None]
+        s += fi[a] * (fi[:a] * np.sin(idx * qb * d) / d).sum(0)
+    want = 2 * s / O.normalization(tab[sp])[idx]
+    assert rel(f[idx], want) <= TOL_F, rel(f[idx], want)
+
+
+def test_fq_on_the_grid_close_coincident_and_far_pairs(D):
+    """Pairs at tiny distances (power sums), under 0.1 A and beyond 128 A
+    (general distance) against the oracle; a coincident pair makes every bin
+    0, as the reference's NaN does, and so does a NaN position, in its own
+    configuration only."""
+    qb, nb = 0.05, 300
+    pos, nums = cluster(420, 9, 2)
+    pos[30] = pos[7] + np.float32([1e-3, 0, 0])
+    pos[31] = pos[8] + np.float32([0.02, 0.03, 0.01])
+    pos[32] += np.float32([150.0, 0, 0])
+    sp, tab = tables(nums, qb, nb)
+    want = fq64(pos, sp, tab, qb)
+    assert rel(D.fq(pos, sp, tab, qb).cpu().numpy(), want) <= TOL_F
+    bad = pos.copy()
+    bad[30] = bad[7]
+    nan = pos.copy()
+    nan[5, 1] = np.nan
+    both = np.concatenate([bad, pos, nan])
+    f = D.batch_fq(both, np.tile(sp, 3), np.array([0, 420, 840, 1260]), tab,
+                   qb).cpu().numpy()
+    assert np.all(f[0] == 0) and np.all(f[2] == 0)
+    assert rel(f[1], want) <= TOL_F
+
+
+def test_mixed_batch_of_grid_and_direct_configurations(D):
+    """Small configurations of a batch stay on the direct kernels beside the
+    ones on the grid; a CUDA graph replay equals the eager call bitwise."""
+    import torch
+    qb, nb = 0.05, 500
+    sizes = [3, 500, 0, 60, 450, 1, 33, 600]
+    parts = [cluster(n, 60 + n, 2) for n in sizes if n]
+    pos = torch.as_tensor(np.concatenate([p for p, _ in parts]).astype(
+        np.float32), device='cuda')
+    sp, tab = tables(np.concatenate([z for _, z in parts]), qb, nb)
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    f = D.batch_fq(pos, sp, off, tab, qb, 2)
+    out = torch.empty_like(f)
+    D.batch_fq(pos, sp, off, tab, qb, 2, out=out)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        D.batch_fq(pos, sp, off, tab, qb, 2, out=out)
+    out.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, f)
+    p = pos.cpu().numpy()
+    for i, n in enumerate(sizes):
+        a, b = off[i], off[i + 1]
+        got = f[i].cpu().numpy()
+        if n < 2:
+            assert np.all(got == 0)
+        else:
+            assert rel(got[2:], fq64(p[a:b], sp[a:b], tab, qb)[2:]) <= TOL_F
