@@ -27,6 +27,7 @@
 #include "adjoint_grid.cuh"
 #include "debye_kernels.cuh"
 #include "fq_grid.cuh"
+#include "grad_grid.cuh"
 #include "move_kernels.cuh"
 #include "spring_kernels.cuh"
 #include "transform_kernels.cuh"
@@ -200,15 +201,23 @@ struct DevBuf {
 struct FqGridWork {
   int n_bins = 0;
   int n_segs = 0, total = 0, n_keys = 0, n_cfgs = 0;  // n_cfgs 0: no work
-  int max_cols = 0;  // most columns of one key
   int n_direct = 0;  // work items of the other configurations
   GridSeg *d_segs = nullptr;
   int *d_seg_begin = nullptr;
-  int2 *d_key_cols = nullptr;
+  KeyCols *d_key_cols = nullptr;
   int *d_key_spair = nullptr;
   int4 *d_cfg_keys = nullptr;
   int *d_direct_order = nullptr;
   unsigned char *d_skip = nullptr;
+};
+
+// Work of the gradient's grid path for a layout of one configuration.
+struct GradGridWork {
+  int total = 0, units = 0, staged = 0;
+  GradBlock *d_blocks = nullptr;   // [n_species][n_species]
+  KeyCols *d_key_cols = nullptr;   // columns of each species pair
+  int *d_key_spair = nullptr;
+  int4 *d_cfg_keys = nullptr;
 };
 
 struct Layout {
@@ -249,6 +258,7 @@ struct Layout {
   int *d_key_item_begin = nullptr;
   int2 *d_spair = nullptr;
   std::vector<std::unique_ptr<FqGridWork>> fq_grid;  // by n_bins, newest first
+  std::unique_ptr<GradGridWork> grad_grid;
 };
 
 // Phase grid of n_bins bins (independent of their step): the window's
@@ -257,6 +267,8 @@ struct PhaseGrid {
   int n_bins = 0, m = 0;
   float *d_taps = nullptr;      // [kTaps][kTapCoef]
   double *d_inv_phi = nullptr;  // [n_bins]
+  // gradient grids only: (P, R) of each bin, e^{-2 pi i n / m} for n < m
+  float2 *d_pr = nullptr, *d_tw = nullptr;
 };
 
 struct TMatrix {
@@ -400,8 +412,21 @@ void free_fq_grid(FqGridWork *W) {
   cudaFree(W->d_skip);
 }
 
+void free_phase_grid(PhaseGrid *G) {
+  cudaFree(G->d_taps);
+  cudaFree(G->d_inv_phi);
+  cudaFree(G->d_pr);
+  cudaFree(G->d_tw);
+}
+
 void free_layout(Layout *L) {
   for (auto &W : L->fq_grid) free_fq_grid(W.get());
+  if (L->grad_grid) {
+    cudaFree(L->grad_grid->d_blocks);
+    cudaFree(L->grad_grid->d_key_cols);
+    cudaFree(L->grad_grid->d_key_spair);
+    cudaFree(L->grad_grid->d_cfg_keys);
+  }
   cudaFree(L->d_perm);
   cudaFree(L->d_tiles);
   cudaFree(L->d_cfg_tiles);
@@ -728,8 +753,11 @@ void split_double(double x, float &hi, float &lo) {
   lo = (float)(x - (double)hi);
 }
 
+int set_grad_grid_attrs(pyiid_ctx *ctx);
+
 int set_attrs(pyiid_ctx *ctx) {
   if (ctx->attrs_set) return PYIID_OK;
+  TRY(set_grad_grid_attrs(ctx));
   for (int i = 0; i < kNumGrad; ++i)
     CUDA_TRY(ctx, cudaFuncSetAttribute(
                       kGradTable[i].k,
@@ -764,8 +792,8 @@ int set_attrs(pyiid_ctx *ctx) {
   CUDA_TRY(ctx, cudaFuncSetAttribute(
                     fq_grid_finish_kernel,
                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                    (int)(fq_dft_floats(kFqCellsPerBin * kFqGridMaxBins) *
-                          sizeof(float))));
+                    (int)(fq_dft_float4(kFqCellsPerBin * kFqGridMaxBins) *
+                          sizeof(float4))));
   CUDA_TRY(ctx, cudaFuncSetAttribute(adjoint_grid_kernel<true>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kAdjTabSmem));
@@ -866,26 +894,42 @@ void window_spectrum(const float *taps, int m, int n_bins, double *phi,
   }
 }
 
-int get_fq_phase_grid(pyiid_ctx *ctx, int n_bins, PhaseGrid **out) {
+// The grid of m cells for n_bins bins (with_grad: the gradient's tables too).
+int get_phase_grid(pyiid_ctx *ctx, int n_bins, int m, bool with_grad,
+                   PhaseGrid **out) {
   for (auto &G : ctx->grids)
-    if (G->n_bins == n_bins) {
+    if (G->n_bins == n_bins && G->m == m && (G->d_pr != nullptr) == with_grad) {
       *out = G.get();
       return PYIID_OK;
     }
   auto G = std::make_unique<PhaseGrid>();
   G->n_bins = n_bins;
-  G->m = (kFqCellsPerBin * n_bins + 3) & ~3;
+  G->m = m;
   std::vector<float> taps(kTaps * kTapCoef);
-  window_taps((double)G->m / (2.0 * n_bins), taps.data());
-  std::vector<double> phi(n_bins);
-  window_spectrum(taps.data(), G->m, n_bins, phi.data(), nullptr);
-  for (double &v : phi) v = 1.0 / v;
+  window_taps((double)m / (2.0 * n_bins), taps.data());
+  std::vector<double> phi(n_bins), dphi(n_bins);
+  window_spectrum(taps.data(), m, n_bins, phi.data(), dphi.data());
+  std::vector<float2> pr(n_bins);
+  for (int k = 0; k < n_bins; ++k) {
+    const double th = 2.0 * M_PI * k / m;
+    pr[k] = make_float2((float)(th / phi[k]),
+                        (float)((1.0 + th * dphi[k] / phi[k]) / phi[k]));
+    phi[k] = 1.0 / phi[k];
+  }
   TRY(upload(ctx, &G->d_taps, taps));
   TRY(upload(ctx, &G->d_inv_phi, phi));
+  if (with_grad) {
+    std::vector<float2> tw(m);
+    for (int n = 0; n < m; ++n) {
+      const double x = 2.0 * M_PI * n / m;
+      tw[n] = make_float2((float)std::cos(x), (float)-std::sin(x));
+    }
+    TRY(upload(ctx, &G->d_pr, pr));
+    TRY(upload(ctx, &G->d_tw, tw));
+  }
   ctx->grids.insert(ctx->grids.begin(), std::move(G));
   while (ctx->grids.size() > 16) {
-    cudaFree(ctx->grids.back()->d_taps);
-    cudaFree(ctx->grids.back()->d_inv_phi);
+    free_phase_grid(ctx->grids.back().get());
     ctx->grids.pop_back();
   }
   *out = ctx->grids[0].get();
@@ -944,7 +988,7 @@ int get_fq_grid_work(pyiid_ctx *ctx, Layout *L, int n_bins,
   std::vector<GridSeg> segs;
   std::vector<int> begin, key_spair, direct;
   std::vector<int4> cfg_keys;
-  std::vector<int2> cols;  // columns [x, y) of each key
+  std::vector<KeyCols> cols;  // columns of each key
   std::vector<unsigned char> skip(L->n_configs, 0);
   long long total = 0;
   for (int c : fq_grid_configs(L, n_bins)) {
@@ -972,7 +1016,7 @@ int get_fq_grid_work(pyiid_ctx *ctx, Layout *L, int n_bins,
         begin.push_back((int)total);
         total += nb;
       }
-      cols.push_back(make_int2(x, (int)total));
+      cols.push_back(KeyCols{x, (int)total, (int)key_spair.size(), 0, 0, 0});
       key_spair.push_back(sp);
     }
     cfg_keys.push_back(
@@ -986,7 +1030,6 @@ int get_fq_grid_work(pyiid_ctx *ctx, Layout *L, int n_bins,
   if (W->n_keys <= 65535 && total < INT32_MAX / 2)
     W->n_cfgs = (int)cfg_keys.size();
   if (W->n_cfgs > 0) {
-    for (const int2 &k : cols) W->max_cols = std::max(W->max_cols, k.y - k.x);
     for (int i : L->item_order)
       if (!skip[L->items[i].w / L->n_spairs]) direct.push_back(i);
     W->n_direct = (int)direct.size();
@@ -1114,46 +1157,77 @@ int check_common(pyiid_ctx *ctx, int n_configs, const int32_t *offsets,
   return PYIID_OK;
 }
 
+// Sums the partial histograms of n_keys keys, at most about
+// `most` of each: about four of them per thread row.  Many rows over few cells take
+// CTAs of eight cells, so that there are enough of those.
+int launch_grid_reduce(pyiid_ctx *ctx, const HistRows &rows,
+                       const KeyCols *d_key_cols, const int *ext, int n_cfgs,
+                       PlanShape shape, int total, int m, int n_keys,
+                       double most, float *out) {
+  int ny = 1;
+  const int nx = most > 128 ? 8 : 32;
+  while (ny < 512 / nx && ny * 4 < most) ny *= 2;
+  fq_grid_reduce_kernel<<<dim3(fq_reduce_blocks(m, nx), n_keys), nx * ny,
+                          4 * nx * ny * sizeof(float), ctx->stream>>>(
+      rows, d_key_cols, ext, n_cfgs, shape, total, m, nx, ny, out);
+  LAUNCH_CHECK(ctx);
+  return PYIID_OK;
+}
+
+// Buffers `name` for the partial histograms of n_keys keys.
+int hist_rows(pyiid_ctx *ctx, const std::string &name, int n_keys,
+              int row_words, HistRows *out) {
+  const int n_ctas = ctx->n_sms;
+  const size_t slots = (size_t)kSpreadWarps * n_ctas + n_keys;
+  void *p;
+  TRY(ensure(ctx, (name + "_rows").c_str(),
+             (slots + n_ctas) * row_words * sizeof(float), &p));
+  out->rows = static_cast<float *>(p);
+  TRY(ensure(ctx, (name + "_flag").c_str(), slots * sizeof(int), &p));
+  out->flag = static_cast<int *>(p);
+  TRY(ensure(ctx, (name + "_cta").c_str(), n_ctas * sizeof(int2), &p));
+  out->cta = static_cast<int2 *>(p);
+  out->n_ctas = n_ctas;
+  out->row_words = row_words;
+  return PYIID_OK;
+}
+
 // F(Q) of the configurations of W (fq_grid.cuh): spread, sum, transform.
 int run_fq_grid(pyiid_ctx *ctx, const Layout *L, const FqGridWork *W,
                 const float *positions, const float *d_ftab,
                 const double *d_na, int n_bins, double qbin, int kb_out,
                 float *fq, double *fq_raw) {
   PhaseGrid *G;
-  TRY(get_fq_phase_grid(ctx, n_bins, &G));
-  const int m = G->m, quarter = m / 4;
-  const int row_words = grid_words(m / 2), n_ctas = ctx->n_sms;
+  const int m = (kFqCellsPerBin * n_bins + 3) & ~3;
+  TRY(get_phase_grid(ctx, n_bins, m, false, &G));
+  const int n_ctas = ctx->n_sms;
+  HistRows rows;
+  TRY(hist_rows(ctx, "fqg", W->n_keys, grid_words(m / 2), &rows));
   void *p;
-  TRY(ensure(ctx, "fqg_rows",
-             ((size_t)kSpreadWarps * n_ctas + W->n_keys) * row_words *
-                 sizeof(float),
-             &p));
-  float *rows = static_cast<float *>(p);
   TRY(ensure(ctx, "fqg_sum",
-             (size_t)W->n_keys * (2 * (quarter + 1) + 8) * sizeof(float), &p));
+             (size_t)W->n_keys * fq_sum_floats(m) * sizeof(float), &p));
   float *hsum = static_cast<float *>(p);
   TRY(ensure(ctx, "fqg_ext", (size_t)W->n_cfgs * sizeof(int), &p));
   int *ext = static_cast<int *>(p);
   const GridScale gs = grid_scale(qbin, m);
-  grid_extent_kernel<<<W->n_cfgs, 256, 0, ctx->stream>>>(
-      positions, L->d_offsets, W->d_cfg_keys, gs.hi, m / 2, ext);
+  // (about twenty atoms per thread, but small CTAs for batches)
+  grid_extent_kernel<<<W->n_cfgs, W->n_cfgs > 8 ? 256 : 1024, 0,
+                       ctx->stream>>>(positions, L->d_offsets, W->d_cfg_keys,
+                                      gs.hi, m / 2, ext);
   LAUNCH_CHECK(ctx);
   fq_spread_kernel<<<n_ctas, 32 * kSpreadWarps, kSpreadSmem, ctx->stream>>>(
       positions, L->d_perm, W->d_segs, W->d_seg_begin, W->n_segs, W->total,
       ext, W->n_cfgs, gs, (float)(kNearPhase / (n_bins * qbin)),
-      (float)(n_bins * qbin), G->d_taps, row_words, rows);
+      (float)(n_bins * qbin), G->d_taps, rows);
   LAUNCH_CHECK(ctx);
-  // a share of about eight slots per thread row, at most 32 rows
+  // partial histograms of a key: one per CTA, or per warp where the keys are
+  // so many that CTAs hold several
   const double most =
-      (double)W->max_cols / W->total * kSpreadWarps * n_ctas + 2;
-  const int ny = std::max(1, std::min(32, (int)(most / 8)));
-  fq_grid_reduce_kernel<<<dim3((quarter + kNearTerms) / 32 + 1, W->n_keys),
-                          dim3(32, ny), 4 * ny * 32 * sizeof(float),
-                          ctx->stream>>>(rows, W->d_key_cols, ext, W->n_cfgs,
-                                         n_ctas, W->total, m, row_words, hsum);
-  LAUNCH_CHECK(ctx);
+      (double)n_ctas / W->n_keys * (W->n_keys > n_ctas / 4 ? kSpreadWarps : 1);
+  TRY(launch_grid_reduce(ctx, rows, W->d_key_cols, ext, W->n_cfgs, kFqPlan,
+                         W->total, m, W->n_keys, most, hsum));
   fq_grid_finish_kernel<<<dim3((n_bins + 31) / 32, W->n_cfgs),
-                          32 * kFqDftWarps, fq_dft_floats(m) * sizeof(float),
+                          32 * kFqDftWarps, fq_dft_float4(m) * sizeof(float4),
                           ctx->stream>>>(
       hsum, W->d_cfg_keys, W->d_key_spair, L->d_spair, d_ftab, d_na,
       G->d_inv_phi, m, 1.0f / (float)m, n_bins, kb_out, qbin,
@@ -1229,6 +1303,195 @@ int run_fq(pyiid_ctx *ctx, Layout *L, const float *positions,
   fq_finish_kernel<<<g2, 128, 0, ctx->stream>>>(
       partial, L->d_key_item_begin, d_ftab, L->d_spair, d_na, L->n_spairs,
       n_bins, kb_out, fq, fq_raw, skip);
+  LAUNCH_CHECK(ctx);
+  return PYIID_OK;
+}
+
+// ------------------------------------------------ gradient on the grid
+using GradTransform = void (*)(const float *, const float *, const int *,
+                               const int2 *, const GradBlock *, int,
+                               const int *, const int *, const float2 *,
+                               const float2 *, const float *, int, int, float,
+                               float, float *, FqReduceArgs);
+// Transforms by length L = M / 2, shortest first.
+struct GradTransformEntry {
+  int len, threads;
+  GradTransform k;
+};
+template <int R0, int R1, int R2>
+constexpr GradTransformEntry grad_transform_entry() {
+  return {R0 * R1 * R2, fft_threads(R0 * R1 * R2),
+          grad_transform_kernel<R0, R1, R2>};
+}
+const GradTransformEntry kGradTransforms[] = {
+    grad_transform_entry<12, 8, 4>(),   grad_transform_entry<8, 8, 8>(),
+    grad_transform_entry<12, 8, 8>(),   grad_transform_entry<16, 8, 8>(),
+    grad_transform_entry<12, 16, 8>(),  grad_transform_entry<16, 16, 8>(),
+    grad_transform_entry<12, 16, 16>(), grad_transform_entry<16, 16, 16>(),
+};
+size_t grad_transform_smem(int len) {
+  return 2 * (size_t)(len + len / 16) * sizeof(float2);
+}
+
+int set_grad_grid_attrs(pyiid_ctx *ctx) {
+  CUDA_TRY(ctx, cudaFuncSetAttribute(
+                    grad_spread_kernel<true>,
+                    cudaFuncAttributeMaxDynamicSharedMemorySize, kSpreadSmem));
+  CUDA_TRY(ctx, cudaFuncSetAttribute(
+                    grad_spread_kernel<false>,
+                    cudaFuncAttributeMaxDynamicSharedMemorySize, kSpreadSmem));
+  for (const GradTransformEntry &E : kGradTransforms)
+    CUDA_TRY(ctx, cudaFuncSetAttribute(
+                      E.k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                      (int)grad_transform_smem(E.len)));
+  return PYIID_OK;
+}
+
+// The shortest transform with M >= 4.08 n_bins (nullptr: too many bins).
+// At sigma = M / (2 n_bins) = 2.04 the window leaves 8e-8 rms of a term out,
+// 1e-8 at 2.7; the direct kernels' seeds and recurrences leave 2e-7.
+const GradTransformEntry *grad_transform_for(int n_bins) {
+  for (const GradTransformEntry &E : kGradTransforms)
+    if (2.0 * E.len >= 4.08 * n_bins) return &E;
+  return nullptr;
+}
+
+// Whether a gradient (with_f: and F(Q) beside it) goes through the grid.
+// Times in us of both paths, fitted to 16 to 640 atoms of one to three
+// elements at 250, 500 and 1,500 bins.  Direct: a tile's 32 partners one
+// after the other while the pairs do not fill the GPU, then 5.1e-7 per pair
+// and bin.  Grid: its launches, and per species pair of F a transform or per
+// species the sums of the rows.  Measured, direct / grid: 16 atoms at 500
+// bins 20.7 / 24.2 (gradient alone 18.6 / 13.3), 32 35.2 / 21.5, 249
+// 52.8 / 26.5, 1,000 276 / 77; of two elements 64 36.1 / 36.3, 249
+// 53.4 / 40.8; of three 160 37.8 / 50.1, 400 79.2 / 73.9; of two at 1,500
+// bins 160 54.9 / 65.8, 249 78.7 / 75.3, 2,001 (gradient) 2,050 / 374.
+bool grad_on_grid(const Layout *L, int n_bins, bool with_f) {
+  const GradTransformEntry *E = grad_transform_for(n_bins);
+  if (!E || L->n_configs != 1 || L->total < 2) return false;
+  std::vector<int> count(L->n_species, 0);
+  for (const int4 &t : L->tiles) count[t.w] += t.y;
+  double s = 0;
+  for (int c : count) s += c > 0;
+  const double n = L->total, k = n_bins, x = n * n * k;
+  double direct = x > 2.5e7 ? 37.7 + 5.1e-7 * x
+                            : 9.5 + 0.78 * std::min(32.0, n / s);
+  if (!with_f) direct *= 0.85;
+  const double grid =
+      (with_f ? 18 + s * (s + 1) / 2 * (2.5 + k / 165) : 12 + s * (4 + k / 300)) +
+      5e-5 * s * k * std::max(0.0, n - 100);
+  // the rows of all units (and those of far pairs) stay under 24 GB, and the
+  // columns under 2^31
+  const double rows = 6.0 * 4.0 * (n * s + 1e4) * grid_words(E->len);
+  return grid < direct && rows < 24e9 && n * (n / 32 + s) < 2e9;
+}
+
+int get_grad_grid_work(pyiid_ctx *ctx, Layout *L, GradGridWork **out) {
+  if (!L->grad_grid) {
+    const int S = L->n_species;
+    std::vector<int> start(S, 0), count(S, 0), staged(S + 1, 0);
+    for (const int4 &t : L->tiles) count[t.w] += t.y;
+    for (int s = 1; s < S; ++s) start[s] = start[s - 1] + count[s - 1];
+    for (int s = 0; s < S; ++s)
+      staged[s + 1] = staged[s] + (count[s] + 31) / 32 * 32;
+    auto W = std::make_unique<GradGridWork>();
+    W->staged = staged[S];
+    std::vector<GradBlock> blocks;
+    std::vector<int2> cols;
+    long long total = 0;
+    for (int sa = 0; sa < S; ++sa)
+      for (int sb = 0; sb < S; ++sb) {
+        const int nc = (count[sb] + 31) / 32;
+        blocks.push_back(GradBlock{(int)total, count[sa] ? nc : 0, W->units,
+                                   start[sa], count[sa], start[sb], count[sb],
+                                   staged[sa], staged[sb]});
+        const long long end = total + (long long)nc * count[sa];
+        cols.push_back(make_int2((int)total, (int)end));
+        total = end;
+        if (nc) W->units += count[sa];
+      }
+    // F(Q): both orders of a species pair together
+    std::vector<KeyCols> keys;
+    std::vector<int> spair;
+    for (int sa = 0; sa < S; ++sa)
+      for (int sb = 0; sb <= sa; ++sb) {
+        const int p = sa * S + sb, q = sb * S + sa;
+        keys.push_back(KeyCols{cols[p].x, cols[p].y, p, sa == sb ? 0 : cols[q].x,
+                               sa == sb ? 0 : cols[q].y, q});
+        spair.push_back(sa * (sa + 1) / 2 + sb);
+      }
+    W->total = (int)total;
+    TRY(upload(ctx, &W->d_blocks, blocks));
+    TRY(upload(ctx, &W->d_key_cols, keys));
+    TRY(upload(ctx, &W->d_key_spair, spair));
+    TRY(upload(ctx, &W->d_cfg_keys,
+               std::vector<int4>{make_int4(0, 0, (int)keys.size(), 0)}));
+    L->grad_grid = std::move(W);
+  }
+  *out = L->grad_grid.get();
+  return PYIID_OK;
+}
+
+// grad (and fq, unless nullptr) of one configuration (grad_grid.cuh).
+int run_grad_grid(pyiid_ctx *ctx, Layout *L, const float *positions,
+                  const float *d_ftab, const double *d_na, int n_bins,
+                  double qbin, int kbo, float *fq, float *grad) {
+  const GradTransformEntry *E = grad_transform_for(n_bins);
+  GradGridWork *W;
+  TRY(get_grad_grid_work(ctx, L, &W));
+  PhaseGrid *G;
+  const int m = 2 * E->len, S = L->n_species, n_keys = S * (S + 1) / 2;
+  TRY(get_phase_grid(ctx, n_bins, m, true, &G));
+  const int n_ctas = ctx->n_sms, max_warps = kSpreadWarps * n_ctas;
+  const int row_words = grid_words(m / 2);
+  const size_t n_rows = (size_t)W->units + max_warps;
+  void *p;
+  TRY(ensure(ctx, "gg_rows", n_rows * 3 * row_words * sizeof(float), &p));
+  float *rows = static_cast<float *>(p);
+  TRY(ensure(ctx, "gg_rows2", n_rows * 3 * row_words * sizeof(float), &p));
+  float *rows2 = static_cast<float *>(p);
+  TRY(ensure(ctx, "gg_flag", n_rows * sizeof(int), &p));
+  int *flag = static_cast<int *>(p);
+  TRY(ensure(ctx, "gg_parts", W->units * sizeof(int2), &p));
+  int2 *parts = static_cast<int2 *>(p);
+  HistRows frows;
+  TRY(hist_rows(ctx, "ggf", S * S, row_words, &frows));
+  TRY(ensure(ctx, "gg_fsum",
+             (size_t)n_keys * fq_sum_floats(m) * sizeof(float), &p));
+  float *fsum = static_cast<float *>(p);
+  TRY(ensure(ctx, "gg_ext", sizeof(int), &p));
+  int *ext = static_cast<int *>(p);
+  const GridScale gs = grid_scale(qbin, m);
+  TRY(ensure(ctx, "gg_atoms", 2 * (size_t)W->staged * sizeof(float4), &p));
+  float4 *atoms = static_cast<float4 *>(p);
+  TRY(ensure(ctx, "coef", (size_t)S * S * n_bins * sizeof(float), &p));
+  float *coef = static_cast<float *>(p);
+  grad_prep_kernel<<<1 + std::min(n_ctas, 1 + std::max(W->staged, S * S * n_bins) /
+                                                  kPrepBlock),
+                     kPrepBlock, 0, ctx->stream>>>(
+      positions, L->d_perm, L->total, W->d_blocks, S, gs.hi, m / 2, ext, d_na,
+      d_ftab, n_bins, coef, atoms);
+  LAUNCH_CHECK(ctx);
+  const float near_r = (float)(kNearPhase / (n_bins * qbin));
+  const float near_scale = (float)(n_bins * qbin);
+  (fq ? grad_spread_kernel<true> : grad_spread_kernel<false>)<<<
+      n_ctas, 32 * kSpreadWarps, kSpreadSmem, ctx->stream>>>(
+      atoms, W->d_blocks, W->total, ext, gs, near_r, near_scale, G->d_taps, rows, rows2, flag, parts, frows);
+  LAUNCH_CHECK(ctx);
+  // (one more layer of CTAs sums F's histograms beside the transforms)
+  E->k<<<dim3(L->total, fq ? 4 : 3), E->threads, grad_transform_smem(E->len),
+         ctx->stream>>>(rows, rows2, flag, parts, W->d_blocks, S, ext,
+                        L->d_perm, G->d_tw, G->d_pr, coef, n_bins, kbo,
+                        (float)qbin, 1.0f / (float)n_bins, grad,
+                        FqReduceArgs{frows, W->d_key_cols, n_keys, W->total,
+                                     fsum});
+  LAUNCH_CHECK(ctx);
+  if (!fq) return PYIID_OK;
+  fq_grid_finish_kernel<<<dim3((n_bins + 31) / 32, 1), 32 * kFqDftWarps,
+                          fq_dft_float4(m) * sizeof(float4), ctx->stream>>>(
+      fsum, W->d_cfg_keys, W->d_key_spair, L->d_spair, d_ftab, d_na,
+      G->d_inv_phi, m, 1.0f / (float)m, n_bins, kbo, qbin,
+      1.0f / (float)n_bins, fq, nullptr);
   LAUNCH_CHECK(ctx);
   return PYIID_OK;
 }
@@ -1310,10 +1573,7 @@ int pyiid_destroy(pyiid_ctx *ctx) {
   for (auto &L : ctx->layouts) free_layout(L.get());
   for (auto &T : ctx->tmats) free_tmatrix(T.get());
   for (auto &N : ctx->nas) cudaFree(N->d_na);
-  for (auto &G : ctx->grids) {
-    cudaFree(G->d_taps);
-    cudaFree(G->d_inv_phi);
-  }
+  for (auto &G : ctx->grids) free_phase_grid(G.get());
   cudaFree(ctx->d_status);
   delete ctx;
   return PYIID_OK;
@@ -1390,6 +1650,9 @@ int pyiid_grad_fq(pyiid_ctx *ctx, const float *positions,
   TRY(get_na(ctx, L, scatter, n_bins, &d_na));
   const int kbo = std::min(k_begin, n_bins);
   const int kb0 = kbo & ~1;
+  if (kbo < n_bins && grad_on_grid(L, n_bins, false))
+    return run_grad_grid(ctx, L, positions, d_ftab, d_na, n_bins, qbin, kbo,
+                         nullptr, grad);
   void *p;
   TRY(ensure(ctx, "coef",
              (size_t)n_species * n_species * n_bins * sizeof(float), &p));
@@ -1468,6 +1731,9 @@ int pyiid_fq_grad(pyiid_ctx *ctx, const float *positions,
   const int kbo = std::min(k_begin, n_bins);
   const int kb0 = kbo & ~1;
   const int n_tiles = (int)L->tiles.size();
+  if (kbo < n_bins && grad_on_grid(L, n_bins, true))
+    return run_grad_grid(ctx, L, positions, d_ftab, d_na, n_bins, qbin, kbo,
+                         fq, grad);
   double *fpart = nullptr;
   int n_split = 1;
   if (n_atoms > 0 && kb0 < n_bins) {

@@ -38,23 +38,21 @@ struct GridSeg {
   int a0, na, b0, key;
 };
 
-// Cells that the distances of a configuration can reach: ext[c] = the cell
-// of twice the largest distance from the centre of the atoms' box (at most
-// M/2, where the period folds).  One CTA per configuration.
-__global__ void __launch_bounds__(256)
-    grid_extent_kernel(const float *__restrict__ pos,
-                       const int *__restrict__ offsets,
-                       const int4 *__restrict__ cfg_keys, float scale, int half,
-                       int *__restrict__ ext) {
-  __shared__ float red[8][6];
-  __shared__ float mx[8];
-  const int c = cfg_keys[blockIdx.x].x;
-  const int i0 = offsets[c], i1 = offsets[c + 1];
+// Cells that the distances of the atoms [i0, i1) can reach: the cell of
+// twice the largest distance from the centre of their box (at most M/2,
+// where the period folds).  One CTA, at most 1,024 threads.
+__device__ __forceinline__ void grid_extent(const float *__restrict__ pos,
+                                            int i0, int i1, float scale,
+                                            int half, int *__restrict__ ext) {
+  __shared__ float red[32][6];
+  __shared__ float mx[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n_warps = blockDim.x >> 5;
   float lo[3], hi[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) lo[d] = 3e38f, hi[d] = -3e38f;
-  for (int i = i0 + threadIdx.x; i < i1; i += 256) {
+#pragma unroll 4
+  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       const float x = pos[3 * (size_t)i + d];
@@ -75,12 +73,13 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     float l = red[0][d], h = red[0][3 + d];
-    for (int w = 1; w < 8; ++w)
+    for (int w = 1; w < n_warps; ++w)
       l = fminf(l, red[w][d]), h = fmaxf(h, red[w][3 + d]);
     mid[d] = 0.5f * l + 0.5f * h;
   }
   float r2 = 0.f;
-  for (int i = i0 + threadIdx.x; i < i1; i += 256) {
+#pragma unroll 4
+  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
     const float x = pos[3 * (size_t)i] - mid[0];
     const float y = pos[3 * (size_t)i + 1] - mid[1];
     const float z = pos[3 * (size_t)i + 2] - mid[2];
@@ -91,12 +90,24 @@ __global__ void __launch_bounds__(256)
   if (lane == 0) mx[warp] = r2;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < 8; ++w) r2 = fmaxf(r2, mx[w]);
-    // a millionth more for the roundings here; cells are floor(u)
+    for (int w = 1; w < n_warps; ++w) r2 = fmaxf(r2, mx[w]);
+    // a millionth more for the roundings here; cells are floor(u).  NaN
+    // positions are not seen (their pairs have no cell); with infinite ones
+    // every cell is kept
     const float u = 2.000002f * sqrtf(r2) * scale + 2.0f;
     const bool fin = fabsf(mid[0] + mid[1] + mid[2]) < 3e38f;
-    ext[blockIdx.x] = fin && u < (float)half ? (int)u : half;
+    *ext = fin && u < (float)half ? (int)u : half;
   }
+}
+
+// ext[c] of the configurations on the grid, one CTA each
+__global__ void __launch_bounds__(1024)
+    grid_extent_kernel(const float *__restrict__ pos,
+                       const int *__restrict__ offsets,
+                       const int4 *__restrict__ cfg_keys, float scale, int half,
+                       int *__restrict__ ext) {
+  const int c = cfg_keys[blockIdx.x].x;
+  grid_extent(pos, offsets[c], offsets[c + 1], scale, half, ext + blockIdx.x);
 }
 
 // How the spreading kernel's warps share the columns, which depends on the
@@ -106,32 +117,87 @@ struct SpreadPlan {
   int used, per_cta, n;
 };
 
+constexpr int kSpreadWarps = 16;               // at most, per CTA
+constexpr int kSpreadSmem = 224 * 1024;        // of a CTA
+constexpr int kSpreadStage = 32 * 32;          // of a warp, beside its cells
+
+struct PlanShape {
+  int cell_bytes;  // shared memory per cell and warp
+  int min_cols;    // columns that make a warp worth its flush
+};
+
 // (all threads of a CTA call this; s: shared scratch of 32 ints)
 __device__ __forceinline__ SpreadPlan spread_plan(const int *__restrict__ ext,
                                                   int n_cfgs, int n_ctas,
-                                                  int max_warps, int warp_bytes,
-                                                  int cell_bytes, int smem,
-                                                  int total, int *s) {
+                                                  PlanShape sh, int total,
+                                                  int *s) {
   int u = 0;
-  for (int i = threadIdx.y * blockDim.x + threadIdx.x; i < n_cfgs;
-       i += blockDim.x * blockDim.y)
-    u = max(u, ext[i]);
-  const int t = threadIdx.y * blockDim.x + threadIdx.x;
+  const int t = threadIdx.x;
+  for (int i = t; i < n_cfgs; i += blockDim.x) u = max(u, ext[i]);
   u = __reduce_max_sync(0xffffffffu, u);
   if ((t & 31) == 0) s[t >> 5] = u;
   __syncthreads();
-  const int nw = (blockDim.x * blockDim.y + 31) >> 5;
+  const int nw = (blockDim.x + 31) >> 5;
   for (int w = 0; w < nw; ++w) u = max(u, s[w]);
   SpreadPlan p;
   p.used = u;
-  // as many warps as have room for a histogram, each with at least eight
-  // columns (its flush costs about four)
-  p.per_cta = min(max_warps, smem / (warp_bytes + cell_bytes * grid_words(u)));
+  // as many warps as have room for a histogram
+  p.per_cta = min(kSpreadWarps,
+                  kSpreadSmem / (kSpreadStage + sh.cell_bytes * grid_words(u)));
   // the four schedulers of the SM get equal numbers of warps
   if (p.per_cta > 4) p.per_cta &= ~3;
-  p.per_cta = max(1, min(p.per_cta, (total + 8 * n_ctas - 1) / (8 * n_ctas)));
-  p.n = p.per_cta * n_ctas;
+  const int per = sh.min_cols * n_ctas;
+  p.per_cta = max(1, min(p.per_cta, (total + per - 1) / per));
+  p.n = min(p.per_cta * n_ctas, total);  // no warp without a column
   return p;
+}
+
+// Where the partial histograms of a launch go.  A warp that leaves a key
+// writes its row at slot warp + key (flag 1).  What its last key holds stays
+// in shared memory until the CTA is done: if all its warps end on one key,
+// their sum is one row of the CTA (cta[b].x = the key, flag 0 at the slots),
+// sixteen times less to write and to add up; else each writes its own.
+// cta[b].y: whether any warp of CTA b wrote a row of its own.
+struct HistRows {
+  float *rows;  // [n_ctas] rows of the CTAs, then those of the slots
+  int *flag;    // [slots]
+  int2 *cta;    // [n_ctas]
+  int n_ctas, row_words;
+  __device__ __forceinline__ float *cta_row(int b) const {
+    return rows + (size_t)b * row_words;
+  }
+  __device__ __forceinline__ float *warp_row(int slot) const {
+    return rows + ((size_t)n_ctas + slot) * row_words;
+  }
+};
+
+// End of a spreading CTA (all threads call it): whether this warp has to
+// write its last key itself.  Else, if s[0] >= 0, the CTA's warps 0 .. s[1]-1
+// are to be summed into its row.  s: shared scratch of 32 ints.
+__device__ __forceinline__ bool finish_rows(const HistRows &out, int wi,
+                                            int key, bool alone, int *s) {
+  __syncthreads();
+  const int warp = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) s[warp] = key * 2 + alone;
+  __syncthreads();
+  // (s[w] is negative for warps without work, which come last)
+  const int n_warps = blockDim.x >> 5;
+  int n = 0, first = s[0] >> 1;
+  bool same = true, own = false;
+  for (; n < n_warps && s[n] >= 0; ++n) {
+    same &= (s[n] >> 1) == first;
+    own |= s[n] & 1;
+  }
+  __syncthreads();
+  const bool join = n > 0 && same;
+  if (threadIdx.x == 0) {
+    out.cta[blockIdx.x] = make_int2(join ? first : -1, own || (n > 0 && !same));
+    s[0] = join ? first : -1;
+    s[1] = n;
+  }
+  if (join && key >= 0 && (threadIdx.x & 31) == 0) out.flag[wi + key] = 0;
+  __syncthreads();
+  return key >= 0 && !join;
 }
 
 // One CTA per SM.  Each warp has a private histogram (no atomics, a fixed
@@ -155,11 +221,9 @@ __device__ __forceinline__ SpreadPlan spread_plan(const int *__restrict__ ext,
 // 64 x 1,000 atoms at 330 bins: 253 us (fq_pair3_kernel 1,451); 256 alloys of
 // 55 to 2,000 atoms at 500 bins 1.45 ms (11.5); 10,007 atoms at 1,500 bins
 // 0.60 ms (9.5).
-constexpr int kSpreadWarps = 16;
 constexpr int kSpreadSlots = 8;
 constexpr int kSpreadCols = 2;
-constexpr int kSpreadSmem = 224 * 1024;
-constexpr int kSpreadStage = 32 * 32;  // bytes of 32 staged atoms
+constexpr PlanShape kFqPlan{4 * kSpreadSlots, 8};
 __global__ void __launch_bounds__(32 * kSpreadWarps)
     fq_spread_kernel(const float *__restrict__ pos,
                      const int *__restrict__ perm,
@@ -167,18 +231,16 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
                      const int *__restrict__ seg_begin, int n_segs, int total,
                      const int *__restrict__ ext, int n_cfgs, GridScale gs,
                      float near_r, float near_scale,
-                     const float *__restrict__ taps, int row_words,
-                     float *__restrict__ rows) {
+                     const float *__restrict__ taps, HistRows out) {
   extern __shared__ float4 smem4[];
   __shared__ int splan[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const SpreadPlan plan =
-      spread_plan(ext, n_cfgs, gridDim.x, kSpreadWarps, kSpreadStage,
-                  4 * kSpreadSlots, kSpreadSmem, total, splan);
+      spread_plan(ext, n_cfgs, gridDim.x, kFqPlan, total, splan);
   const int wi = blockIdx.x * plan.per_cta + warp;
   const int c0 = (int)((long long)wi * total / plan.n);
   const int c1 = (int)((long long)(wi + 1) * total / plan.n);
-  if (warp >= plan.per_cta || c0 >= c1) return;
+  const bool works = warp < plan.per_cta && wi < plan.n;
   const int words = grid_words(plan.used);
   float4 *stage = smem4 + warp * (kSpreadStage / 16 + 2 * words);
   float4 *hist4 = stage + kSpreadStage / 16;  // [word][slot]
@@ -188,7 +250,7 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
 #pragma unroll
   for (int i = 0; i < kTapCoef; ++i)
     cf[i] = make_float2(taps[tp * kTapCoef + i], taps[(tp + 4) * kTapCoef + i]);
-  for (int i = lane; i < 2 * words; i += 32)
+  for (int i = lane; works && i < 2 * words; i += 32)
     hist4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   __syncwarp();
   // the row that holds column c0
@@ -202,24 +264,32 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
   }
   // tap p of cell j is cell j - 3 + p
   float *const base = hist + (8 + tp) * kSpreadSlots + slot;
+  auto word = [](const float4 *h, int i) {  // the eight copies of word i
+    const float4 v = h[2 * i], w = h[2 * i + 1];
+    return ((v.x + v.y) + (v.z + v.w)) + ((w.x + w.y) + (w.z + w.w));
+  };
   auto flush = [&](int key) {
     __syncwarp();
-    float *out = rows + (size_t)(wi + key) * row_words;
+    float *row = out.warp_row(wi + key);
     for (int i = lane; i < words; i += 32) {
-      const float4 v = hist4[2 * i], w = hist4[2 * i + 1];
-      out[i] = ((v.x + v.y) + (v.z + v.w)) + ((w.x + w.y) + (w.z + w.w));
+      row[i] = word(hist4, i);
       hist4[2 * i] = make_float4(0.f, 0.f, 0.f, 0.f);
       hist4[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    if (lane == 0) out.flag[wi + key] = 1;
     __syncwarp();
   };
   int cur = -1;
+  bool alone = false;
   int c = c0;
-  for (int sgi = lo; c < c1; ++sgi) {
+  for (int sgi = lo; works && c < c1; ++sgi) {
     const GridSeg sg = segs[sgi];
     const int begin = seg_begin[sgi], end = min(seg_begin[sgi + 1], c1);
     if (sg.key != cur) {
-      if (cur >= 0) flush(cur);
+      if (cur >= 0) {
+        flush(cur);
+        alone = true;
+      }
       cur = sg.key;
     }
     // (lanes past the tile count no pair: no b is below 0)
@@ -328,36 +398,60 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
     }
     c = end;
   }
-  flush(cur);
+  if (finish_rows(out, wi, works ? cur : -1, alone, splan))
+    flush(cur);
+  else if (splan[0] >= 0)
+    for (int i = threadIdx.x; i < words; i += blockDim.x) {
+      float s = 0.f;
+      for (int w = 0; w < splan[1]; ++w)
+        s += word(smem4 + w * (kSpreadStage / 16 + 2 * words) +
+                      kSpreadStage / 16,
+                  i);
+      out.cta_row(blockIdx.x)[i] = s;
+    }
 }
+
+// The partial histograms of a key: those of columns [c0, c1) at slot offset
+// s0, and for ordered species pairs of [d0, d1) at s1.
+struct KeyCols {
+  int c0, c1, s0, d0, d1, s1;
+};
 
 // Sums the partial histograms of a key and folds them for the transform.
 // With j' = M/2 - j, sin(2 pi k j'/M) is -(-1)^k sin(2 pi k j/M), so even
 // bins need G-_j = H_j - H_j' and odd bins G+_j = H_j + H_j' for j <= M/4
-// only: out[key][j] = (G-_j, G+_j), then the power sums.  The slots follow
-// from the plan of the spreading kernel, made again here from its arguments.
-// Threads (x: cell, y: a share of the slots) add in float pairs.
-__global__ void fq_grid_reduce_kernel(const float *__restrict__ rows,
-                                      const int2 *__restrict__ key_cols,
-                                      const int *__restrict__ ext, int n_cfgs,
-                                      int n_ctas, int total, int m,
-                                      int row_words, float *__restrict__ out) {
-  extern __shared__ float sred[];  // [4][blockDim.y][32]
-  __shared__ int splan[32];
+// only: out[j] = (G-_j, G+_j), then the power sums.  The slots follow from
+// the plan of the spreading kernel, made again here from its arguments.
+// (A key's columns are contiguous, so of the CTAs that hold them only the
+// first and the last can hold other keys too.)
+// One CTA does cells [nx block, nx (block + 1)); thread (x: cell, y: every
+// ny-th row) adds in float pairs, then the thread rows are added in order.
+// sred: 4 nx ny floats, splan: 32 ints of shared memory.
+__device__ __forceinline__ void fq_grid_reduce(
+    const HistRows &in, const KeyCols &kc, const int *__restrict__ ext,
+    int n_cfgs, PlanShape shape, int total, int m, int block, int nx, int ny,
+    float *__restrict__ out, float *sred, int *splan) {
+  const int tid = threadIdx.x;
   const SpreadPlan plan =
-      spread_plan(ext, n_cfgs, n_ctas, kSpreadWarps, kSpreadStage,
-                  4 * kSpreadSlots, kSpreadSmem, total, splan);
-  const int2 kc = key_cols[blockIdx.y];  // columns [x, y) of the key
-  // warps of column x and of column y - 1
+      spread_plan(ext, n_cfgs, in.n_ctas, shape, total, splan);
+  // the warp of a column
   auto warp_of = [&](long long col) {
     long long i = col * plan.n / total;
     while (i > 0 && i * total / plan.n > col) --i;
     while ((i + 1) * total / plan.n <= col) ++i;
     return (int)i;
   };
-  const int w0 = warp_of(kc.x), n_rows = warp_of(kc.y - 1) - w0 + 1;
+  __syncthreads();  // splan has been read
+  if (tid < 2) {
+    const int c0 = tid ? kc.d0 : kc.c0, c1 = tid ? kc.d1 : kc.c1;
+    const int w0 = c0 < c1 ? warp_of(c0) : 0;
+    splan[2 * tid] = w0;
+    splan[2 * tid + 1] = c0 < c1 ? warp_of(c1 - 1) + 1 : w0;
+  }
+  __syncthreads();
   const int quarter = m / 4, half = m / 2;
-  const int j = blockIdx.x * 32 + threadIdx.x;
+  const int tx = tid % nx, ty = tid / nx;
+  const int j = block * nx + tx;
   // the cells that meet in (G-_j, G+_j): j, its mirror images at 0 and M/2
   float hs = 0.f, hc = 0.f, ms = 0.f, mc = 0.f;
   const bool on = j <= quarter, near = j > quarter && j <= quarter + kNearTerms;
@@ -367,59 +461,112 @@ __global__ void fq_grid_reduce_kernel(const float *__restrict__ rows,
     c = __fsub_rn(y, __fsub_rn(t, s));
     s = t;
   };
-  if (on || near) {
+  if (ty < ny && (on || near)) {
     const int j1 = half - j, last = plan.used + 4;
-    for (int i = threadIdx.y; i < n_rows; i += blockDim.y) {
-      const float *r = rows + (size_t)(w0 + blockIdx.y + i) * row_words;
+    auto take = [&](const float *r) {
       if (near) {
         add(r[j - quarter - 1], hs, hc);
-      } else {
-        // cells below 0 and above M/2 are images with the opposite sign
-        r += kGridCell0;
-        float x = j <= last ? r[j] : 0.f, y = j1 <= last ? r[j1] : 0.f;
-        if (j >= 1 && j <= 3) x -= r[-j];
-        if (j >= 1 && half + j <= last) y -= r[half + j];
-        add(x, hs, hc);
-        add(y, ms, mc);
+        return;
+      }
+      r += kGridCell0;
+      // cells below 0 and above M/2 are images with the opposite sign
+      float x = j <= last ? r[j] : 0.f, y = j1 <= last ? r[j1] : 0.f;
+      if (j >= 1 && j <= 3) x -= r[-j];
+      if (j >= 1 && half + j <= last) y -= r[half + j];
+      add(x, hs, hc);
+      add(y, ms, mc);
+    };
+    auto own = [&](int w, int key) {
+      if (in.cta[w / plan.per_cta].y && in.flag[w + key])
+        take(in.warp_row(w + key));
+    };
+    for (int part = 0; part < 2; ++part) {
+      const int w0 = splan[2 * part], w1 = splan[2 * part + 1];
+      if (w0 == w1) continue;
+      const int key = part ? kc.s1 : kc.s0;
+      const int b0 = w0 / plan.per_cta, b1 = (w1 - 1) / plan.per_cta;
+#pragma unroll 2
+      for (int b = b0 + ty; b <= b1; b += ny)
+        if (in.cta[b].x == key) take(in.cta_row(b));
+      // warps that wrote their own row
+      {
+        const int e0 = min(w1, (b0 + 1) * plan.per_cta);
+        for (int w = w0 + ty; w < e0; w += ny) own(w, key);
+        for (int w = max(e0, b1 * plan.per_cta) + ty; w < w1; w += ny)
+          own(w, key);
       }
     }
   }
-  float *sh = sred + threadIdx.y * 32 + threadIdx.x;
-  const int st = blockDim.y * 32;
-  sh[0] = hs;
-  sh[st] = hc;
-  sh[2 * st] = ms;
-  sh[3 * st] = mc;
-  __syncthreads();
-  if (threadIdx.y != 0 || !(on || near)) return;
-  for (int y = 1; y < (int)blockDim.y; ++y) {
-    add(sh[y * 32], hs, hc);
-    hc += sh[st + y * 32];
-    add(sh[2 * st + y * 32], ms, mc);
-    mc += sh[3 * st + y * 32];
+  const int st = nx * ny;
+  if (ty < ny) {
+    float *sh = sred + tid;
+    sh[0] = hs;
+    sh[st] = hc;
+    sh[2 * st] = ms;
+    sh[3 * st] = mc;
   }
-  float *o = out + (size_t)blockIdx.y * (2 * (quarter + 1) + 8);
+  __syncthreads();
+  if (ty != 0 || !(on || near)) return;
+  for (int y = 1; y < ny; ++y) {
+    const float *sh = sred + y * nx + tx;
+    add(sh[0], hs, hc);
+    hc += sh[st];
+    add(sh[2 * st], ms, mc);
+    mc += sh[3 * st];
+  }
   if (near) {
-    o[2 * (quarter + 1) + (j - quarter - 1)] = hs + hc;
+    out[2 * (quarter + 1) + (j - quarter - 1)] = hs + hc;
   } else {
     const bool mid = j == quarter;  // its own mirror image
-    o[2 * j] = j == 0 || mid ? 0.f : (hs - ms) + (hc - mc);
-    o[2 * j + 1] = j == 0 ? 0.f : mid ? hs + hc : (hs + ms) + (hc + mc);
+    out[2 * j] = j == 0 || mid ? 0.f : (hs - ms) + (hc - mc);
+    out[2 * j + 1] = j == 0 ? 0.f : mid ? hs + hc : (hs + ms) + (hc + mc);
   }
 }
 
-// F(Q) of the configurations on the grid.  CTA = (32 bins, configuration),
-// lane = bin k; the warps share the cells j in blocks of 17 around an
-// accurate centre sin(theta_k jc), from which the others are one rotation by
-// n theta_k, n <= 8.  About 6 instructions per (bin, cell), FP32 issue bound;
-// block sums are added in float pairs, the rest is FP64 per bin.
-constexpr int kFqDftWarps = 8;
-constexpr int kFqDftReach = 8;
-// floats of shared memory: (G-, G+) up to a whole round of blocks past M/4
-__host__ __device__ constexpr int fq_dft_floats(int m) {
-  return 2 * (m / 4 + 2 + kFqDftWarps * (2 * kFqDftReach + 1)) + 8;
+// floats of one key's sums (even, so that the pairs stay 8-byte aligned)
+__host__ __device__ constexpr int fq_sum_floats(int m) {
+  return 2 * (m / 4 + 1) + 8;
 }
-__global__ void __launch_bounds__(32 * kFqDftWarps)
+__host__ __device__ constexpr int fq_reduce_blocks(int m, int nx) {
+  return (m / 4 + kNearTerms) / nx + 1;
+}
+
+__global__ void fq_grid_reduce_kernel(HistRows in,
+                                      const KeyCols *__restrict__ key_cols,
+                                      const int *__restrict__ ext, int n_cfgs,
+                                      PlanShape shape, int total, int m, int nx,
+                                      int ny, float *__restrict__ out) {
+  extern __shared__ float sred[];
+  __shared__ int splan[32];
+  fq_grid_reduce(in, key_cols[blockIdx.y], ext, n_cfgs, shape, total, m,
+                 blockIdx.x, nx, ny,
+                 out + (size_t)blockIdx.y * fq_sum_floats(m), sred, splan);
+}
+
+// F(Q) of the configurations on the grid.  CTA = (32 bins, configuration),
+// lane = bin k.  sum_j G_j sin(theta_k j) goes in blocks of 2 R + 1 cells
+// around a centre c: sin(theta (c +- n)) = sin(theta c) cos(theta n) +-
+// cos(theta c) sin(theta n), so a block is
+//   sin(theta c) sum_n cos(theta n) (G_c+n + G_c-n)
+//   + cos(theta c) sum_n sin(theta n) (G_c+n - G_c-n)
+// with the sums and differences formed once per CTA as the cells are staged
+// in shared memory, and the rotations of n <= R kept in registers: 1.5
+// instructions per (bin, cell) and one accurate sine and cosine per block.
+// The warps share the blocks; block sums are added in float pairs, the rest
+// is FP64 per bin.  Four keys at a time, so that their copies and barriers
+// are waited for once.
+constexpr int kFqDftWarps = 8;
+constexpr int kFqDftReach = 16;
+constexpr int kFqDftKeys = 4;
+__host__ __device__ constexpr int fq_dft_blocks(int m) {
+  return (m / 4 + 2 * kFqDftReach) / (2 * kFqDftReach + 1);
+}
+// float4 of shared memory, per key: (sum, difference) of even bins, then of
+// odd ones
+__host__ __device__ constexpr int fq_dft_float4(int m) {
+  return kFqDftKeys * fq_dft_blocks(m) * (kFqDftReach + 1);
+}
+__global__ void __launch_bounds__(32 * kFqDftWarps, 3)
     fq_grid_finish_kernel(const float *__restrict__ hsum,
                           const int4 *__restrict__ cfg_keys,
                           const int *__restrict__ key_spair,
@@ -427,57 +574,88 @@ __global__ void __launch_bounds__(32 * kFqDftWarps)
                           const float *__restrict__ ftab,
                           const double *__restrict__ na,
                           const double *__restrict__ inv_phi, int m,
-                          float inv_m, int n_bins, int kb_out, double dq, float near_unit,
-                          float *__restrict__ fq, double *__restrict__ fq_raw) {
-  constexpr int R = kFqDftReach;
-  extern __shared__ float sh[];  // the key's folded histogram, zero-padded
-  __shared__ float red[2][kFqDftWarps][32];
+                          float inv_m, int n_bins, int kb_out, double dq,
+                          float near_unit, float *__restrict__ fq,
+                          double *__restrict__ fq_raw) {
+  constexpr int R = kFqDftReach, B = 2 * R + 1, Q = kFqDftKeys;
+  extern __shared__ float4 sh4[];
+  __shared__ float red[Q][2][kFqDftWarps][32];
+  __shared__ double terms[Q][32];
   const int4 ck = cfg_keys[blockIdx.y];  // configuration, first key, keys
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int k = min((int)(blockIdx.x * 32 + lane), n_bins - 1);
-  const int quarter = m / 4;
-  float sn[R], cn[R];
+  const int quarter = m / 4, blocks = fq_dft_blocks(m);
+  // e^{i theta n}: each fourth from the table's accuracy, the rest one
+  // product each
+  float sn[R + 1], cn[R + 1];
+  sn[0] = 0.f;
+  cn[0] = 1.f;
 #pragma unroll
-  for (int n = 0; n < R; ++n)
-    sincos_turn((int)((unsigned)(n + 1) * (unsigned)k % (unsigned)m), m, inv_m,
-                sn[n], cn[n]);
+  for (int n = 1; n <= R; ++n) {
+    const int r = n & 3;
+    if (r == 0 || n < 4) {
+      sincos_turn((int)((unsigned)n * (unsigned)k % (unsigned)m), m, inv_m,
+                  sn[n], cn[n]);
+    } else {
+      sn[n] = fmaf(sn[n - r], cn[r], cn[n - r] * sn[r]);
+      cn[n] = fmaf(cn[n - r], cn[r], -sn[n - r] * sn[r]);
+    }
+  }
   double sum = 0.0;
-  for (int q = 0; q < ck.z; ++q) {
-    const float *h = hsum + (size_t)(ck.y + q) * (2 * (quarter + 1) + 8);
+  for (int q0 = 0; q0 < ck.z; q0 += Q) {
+    const int nq = min(Q, ck.z - q0), per = blocks * (R + 1);
+    const float *hq = hsum + (size_t)(ck.y + q0) * fq_sum_floats(m);
     __syncthreads();
-    for (int i = threadIdx.x; i < fq_dft_floats(m) - 8; i += blockDim.x)
-      sh[i] = i < 2 * (quarter + 1) ? h[i] : 0.f;
-    __syncthreads();
-    const float *hk = sh + (k & 1);
-    float s = 0.f, c = 0.f;
-    for (int j0 = 1 + warp * (2 * R + 1); j0 <= quarter;
-         j0 += kFqDftWarps * (2 * R + 1)) {
-      float sc, cc;
-      sincos_turn((int)((unsigned)k * (unsigned)(j0 + R) % (unsigned)m), m,
-                  inv_m, sc, cc);
-      const float *hj = hk + 2 * (j0 + R);
-      float blk = sc * hj[0];
-#pragma unroll
-      for (int n = 1; n <= R; ++n) {
-        const float u = sc * cn[n - 1], v = cc * sn[n - 1];
-        blk = fmaf(u + v, hj[2 * n], blk);
-        blk = fmaf(u - v, hj[-2 * n], blk);
-      }
-      const float y = __fadd_rn(blk, c);
-      const float t = __fadd_rn(s, y);
-      c = __fsub_rn(y, __fsub_rn(t, s));
-      s = t;
+    for (int i = threadIdx.x; i < nq * per; i += blockDim.x) {
+      const int q = i / per, b = (i - q * per) / (R + 1);
+      const int n = i - q * per - b * (R + 1);
+      const float *h = hq + (size_t)q * fq_sum_floats(m);
+      const int jp = 1 + b * B + R + n, jm = 1 + b * B + R - n;
+      float2 p = make_float2(0.f, 0.f), o = p;
+      if (jp <= quarter) p = *reinterpret_cast<const float2 *>(h + 2 * jp);
+      if (n > 0 && jm <= quarter)
+        o = *reinterpret_cast<const float2 *>(h + 2 * jm);
+      sh4[i] = make_float4(p.x + o.x, p.x - o.x, p.y + o.y, p.y - o.y);
     }
     __syncthreads();
-    red[0][warp][lane] = s;
-    red[1][warp][lane] = c;
+    for (int q = 0; q < nq; ++q) {
+      const float2 *hk =
+          reinterpret_cast<const float2 *>(sh4 + q * per) + (k & 1);
+      float s = 0.f, c = 0.f;
+      // (the warps take turns at who gets one block more)
+      for (int b = (warp + q * blocks) % kFqDftWarps; b < blocks;
+           b += kFqDftWarps) {
+        float sc, cc;
+        sincos_turn(
+            (int)((unsigned)k * (unsigned)(1 + b * B + R) % (unsigned)m), m,
+            inv_m, sc, cc);
+        float u = 0.f, v = 0.f;
+#pragma unroll
+        for (int n = 0; n <= R; ++n) {
+          const float2 x = hk[2 * (b * (R + 1) + n)];
+          u = fmaf(cn[n], x.x, u);
+          v = fmaf(sn[n], x.y, v);
+        }
+        const float y = __fadd_rn(fmaf(sc, u, cc * v), c);
+        const float t = __fadd_rn(s, y);
+        c = __fsub_rn(y, __fsub_rn(t, s));
+        s = t;
+      }
+      red[q][0][warp][lane] = s;
+      red[q][1][warp][lane] = c;
+    }
     __syncthreads();
-    if (warp == 0) {
-      double d = 0.0;
-      for (int w = 0; w < kFqDftWarps; ++w)
-        d += (double)red[0][w][lane] + (double)red[1][w][lane];
-      d *= inv_phi[k];
-      const float *nr = h + 2 * (quarter + 1);
+    if (warp < nq) {  // one key per warp
+      float s = 0.f, c = 0.f;
+      for (int w = 0; w < kFqDftWarps; ++w) {
+        const float y = __fadd_rn(red[warp][0][w][lane], c);
+        const float t = __fadd_rn(s, y);
+        c = __fsub_rn(y, __fsub_rn(t, s)) + red[warp][1][w][lane];
+        s = t;
+      }
+      double d = ((double)s + (double)c) * inv_phi[k];
+      const float *nr =
+          hq + (size_t)warp * fq_sum_floats(m) + 2 * (quarter + 1);
       if (nr[0] != 0.f) {
         // sum over near pairs of sin(Q r)/r = Q sum_n (-1)^n (Q r)^2n /
         // (2n + 1)!; nr[n] = sum (Q_max r)^2n
@@ -489,10 +667,13 @@ __global__ void __launch_bounds__(32 * kFqDftWarps)
                       z * (nr[3] / 5040.f + z * (nr[4] / 362880.f))));
         d += (double)k * dq * (double)v;
       }
-      const int2 ss = spair_species[key_spair[ck.y + q]];
-      sum += (double)ftab[ss.x * n_bins + k] * (double)ftab[ss.y * n_bins + k] *
-             d;
+      const int2 ss = spair_species[key_spair[ck.y + q0 + warp]];
+      terms[warp][lane] = (double)ftab[ss.x * n_bins + k] *
+                          (double)ftab[ss.y * n_bins + k] * d;
     }
+    __syncthreads();
+    if (warp == 0)
+      for (int q = 0; q < nq; ++q) sum += terms[q][lane];
   }
   const int kk = blockIdx.x * 32 + lane;
   if (warp != 0 || kk >= n_bins) return;

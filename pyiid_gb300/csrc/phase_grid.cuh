@@ -113,14 +113,15 @@ __device__ __forceinline__ PairDist pair_dist(const SplitAtom &a,
 }
 
 // Grid position of a distance: u = r scale as a float pair (uh, ul), taken
-// to [-M/2, M/2] by whole periods (the multiple of M is exact).
-__device__ __forceinline__ void grid_pos(const GridScale &g, float r, float rl,
-                                         float &uh, float &ul) {
+// to [-M/2, M/2] by n whole periods (the multiple of M is exact); returns n.
+__device__ __forceinline__ float grid_pos(const GridScale &g, float r,
+                                          float rl, float &uh, float &ul) {
   float p, e;
   two_prod(g.hi, r, p, e);
   ul = fmaf(g.hi, rl, fmaf(g.lo, r, e));
   const float n = rintf(p * g.inv_m);
   uh = __fmaf_rn(-n, g.m, p);
+  return n;
 }
 
 // sin and cos of 2 pi i / m for 0 <= i < m: the fraction 2 i / m is rounded

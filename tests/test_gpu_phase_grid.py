@@ -188,3 +188,85 @@ def test_mixed_batch_of_grid_and_direct_configurations(D):
             assert np.all(got == 0)
         else:
             assert rel(got[2:], fq64(p[a:b], sp[a:b], tab, qb)[2:]) <= TOL_F
+
+
+# tile and column edges (31 to 97 atoms); one to three elements; a period of Q
+# far shorter than the cluster (q step 0.7: pairs several periods apart, the
+# second sweep); the shortest and longest transforms and the first bin count
+# beyond them (2,008, the direct kernels); odd and zero k_begin; one bin
+# above k_begin; a cluster away from the origin
+@pytest.mark.parametrize('n,species,qb,nb,kb,shift', [
+    (32, 1, 0.05, 500, 2, 0.0),
+    (33, 1, 0.1, 187, 1, 30.0),
+    (65, 2, 0.1, 250, 0, 0.0),
+    (97, 3, 0.05, 301, 3, -200.0),
+    (64, 1, 0.7, 90, 0, 0.0),
+    (97, 2, 0.45, 250, 5, 0.0),
+    (40, 1, 0.012, 2007, 25, 0.0),
+    (40, 1, 0.012, 2008, 25, 0.0),
+    (64, 1, 0.05, 400, 399, 0.0),
+    (64, 1, 0.02, 1475, 25, 0.0),
+])
+def test_gradient_on_the_grid_matches_oracle(D, n, species, qb, nb, kb, shift):
+    pos, nums = cluster(n, n, species, shift)
+    sp, tab = tables(nums, qb, nb)
+    f, g = (t.cpu().numpy() for t in D.fq_grad(pos, sp, tab, qb, k_begin=kb))
+    g1 = D.grad_fq(pos, sp, tab, qb, k_begin=kb).cpu().numpy()
+    want_f = fq64(pos, sp, tab, qb)
+    want_g = O.grad_fq(pos, tab[sp], qb)
+    assert np.all(f[:kb] == 0)
+    assert np.all(g[:, :, :kb] == 0) and np.all(g1[:, :, :kb] == 0)
+    assert rel(f[kb:], want_f[kb:]) <= TOL_F
+    assert rel(g[:, :, kb:], want_g[:, :, kb:]) <= TOL_G
+    assert rel(g1[:, :, kb:], want_g[:, :, kb:]) <= TOL_G
+
+
+def test_gradient_on_the_grid_close_coincident_and_far_pairs(D):
+    """Pairs at tiny distances, under 0.1 A, beyond 128 A and several periods
+    apart, each against the oracle's rows; the rows of a coincident pair are
+    0 and F is 0, the others' rows stay."""
+    qb, nb = 0.3, 250
+    pos, nums = cluster(90, 19, 2)
+    pos[30] = pos[7] + np.float32([2e-4, 1e-4, 0])
+    pos[31] = pos[8] + np.float32([0.02, 0.03, 0.01])
+    pos[32] += np.float32([150.0, 0, 0])
+    sp, tab = tables(nums, qb, nb)
+    f, g = (t.cpu().numpy() for t in D.fq_grad(pos, sp, tab, qb))
+    want = O.grad_fq(pos, tab[sp], qb)
+    assert rel(f, fq64(pos, sp, tab, qb)) <= TOL_F
+    for a in (7, 30, 8, 31, 32, 50):
+        assert rel(g[a], want[a]) <= TOL_G, (a, rel(g[a], want[a]))
+    bad = pos.copy()
+    bad[30] = bad[7]
+    f, g = (t.cpu().numpy() for t in D.fq_grad(bad, sp, tab, qb))
+    assert np.all(f == 0) and np.all(g[[7, 30]] == 0)
+    want = O.grad_fq(bad, tab[sp], qb)
+    keep = np.setdiff1d(np.arange(90), [7, 30])
+    assert rel(g[keep], want[keep]) <= TOL_G
+
+
+def test_gradient_on_the_grid_under_capture(D):
+    """One element with more columns than warps, and three whose blocks end
+    inside a CTA's share of the columns: eager, repeated and graph-replayed
+    calls are bitwise equal, also into an output at an odd offset."""
+    import torch
+    for n, species in ((400, 1), (460, 3)):
+        pos, nums = cluster(n, n, species)
+        sp, tab = tables(nums, 0.05, 300)
+        p = torch.as_tensor(pos.astype(np.float32), device='cuda')
+        f, g = D.fq_grad(p, sp, tab, 0.05, 1)
+        big = torch.full((n * 900 + 4,), float('nan'), device='cuda')
+        out = big[1:1 + n * 900].view(n, 3, 300)
+        f2 = torch.empty_like(f)
+        D.fq_grad(p, sp, tab, 0.05, 1, out_fq=f2, out_grad=out)
+        assert torch.equal(f2, f) and torch.equal(out, g)
+        assert torch.isnan(big[0]) and torch.isnan(big[-3:]).all()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            D.fq_grad(p, sp, tab, 0.05, 1, out_fq=f2, out_grad=out)
+        out.zero_()
+        f2.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(f2, f) and torch.equal(out, g)
+        assert rel(f.cpu().numpy()[1:], fq64(pos, sp, tab, 0.05)[1:]) <= TOL_F
