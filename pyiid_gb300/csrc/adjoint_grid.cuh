@@ -29,52 +29,57 @@ constexpr int kAdjCoef = 8;     // polynomial coefficients per cell
 constexpr int kAdjBlock = 256;  // threads of both kernels
 
 // wk[key][k][p]: W_k times the coefficient of t^p in cos(k delta t) (p even)
-// and sin(k delta t) (p odd), delta = 2 pi / M; zero outside [kmin, n_bins)
-// or where na_k = 0.  key = configuration x species pair (sa >= sb).
-__global__ void adjoint_grid_weights_kernel(
-    const double *__restrict__ w, const double *__restrict__ na,
-    const float *__restrict__ ftab, const int2 *__restrict__ spair_species,
-    int n_spairs, int n_bins, int kmin, int n_configs, float delta,
-    float4 *__restrict__ wk) {
-  const size_t total = (size_t)n_configs * n_spairs * n_bins;
-  for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (size_t)gridDim.x * blockDim.x) {
-    const int k = idx % n_bins;
-    const size_t key = idx / n_bins;
-    const int2 ss = spair_species[key % n_spairs];
-    const size_t b = key / n_spairs;
-    float W = 0.f;
-    if (k >= kmin) {
-      const double nak = na[b * n_bins + k];
-      if (nak != 0.0)
-        W = (float)(2.0 * w[b * n_bins + k] * (double)ftab[ss.x * n_bins + k] *
-                    (double)ftab[ss.y * n_bins + k] / nak);
-    }
-    // Taylor terms z^p / p! of z = k delta <= pi/4; with tau = 2 t,
-    // tau^8 = 2 tau^6 - 5/4 tau^4 + tau^2/4 - 1/128 + T_8(tau)/128
-    const float z = (float)k * delta, z2 = z * z;
-    const float z4 = z2 * z2;
-    const float e8 = z4 * z4 * (1.0f / 40320.0f);
-    const float e0 = 1.0f - e8 * (1.0f / 32768.0f);
-    const float e2 = -0.5f * z2 + e8 * (1.0f / 256.0f);
-    const float e4 = z4 * (1.0f / 24.0f) - e8 * (5.0f / 64.0f);
-    const float e6 = -z4 * z2 * (1.0f / 720.0f) + e8 * 0.5f;
-    const float o3 = -z * z2 * (1.0f / 6.0f), o5 = z * z4 * (1.0f / 120.0f);
-    const float o7 = -z * z4 * z2 * (1.0f / 5040.0f);
-    wk[2 * idx] = make_float4(W * e0, W * z, W * e2, W * o3);
-    wk[2 * idx + 1] = make_float4(W * e4, W * o5, W * e6, W * o7);
+// and sin(k delta t) (p odd), delta = 2 pi / M; zero below kmin or where
+// na_k = 0.  key = configuration x species pair (sa >= sb).
+struct WkArgs {
+  const double *na;
+  const float *ftab;
+  const int2 *spair_species;
+  int n_spairs;
+  float delta;
+  float4 *wk;
+};
+
+// the weights of configuration b and bin k from w_k
+__device__ __forceinline__ void adjoint_grid_weights(const WkArgs &a, int b,
+                                                     int k, bool on, int n_bins,
+                                                     double w) {
+  const double nak = a.na[(size_t)b * n_bins + k];
+  const double w2 = on && nak != 0.0 ? 2.0 * w / nak : 0.0;
+  // Taylor terms z^p / p! of z = k delta <= pi/4; with tau = 2 t,
+  // tau^8 = 2 tau^6 - 5/4 tau^4 + tau^2/4 - 1/128 + T_8(tau)/128
+  const float z = (float)k * a.delta, z2 = z * z;
+  const float z4 = z2 * z2;
+  const float e8 = z4 * z4 * (1.0f / 40320.0f);
+  const float e0 = 1.0f - e8 * (1.0f / 32768.0f);
+  const float e2 = -0.5f * z2 + e8 * (1.0f / 256.0f);
+  const float e4 = z4 * (1.0f / 24.0f) - e8 * (5.0f / 64.0f);
+  const float e6 = -z4 * z2 * (1.0f / 720.0f) + e8 * 0.5f;
+  const float o3 = -z * z2 * (1.0f / 6.0f), o5 = z * z4 * (1.0f / 120.0f);
+  const float o7 = -z * z4 * z2 * (1.0f / 5040.0f);
+  for (int s = 0; s < a.n_spairs; ++s) {
+    const int2 ss = a.spair_species[s];
+    const float W = (float)(w2 * (double)a.ftab[ss.x * n_bins + k] *
+                            (double)a.ftab[ss.y * n_bins + k]);
+    float4 *o = a.wk + 2 * (((size_t)b * a.n_spairs + s) * n_bins + k);
+    o[0] = make_float4(W * e0, W * z, W * e2, W * o3);
+    o[1] = make_float4(W * e4, W * o5, W * e6, W * o7);
   }
 }
 
 // tab[key][j][p], cell centres u = j, 0 <= j <= M/2 (B is odd in u, so half
 // a period is enough): even p sum wk sin(k theta_j), odd p sum wk
-// cos(k theta_j).  Lane = cell, the eight warps each take an eighth of every
-// chunk of bins (keeps the chain of FP32 additions and of the seeds short:
-// 42 bins at 330) and are added in a fixed order.  Bins go in blocks of nine
-// around an accurate centre, each one rotation by +-n theta_j, n <= 4, away
-// from it, so no error builds up along k.  FP32 issue bound: 8 FMA per
-// (cell, bin) and about 9 instructions for the sine and cosine.
-constexpr int kAdjChunk = 8 * 63;  // bins staged in shared memory (16 KB)
+// cos(k theta_j).  The cell j' = M/2 - j has sin(k theta_j') = -(-1)^k
+// sin(k theta_j) and cos(k theta_j') = (-1)^k cos(k theta_j), so the sums of
+// even and of odd bins, kept apart, give both cells for one.
+// Lane = cell j <= M/4, the eight warps each take an eighth of every chunk of
+// bins (keeps the chains of FP32 additions short: 42 bins at 330) and are
+// added in a fixed order.  Bins go in blocks of eight around an accurate
+// centre, each one rotation by +-n theta_j, n <= 4, away from it, so no error
+// builds up along k.  What bounds it is the reads of wk (two of 16 bytes per
+// bin and warp, four cycles each): 38 us for 64 keys of 330 bins with one
+// cell per lane, 20 with two.
+constexpr int kAdjChunk = 512;  // bins staged in shared memory (16 KB)
 __global__ void __launch_bounds__(kAdjBlock)
     adjoint_grid_table_kernel(const float4 *__restrict__ wk, int n_bins,
                               int kmin, int m, float inv_m,
@@ -82,72 +87,76 @@ __global__ void __launch_bounds__(kAdjBlock)
   __shared__ float4 sw[2 * kAdjChunk];
   __shared__ float red[8][kAdjCoef][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int n_cells = m / 2 + 1;
-  const int j = min((int)(blockIdx.x * 32 + lane), n_cells - 1);
+  const int n_cells = m / 2 + 1, n_half = m / 4 + 1;
+  const int j = min((int)(blockIdx.x * 32 + lane), n_half - 1);
   const size_t key = blockIdx.y;
   float sn[4], cn[4];
 #pragma unroll
   for (int n = 0; n < 4; ++n)
     sincos_turn((n + 1) * j % m, m, inv_m, sn[n], cn[n]);
-  float acc[kAdjCoef];
+  float acc[2][kAdjCoef];  // even, odd bins
 #pragma unroll
-  for (int p = 0; p < kAdjCoef; ++p) acc[p] = 0.f;
-  for (int k0 = kmin; k0 < n_bins; k0 += kAdjChunk) {
+  for (int p = 0; p < kAdjCoef; ++p) acc[0][p] = acc[1][p] = 0.f;
+  for (int k0 = kmin & ~1; k0 < n_bins; k0 += kAdjChunk) {
     const int nb = min(kAdjChunk, n_bins - k0);
     __syncthreads();
-    for (int i = threadIdx.x; i < 2 * nb; i += kAdjBlock)
-      sw[i] = wk[2 * (key * n_bins + k0) + i];
+    for (int i = threadIdx.x; i < 2 * kAdjChunk; i += kAdjBlock)
+      sw[i] = i < 2 * nb ? wk[2 * (key * n_bins + k0) + i]
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
-    const int per = ((nb + 7) / 8 + 8) / 9 * 9;  // bins per warp
+    const int per = ((nb + 7) / 8 + 7) / 8 * 8;  // bins per warp
     const int i1 = min((warp + 1) * per, nb);
-    float part[kAdjCoef];
-#pragma unroll
-    for (int p = 0; p < kAdjCoef; ++p) part[p] = 0.f;
-    for (int i0 = warp * per; i0 < i1; i0 += 9) {
+    for (int i0 = warp * per; i0 < i1; i0 += 8) {
+      // (12,292 x 24,577 stays under 2^31)
       float sc, cc;
-      // (12,292 x 49,152 stays under 2^31)
       sincos_turn((k0 + i0 + 4) * j % m, m, inv_m, sc, cc);
 #pragma unroll
-      for (int n = -4; n <= 4; ++n) {
-        const int i = i0 + 4 + n;
-        if (i < i1) {
-          float s = sc, c = cc;
-          if (n > 0) {
-            s = fmaf(cc, sn[n - 1], sc * cn[n - 1]);
-            c = fmaf(-sc, sn[n - 1], cc * cn[n - 1]);
-          } else if (n < 0) {
-            s = fmaf(-cc, sn[-n - 1], sc * cn[-n - 1]);
-            c = fmaf(sc, sn[-n - 1], cc * cn[-n - 1]);
-          }
-          const float4 a = sw[2 * i], b = sw[2 * i + 1];
-          part[0] = fmaf(a.x, s, part[0]);
-          part[1] = fmaf(a.y, c, part[1]);
-          part[2] = fmaf(a.z, s, part[2]);
-          part[3] = fmaf(a.w, c, part[3]);
-          part[4] = fmaf(b.x, s, part[4]);
-          part[5] = fmaf(b.y, c, part[5]);
-          part[6] = fmaf(b.z, s, part[6]);
-          part[7] = fmaf(b.w, c, part[7]);
+      for (int n = -4; n < 4; ++n) {
+        const int i = i0 + 4 + n;  // < 512; weights past nb are zero
+        float s = sc, c = cc;
+        if (n > 0) {
+          s = fmaf(cc, sn[n - 1], sc * cn[n - 1]);
+          c = fmaf(-sc, sn[n - 1], cc * cn[n - 1]);
+        } else if (n < 0) {
+          s = fmaf(-cc, sn[-n - 1], sc * cn[-n - 1]);
+          c = fmaf(sc, sn[-n - 1], cc * cn[-n - 1]);
         }
+        float(&part)[kAdjCoef] = acc[n & 1];
+        const float4 a = sw[2 * i], b = sw[2 * i + 1];
+        part[0] = fmaf(a.x, s, part[0]);
+        part[1] = fmaf(a.y, c, part[1]);
+        part[2] = fmaf(a.z, s, part[2]);
+        part[3] = fmaf(a.w, c, part[3]);
+        part[4] = fmaf(b.x, s, part[4]);
+        part[5] = fmaf(b.y, c, part[5]);
+        part[6] = fmaf(b.z, s, part[6]);
+        part[7] = fmaf(b.w, c, part[7]);
       }
     }
-#pragma unroll
-    for (int p = 0; p < kAdjCoef; ++p) acc[p] += part[p];
   }
-#pragma unroll
-  for (int p = 0; p < kAdjCoef; ++p) red[warp][p][lane] = acc[p];
-  __syncthreads();
-  // thread = (cell, coefficient): the eight warps' sums, pairwise
-  float *out = reinterpret_cast<float *>(tab);
+  // thread = (cell, coefficient): the eight warps' sums, pairwise; even bins
+  // first, then odd ones
   const int cell = threadIdx.x >> 3, p = threadIdx.x & 7;
-  const int jj = blockIdx.x * 32 + cell;
-  if (jj < n_cells) {
-    const float s = ((red[0][p][cell] + red[1][p][cell]) +
-                     (red[2][p][cell] + red[3][p][cell])) +
-                    ((red[4][p][cell] + red[5][p][cell]) +
-                     (red[6][p][cell] + red[7][p][cell]));
-    out[(key * n_cells + jj) * kAdjCoef + p] = s;
+  float sum[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kAdjCoef; ++q) red[warp][q][lane] = acc[e][q];
+    __syncthreads();
+    sum[e] = ((red[0][p][cell] + red[1][p][cell]) +
+              (red[2][p][cell] + red[3][p][cell])) +
+             ((red[4][p][cell] + red[5][p][cell]) +
+              (red[6][p][cell] + red[7][p][cell]));
   }
+  const int jj = blockIdx.x * 32 + cell;
+  if (jj >= n_half) return;
+  float *out = reinterpret_cast<float *>(tab) + key * n_cells * kAdjCoef + p;
+  // (even p: sines, odd p: cosines; the middle cell is its own image)
+  out[(size_t)jj * kAdjCoef] = sum[0] + sum[1];
+  if (2 * jj < n_cells - 1)
+    out[(size_t)(n_cells - 1 - jj) * kAdjCoef] =
+        (p & 1) ? sum[0] - sum[1] : sum[1] - sum[0];
 }
 
 // grad[a] = sum_b s_ab (x_a - x_b).  CTA = tile I, lane = atom a of it; the
@@ -160,8 +169,8 @@ __global__ void __launch_bounds__(kAdjBlock)
 // run beside them.  TAB_SMEM: the key's table is staged in shared memory
 // (it does not fit for more than about 850 bins: then it is read through
 // L1).  A pair at r = 0 gives NaN, as the closed form does.
-// 64 x 1,000 atoms, 330 bins: 244 us, after 38 us for the tables and 5 for
-// the weights (adjoint_sym_kernel and its reduction: 2,470 us); the gradient
+// 64 x 1,000 atoms, 330 bins: 244 us, after 20 us for the tables
+// (adjoint_sym_kernel and its reduction: 2,470 us); the gradient
 // is 1.1e-7 off the FP64 one (2.3e-7).
 template <bool TAB_SMEM>
 __global__ void __launch_bounds__(kAdjBlock)

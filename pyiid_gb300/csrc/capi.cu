@@ -794,6 +794,10 @@ int set_attrs(pyiid_ctx *ctx) {
                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                     (int)(fq_dft_float4(kFqCellsPerBin * kFqGridMaxBins) *
                           sizeof(float4))));
+  // (partial sums of 12,288 bins beside the staged F)
+  CUDA_TRY(ctx, cudaFuncSetAttribute(pdf_kernel<1>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     48 * 1024));
   CUDA_TRY(ctx, cudaFuncSetAttribute(adjoint_grid_kernel<true>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kAdjTabSmem));
@@ -1496,6 +1500,61 @@ int run_grad_grid(pyiid_ctx *ctx, Layout *L, const float *positions,
   return PYIID_OK;
 }
 
+// One cluster per configuration, of as many CTAs (8, 2 or 1) as leave an SM
+// to each: 64 configurations of 4,000 points take 75 us in clusters of
+// eight, whose sums then queue on the FP64 pipes, 38 in one CTA each and 19
+// in two.
+int run_potential(pyiid_ctx *ctx, const double *gobs, const double *gcalc,
+                  int n_configs, int n_r, int potential, double *out,
+                  float *cvec, const double *weight) {
+  const int ctas = 8 * n_configs <= ctx->n_sms   ? 8
+                   : 2 * n_configs <= ctx->n_sms ? 2
+                                                 : 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas * n_configs);
+  cfg.blockDim = dim3(256);
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = ctas;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, potential_kernel, gobs, gcalc, n_r,
+                                   potential, ctas, out, cvec, weight));
+  LAUNCH_CHECK(ctx);
+  return PYIID_OK;
+}
+
+// G(r) rows of n_configs F(Q) rows.  Eight configurations share the reads of
+// T where there are as many and their partial sums fit 48 KB (1,536 bins).
+int run_pdf(pyiid_ctx *ctx, const float *fq, const TMatrix *T, int n_bins,
+            int n_r, int n_configs, double *gr) {
+  TRY(set_attrs(ctx));
+  const int blocks =
+      std::max(1, (n_bins - T->kmin + kPdfBlock - 1) / kPdfBlock);
+  const int threads = 32 * std::min(16, blocks);
+  const unsigned gx = (n_r + 31) / 32;
+  if (n_configs >= 8 && blocks <= 32) {
+    // (32 KB of partial sums beside 16 KB of staged F at most)
+    pdf_kernel<8><<<dim3(gx, (n_configs + 7) / 8), threads,
+                    (size_t)blocks * 8 * 32 * sizeof(float), ctx->stream>>>(
+        fq, T->d_T, n_bins, n_r, T->kmin, n_configs, gr);
+    LAUNCH_CHECK(ctx);
+    return PYIID_OK;
+  }
+  const size_t smem = (size_t)blocks * 32 * sizeof(float);
+  // (n_bins <= 12,288: 48 KB at most, beside 2 KB)
+  for (int b0 = 0; b0 < n_configs; b0 += 65535) {
+    const int nb = std::min(65535, n_configs - b0);
+    pdf_kernel<1><<<dim3(gx, nb), threads, smem, ctx->stream>>>(
+        fq + (size_t)b0 * n_bins, T->d_T, n_bins, n_r, T->kmin, nb,
+        gr + (size_t)b0 * n_r);
+    LAUNCH_CHECK(ctx);
+  }
+  return PYIID_OK;
+}
+
 int batch_fq(pyiid_ctx *ctx, const float *positions, const int32_t *species,
              const int32_t *offsets, int n_configs, const float *scatter,
              int n_species, int n_bins, double qbin, int k_begin, float *fq) {
@@ -1903,11 +1962,7 @@ int pyiid_pdf(pyiid_ctx *ctx, const float *fq, int n_configs, int n_bins,
   CUDA_TRY(ctx, cudaSetDevice(ctx->device));
   TMatrix *T;
   TRY(get_tmatrix(ctx, n_bins, qstep, rstep, rgrid, n_r, qmin, &T));
-  dim3 grid((n_r + 255) / 256, n_configs);
-  pdf_kernel<<<grid, 256, n_bins * sizeof(float), ctx->stream>>>(
-      fq, T->d_T, n_bins, n_r, T->kmin, gr);
-  LAUNCH_CHECK(ctx);
-  return PYIID_OK;
+  return run_pdf(ctx, fq, T, n_bins, n_r, n_configs, gr);
 }
 
 int pyiid_grad_pdf(pyiid_ctx *ctx, const float *grad_fq, int n_atoms,
@@ -1989,9 +2044,8 @@ int pyiid_potential(pyiid_ctx *ctx, const double *gobs, const double *gcalc,
   if (potential != PYIID_POTENTIAL_RW && potential != PYIID_POTENTIAL_CHI_SQ)
     return fail(ctx, PYIID_ERR_INVALID_ARG, "unknown potential %d", potential);
   CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-  potential_kernel<<<n_configs, 256, 0, ctx->stream>>>(gobs, gcalc, n_r,
-                                                       potential, out, nullptr);
-  LAUNCH_CHECK(ctx);
+  TRY(run_potential(ctx, gobs, gcalc, n_configs, n_r, potential, out, nullptr,
+                    nullptr));
   return PYIID_OK;
 }
 
@@ -2003,9 +2057,8 @@ int pyiid_potential_weighted(pyiid_ctx *ctx, const double *gobs,
     return fail(ctx, PYIID_ERR_INVALID_ARG, "bad sizes");
   if (!weight) return fail(ctx, PYIID_ERR_INVALID_ARG, "null weight");
   CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-  potential_kernel<<<n_configs, 256, 0, ctx->stream>>>(
-      gobs, gcalc, n_r, PYIID_POTENTIAL_RW, out, nullptr, weight);
-  LAUNCH_CHECK(ctx);
+  TRY(run_potential(ctx, gobs, gcalc, n_configs, n_r, PYIID_POTENTIAL_RW, out,
+                    nullptr, weight));
   return PYIID_OK;
 }
 
@@ -2024,9 +2077,7 @@ int pyiid_potential_grad(pyiid_ctx *ctx, const double *grad_pdf,
   double *e = static_cast<double *>(p);
   TRY(ensure(ctx, "cvec", (size_t)n_r * sizeof(float), &p));
   float *cvec = static_cast<float *>(p);
-  potential_kernel<<<1, 256, 0, ctx->stream>>>(gobs, gcalc, n_r, potential, e,
-                                               cvec);
-  LAUNCH_CHECK(ctx);
+  TRY(run_potential(ctx, gobs, gcalc, 1, n_r, potential, e, cvec, nullptr));
   const int rows = 3 * n_atoms;
   potential_grad_rows_kernel<<<(rows * 32 + 255) / 256, 256, 0, ctx->stream>>>(
       grad_pdf, cvec, rows, n_r, grad);
@@ -2072,42 +2123,43 @@ int pyiid_batch_potential_grad(pyiid_ctx *ctx, const float *positions,
   }
   TRY(run_fq(ctx, L, positions, d_ftab, d_na, n_bins, qstep, kmin, d_fq,
              nullptr));
-  dim3 gp((n_r + 255) / 256, n_configs);
-  pdf_kernel<<<gp, 256, n_bins * sizeof(float), ctx->stream>>>(
-      d_fq, T->d_T, n_bins, n_r, kmin, d_gc);
-  LAUNCH_CHECK(ctx);
+  TRY(run_pdf(ctx, d_fq, T, n_bins, n_r, n_configs, d_gc));
   float *cvec = nullptr;
   if (grad) {
     TRY(ensure(ctx, "b_cvec", (size_t)n_configs * n_r * sizeof(float), &p));
     cvec = static_cast<float *>(p);
   }
-  potential_kernel<<<n_configs, 256, 0, ctx->stream>>>(gobs, d_gc, n_r,
-                                                       potential, energy, cvec);
-  LAUNCH_CHECK(ctx);
+  TRY(run_potential(ctx, gobs, d_gc, n_configs, n_r, potential, energy, cvec,
+                    nullptr));
   if (!grad || L->total == 0) return PYIID_OK;
   TRY(ensure(ctx, "b_w", (size_t)n_configs * n_bins * sizeof(double), &p));
   double *w = static_cast<double *>(p);
-  const int nwarps = n_configs * n_bins;
-  wvec_kernel<<<(nwarps * 32 + 255) / 256, 256, 0, ctx->stream>>>(
-      T->d_T, cvec, n_bins, n_r, kmin, n_configs, w);
-  LAUNCH_CHECK(ctx);
-  if (grid_adjoint(L, n_bins)) {
-    const int m = kAdjCellsPerBin * n_bins, n_cells = m / 2 + 1;
-    const size_t n_keys = (size_t)n_configs * L->n_spairs;
+  const bool on_grid = grid_adjoint(L, n_bins);
+  const int m = kAdjCellsPerBin * n_bins, n_cells = m / 2 + 1;
+  const size_t n_keys = (size_t)n_configs * L->n_spairs;
+  WkArgs wa{d_na, d_ftab, L->d_spair, L->n_spairs, (float)(2.0 * M_PI / m),
+            nullptr};
+  if (on_grid) {
     TRY(ensure(ctx, "b_wk", n_keys * n_bins * 2 * sizeof(float4), &p));
-    float4 *wk = static_cast<float4 *>(p);
+    wa.wk = static_cast<float4 *>(p);
+  }
+  if (n_configs >= 8)
+    wvec_kernel<4, 8><<<dim3((n_bins + 3) / 4, (n_configs + 7) / 8), 128, 0,
+                        ctx->stream>>>(T->d_T, cvec, n_bins, n_r, kmin,
+                                       n_configs, w, wa);
+  else
+    wvec_kernel<1, 1><<<dim3(n_bins, n_configs), 128, 0, ctx->stream>>>(
+        T->d_T, cvec, n_bins, n_r, kmin, n_configs, w, wa);
+  LAUNCH_CHECK(ctx);
+  if (on_grid) {
     TRY(ensure(ctx, "b_gtab", n_keys * n_cells * 2 * sizeof(float4), &p));
     float4 *gtab = static_cast<float4 *>(p);
-    adjoint_grid_weights_kernel<<<256, 256, 0, ctx->stream>>>(
-        w, d_na, d_ftab, L->d_spair, L->n_spairs, n_bins, kmin, n_configs,
-        (float)(2.0 * M_PI / m), wk);
-    LAUNCH_CHECK(ctx);
     // keys in grid.y: at most 65,535 per launch
     for (size_t key0 = 0; key0 < n_keys; key0 += 32768) {
-      const dim3 g((n_cells + 31) / 32,
+      const dim3 g((m / 4 + 32) / 32,
                    (unsigned)std::min<size_t>(32768, n_keys - key0));
       adjoint_grid_table_kernel<<<g, kAdjBlock, 0, ctx->stream>>>(
-          wk + key0 * n_bins * 2, n_bins, kmin, m, 1.0f / (float)m,
+          wa.wk + key0 * n_bins * 2, n_bins, kmin, m, 1.0f / (float)m,
           gtab + key0 * n_cells * 2);
       LAUNCH_CHECK(ctx);
     }

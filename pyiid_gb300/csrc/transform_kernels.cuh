@@ -10,31 +10,74 @@
 // from HBM/L2 once per CTA column block.
 #pragma once
 
+#include <cooperative_groups.h>
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "adjoint_grid.cuh"
+
 namespace pyiid {
 
-// gr[b][i] = sum_k fq[b][k] * T[k][i]  (FP32 products, FP32 blocks of 32 bins
-// summed in FP64).  grid (ceil(n_r/256), n_configs)
-__global__ void pdf_kernel(const float *__restrict__ fq,
-                           const float *__restrict__ T, int n_bins, int n_r,
-                           int kmin, double *__restrict__ gr) {
-  extern __shared__ float sf[];
-  const int b = blockIdx.y;
-  for (int k = threadIdx.x; k < n_bins; k += blockDim.x)
-    sf[k] = (k >= kmin) ? fq[(size_t)b * n_bins + k] : 0.f;
-  __syncthreads();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_r) return;
-  double acc = 0.0;
-  for (int k0 = kmin; k0 < n_bins; k0 += 32) {
-    float part = 0.f;
-    const int k1 = min(k0 + 32, n_bins);
-    for (int k = k0; k < k1; ++k) part = fmaf(sf[k], T[(size_t)k * n_r + i], part);
-    acc += (double)part;
+// gr[b][i] = sum_k fq[b][k] * T[k][i]: FP32 products summed over blocks of
+// 32 bins, the blocks in FP64 in their order.  CTA = (32 points r, NB
+// configurations); the warps take the blocks of bins, so that a small batch
+// still fills the GPU (one warp per 256 points and all bins took 30 us for
+// one configuration of 330 x 4,000 against 9), and an element of T read from
+// L2 serves NB configurations (64 of them: 35 us against 30, where the FP64
+// sums of the blocks, 16 cycles an instruction, now take a third).
+// Dynamic shared memory: blocks x NB x 32 partial sums.
+constexpr int kPdfBlock = 32;  // bins
+template <int NB>
+__global__ void __launch_bounds__(512)
+    pdf_kernel(const float *__restrict__ fq, const float *__restrict__ T,
+               int n_bins, int n_r, int kmin, int n_configs,
+               double *__restrict__ gr) {
+  extern __shared__ float spart[];  // [block][NB][32]
+  __shared__ float sf[16][kPdfBlock][NB];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n_warps = blockDim.x >> 5;
+  const int i = blockIdx.x * 32 + lane, b0 = blockIdx.y * NB;
+  const int n_blocks = max(0, (n_bins - kmin + kPdfBlock - 1) / kPdfBlock);
+  const float *Ti = T + min(i, n_r - 1);
+  for (int blk = warp; blk < n_blocks; blk += n_warps) {
+    const int k0 = kmin + blk * kPdfBlock, nk = min(kPdfBlock, n_bins - k0);
+    __syncwarp();
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+      sf[warp][lane][b] = lane < nk && b0 + b < n_configs
+                              ? fq[(size_t)(b0 + b) * n_bins + k0 + lane]
+                              : 0.f;
+    __syncwarp();
+    float part[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) part[b] = 0.f;
+    if (nk == kPdfBlock) {
+#pragma unroll 8
+      for (int k = 0; k < kPdfBlock; ++k) {
+        const float t = Ti[(size_t)(k0 + k) * n_r];
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+          part[b] = fmaf(sf[warp][k][b], t, part[b]);
+      }
+    } else {
+      for (int k = 0; k < nk; ++k) {
+        const float t = Ti[(size_t)(k0 + k) * n_r];
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+          part[b] = fmaf(sf[warp][k][b], t, part[b]);
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b) spart[(blk * NB + b) * 32 + lane] = part[b];
   }
-  gr[(size_t)b * n_r + i] = acc;
+  __syncthreads();
+  for (int b = warp; b < NB && b0 + b < n_configs; b += n_warps) {
+    if (i >= n_r) break;
+    double acc = 0.0;
+    for (int blk = 0; blk < n_blocks; ++blk)
+      acc += (double)spart[(blk * NB + b) * 32 + lane];
+    gr[(size_t)(b0 + b) * n_r + i] = acc;
+  }
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -62,7 +105,7 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double *scratch) {
   __syncthreads();
 }
 
-// Potential per configuration (one CTA each), get_rw / get_chi_sq / get_scale
+// Potential per configuration, get_rw / get_chi_sq / get_scale
 // of kernels/master_kernel.py:206-266, 388-389:
 //   a = (gc.go)/(gc.gc); Rw: a <= 0 -> (1, 1), else sqrt(|go - a gc|^2/|go|^2)
 //   chi^2: s = a if a > 0 else 1, value = |go - s gc|^2
@@ -71,102 +114,157 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double *scratch) {
 // the scale uses the raw a even when the value used scale 1):
 //   c_i = pre [s E_i + (gc.E) (go_i - 2 a gc_i)/(gc.gc)],  E = go - s gc,
 //   pre = -Rw/|E|^2 (Rw) or -2 (chi^2).
-struct PotentialValue {
-  double value, scale;  // potential and the scale it used
-  double a, gcc, ee, gce;
-};
 
-// The potential of one configuration, computed by the whole CTA (every
-// thread returns the same values).  scratch: 32 * 4 doubles of shared memory.
+// Sums over the 256 threads of every CTA of a cluster.  FP64 issues one warp
+// instruction in 16 cycles here, so a warp per value adds what all threads
+// have left in shared memory (13 instructions, against 5 in each of the
+// eight warps by shuffles); the CTAs then read each other's sums there
+// (distributed shared memory), in a fixed order.
+struct ClusterSums {
+  double part[4][256];
+  double mine[4], total[4];
+};
+template <int NV>
+__device__ __forceinline__ void cluster_sum(double (&v)[NV], ClusterSums &m) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) m.part[i][threadIdx.x] = v[i];
+  __syncthreads();
+  if (warp < NV) {
+    double s = 0.0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += m.part[warp][32 * i + lane];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) m.mine[warp] = s;
+  }
+  cl.sync();
+  if (warp < NV) {
+    const int n = (int)cl.num_blocks();  // 1, 2 or 8
+    double s = lane < n ? cl.map_shared_rank(m.mine, lane)[warp] : 0.0;
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) m.total[warp] = s;
+  }
+  cl.sync();  // nobody leaves, or writes again, before all have read
+#pragma unroll
+  for (int i = 0; i < NV; ++i) v[i] = m.total[i];
+}
+
+// Potential of one configuration per cluster of CTAs, which share the points
+// r: get_rw / get_chi_sq with get_scale as above.  FP64 bound; one CTA spent
+// 39 us on 4,000 points, eight spend 11.
 // weight (Rw only, may be null): per-point weights of get_rw
 // (master_kernel.py:226-235): Rw = sqrt(sum w (go - a gc)^2 / sum w go^2)
 // with the unweighted scale a; ee and gce (used by the gradients, which the
 // reference never weights) stay unweighted.
-__device__ __forceinline__ PotentialValue potential_value(
-    const double *__restrict__ gobs, const double *__restrict__ gc, int n_r,
-    int potential, double *scratch,
-    const double *__restrict__ weight = nullptr) {
+__global__ void __launch_bounds__(256)
+    potential_kernel(const double *__restrict__ gobs,
+                     const double *__restrict__ gcalc, int n_r, int potential,
+                     int ctas, double *__restrict__ out,
+                     float *__restrict__ cvec,
+                     const double *__restrict__ weight) {
+  __shared__ ClusterSums sums;
+  const int b = blockIdx.x / ctas;
+  const int first = (blockIdx.x % ctas) * blockDim.x + threadIdx.x;
+  const int step = ctas * blockDim.x;
+  const double *gc = gcalc + (size_t)b * n_r;
   double v3[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int i = threadIdx.x; i < n_r; i += blockDim.x) {
+  for (int i = first; i < n_r; i += step) {
     const double c = gc[i], o = gobs[i];
     v3[0] += c * o;
     v3[1] += c * c;
     v3[2] += o * o;
     if (weight) v3[3] += weight[i] * o * o;
   }
-  block_sum<4>(v3, scratch);
+  cluster_sum<4>(v3, sums);
   const double gco = v3[0], gcc = v3[1];
   const double goo = weight ? v3[3] : v3[2];
   const double a = gco / gcc;
   // the reference replaces a non-positive scale by 1; a NaN scale stays NaN
   const double s = (a <= 0.0) ? 1.0 : a;
   double v2[3] = {0.0, 0.0, 0.0};
-  for (int i = threadIdx.x; i < n_r; i += blockDim.x) {
+  for (int i = first; i < n_r; i += step) {
     const double e = gobs[i] - s * gc[i];
     v2[0] += e * e;
     v2[1] += gc[i] * e;
     if (weight) v2[2] += weight[i] * e * e;
   }
-  block_sum<3>(v2, scratch);
-  PotentialValue r;
-  r.ee = v2[0];
-  r.gce = v2[1];
-  r.a = a;
-  r.gcc = gcc;
-  r.scale = s;
+  cluster_sum<3>(v2, sums);
+  const double ee = v2[0], gce = v2[1];
   const double top = weight ? v2[2] : v2[0];
-  if (potential == 0)
-    r.value = (a <= 0.0) ? 1.0 : sqrt(top / goo);
-  else
-    r.value = r.ee;
-  return r;
-}
-
-__global__ void potential_kernel(const double *__restrict__ gobs,
-                                 const double *__restrict__ gcalc, int n_r,
-                                 int potential, double *__restrict__ out,
-                                 float *__restrict__ cvec,
-                                 const double *__restrict__ weight = nullptr) {
-  __shared__ double scratch[32 * 4];
-  const int b = blockIdx.x;
-  const double *gc = gcalc + (size_t)b * n_r;
-  const PotentialValue pv =
-      potential_value(gobs, gc, n_r, potential, scratch, weight);
-  const double value = pv.value, s = pv.scale, a = pv.a, gcc = pv.gcc;
-  const double ee = pv.ee, gce = pv.gce;
-  const double pre = (potential == 0) ? -value / ee : -2.0;
-  if (threadIdx.x == 0) {
+  const double value =
+      potential == 0 ? (a <= 0.0 ? 1.0 : sqrt(top / goo)) : ee;
+  if (first == 0) {
     out[2 * b] = value;
     out[2 * b + 1] = s;
   }
   if (cvec) {
-    for (int i = threadIdx.x; i < n_r; i += blockDim.x) {
+    const double pre = (potential == 0) ? -value / ee : -2.0;
+    const double ratio = gce / gcc;
+    for (int i = first; i < n_r; i += step) {
       const double e = gobs[i] - s * gc[i];
-      const double ci = pre * (s * e + gce * (gobs[i] - 2.0 * a * gc[i]) / gcc);
-      cvec[(size_t)b * n_r + i] = (float)ci;
+      cvec[(size_t)b * n_r + i] =
+          (float)(pre * (s * e + ratio * (gobs[i] - 2.0 * a * gc[i])));
     }
   }
 }
 
-// w[b][k] = sum_i T[k][i] c[b][i]: one warp per (b, k); FP32 products, lane
-// partials reduced in FP64.
-__global__ void wvec_kernel(const float *__restrict__ T,
-                            const float *__restrict__ cvec, int n_bins,
-                            int n_r, int kmin, int n_configs,
-                            double *__restrict__ w) {
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (gw >= n_configs * n_bins) return;
-  const int b = gw / n_bins, k = gw % n_bins;
-  double acc = 0.0;
-  if (k >= kmin) {
-    const float *row = T + (size_t)k * n_r;
-    const float *c = cvec + (size_t)b * n_r;
-    float part = 0.f;
-    for (int i = lane; i < n_r; i += 32) part = fmaf(row[i], c[i], part);
-    acc = warp_sum((double)part);
+// w[b][k] = sum_i T[k][i] c[b][i] in FP64 from FP32 lane sums, and with wk
+// the weights of the pair-force tables (adjoint_grid.cuh) that follow from
+// it.  CTA = NK bins x NB configurations: an element of T and one of c read
+// serve NB and NK products (64 configurations of 330 x 4,000: 43 us with a
+// warp per bin and configuration, 24 so), and one configuration still has a
+// CTA per bin (19 us against 10).
+template <int NK, int NB>
+__global__ void __launch_bounds__(128)
+    wvec_kernel(const float *__restrict__ T, const float *__restrict__ cvec,
+                int n_bins, int n_r, int kmin, int n_configs,
+                double *__restrict__ w, WkArgs wa) {
+  __shared__ float red[NK * NB][129];
+  const int k0 = blockIdx.x * NK, b0 = blockIdx.y * NB;
+  float acc[NK][NB];
+#pragma unroll
+  for (int k = 0; k < NK; ++k)
+#pragma unroll
+    for (int b = 0; b < NB; ++b) acc[k][b] = 0.f;
+  if (k0 + NK > kmin) {
+#pragma unroll(NK * NB > 1 ? 2 : 8)
+    for (int i = threadIdx.x; i < n_r; i += 128) {
+      float t[NK], c[NB];
+#pragma unroll
+      for (int k = 0; k < NK; ++k)
+        t[k] = T[(size_t)min(k0 + k, n_bins - 1) * n_r + i];
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+        c[b] = cvec[(size_t)min(b0 + b, n_configs - 1) * n_r + i];
+#pragma unroll
+      for (int k = 0; k < NK; ++k)
+#pragma unroll
+        for (int b = 0; b < NB; ++b) acc[k][b] = fmaf(t[k], c[b], acc[k][b]);
+    }
   }
-  if (lane == 0) w[(size_t)b * n_bins + k] = acc;
+#pragma unroll
+  for (int k = 0; k < NK; ++k)
+#pragma unroll
+    for (int b = 0; b < NB; ++b) red[k * NB + b][threadIdx.x] = acc[k][b];
+  __syncthreads();
+  // 128 / (NK NB) threads per value (all of a warp at most) add fours of
+  // lane sums in FP32, these in FP64
+  constexpr int P = 128 / (NK * NB) > 32 ? 32 : 128 / (NK * NB);
+  const int v = threadIdx.x / P, p = threadIdx.x % P;
+  if (v >= NK * NB) return;  // whole warps
+  double sum = 0.0;
+  for (int i = p; i < 32; i += P)
+    sum += (double)((red[v][i] + red[v][i + 32]) +
+                    (red[v][i + 64] + red[v][i + 96]));
+  for (int o = P / 2; o > 0; o >>= 1)
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  const int k = k0 + v / NB, b = b0 + v % NB;
+  if (p != 0 || k >= n_bins || b >= n_configs) return;
+  if (k < kmin) sum = 0.0;
+  w[(size_t)b * n_bins + k] = sum;
+  if (wa.wk) adjoint_grid_weights(wa, b, k, k >= kmin, n_bins, sum);
 }
 
 // Adjoint tables: tabs[b][sa][sb][m] = (A_kk, A_kk+1, B_kk, B_kk+1),

@@ -270,3 +270,41 @@ def test_gradient_on_the_grid_under_capture(D):
         torch.cuda.synchronize()
         assert torch.equal(f2, f) and torch.equal(out, g)
         assert rel(f.cpu().numpy()[1:], fq64(pos, sp, tab, 0.05)[1:]) <= TOL_F
+
+
+# one, two and eight CTAs per cluster (100, 60, 3 configurations), eight
+# configurations at a time with a remainder, bins in part of a block, qmin
+# above the first block, few and odd points
+@pytest.mark.parametrize('n_configs,exp', [
+    (1, {'rmax': 20.0}), (3, {'rmax': 7.01, 'rstep': 0.03}),
+    (8, {'rmax': 33.0, 'qmin': 3.3}), (60, {'rmax': 20.0, 'qmin': 0.5}),
+    (101, {'rmax': 12.0, 'rstep': 0.05}),
+])
+def test_transform_and_potential_of_batches(D, n_configs, exp):
+    import torch
+    e = O.update_experiment(dict({'rstep': 0.02}, **exp))
+    qb, rg = O.pdf_qbin(e), O.r_grid(e)
+    nb = int(np.floor(e['qmax'] / qb))
+    rng = np.random.default_rng(n_configs)
+    fq = rng.normal(0, 1, (n_configs, nb)).astype(np.float32)
+    gr = D.pdf(torch.as_tensor(fq, device='cuda'), qb, e['rstep'], rg,
+               e['qmin'])
+    want = np.stack([O.pdf_fft(f.astype(np.float64), e['rstep'], qb, rg,
+                               e['qmin']) for f in fq])
+    assert rel(gr.cpu().numpy(), want) <= TOL_F
+    gobs = want[0] + rng.normal(0, .3, len(rg))
+    g = torch.as_tensor(want, device='cuda')
+    w = torch.as_tensor(rng.random(len(rg)), device='cuda')
+    for kind, f in (('rw', O.get_rw), ('chi_sq', O.get_chi_sq)):
+        got = D.potential(torch.as_tensor(gobs), g, kind).cpu().numpy()
+        for i in range(n_configs):
+            v, s = f(gobs, want[i])
+            assert abs(got[i, 0] - v) <= 1e-12 * abs(v)
+            assert abs(got[i, 1] - s) <= 1e-12 * abs(s)
+    got = D.potential(torch.as_tensor(gobs), g, 'rw', weight=w).cpu().numpy()
+    wn = w.cpu().numpy()
+    for i in range(n_configs):
+        a = (want[i] @ gobs) / (want[i] @ want[i])
+        v = 1.0 if a <= 0 else np.sqrt((wn * (gobs - a * want[i]) ** 2).sum() /
+                                       (wn * gobs ** 2).sum())
+        assert abs(got[i, 0] - v) <= 1e-12 * abs(v)
