@@ -159,118 +159,148 @@ __global__ void __launch_bounds__(kAdjBlock)
         (p & 1) ? sum[0] - sum[1] : sum[1] - sum[0];
 }
 
-// grad[a] = sum_b s_ab (x_a - x_b).  CTA = tile I, lane = atom a of it; the
-// eight warps share the atoms b, staged kAdjBlock at a time, so all lanes of
-// a warp read one b (a broadcast) and the table at 32 unrelated cells.  Each
-// ordered pair is evaluated: the unordered half would save the distance of
-// every second pair but need its force carried to the other atom (six
-// shuffles and a second pass over partial rows).  About 75 instructions per
-// 32 pairs; the two 16-byte table reads, 8 to 10 shared-memory cycles each,
-// run beside them.  TAB_SMEM: the key's table is staged in shared memory
-// (it does not fit for more than about 850 bins: then it is read through
-// L1).  A pair at r = 0 gives NaN, as the closed form does.
-// 64 x 1,000 atoms, 330 bins: 244 us, after 20 us for the tables
-// (adjoint_sym_kernel and its reduction: 2,470 us); the gradient
-// is 1.1e-7 off the FP64 one (2.3e-7).
+// grad[a] = sum_b s_ab (x_a - x_b), each unordered pair once.  CTA = work item
+// (tile I, a run of tiles J <= I of one species); a warp takes a tile J, or a
+// share of the 32 steps of one where the run is shorter than five.  Lane a
+// holds atom a of I and in step s meets atom (a + s) mod 32 of J; the force
+// on that atom is summed in a register that moves one lane down per step, so
+// it stays with its atom (three shuffles a step; a warp sum would take
+// fifteen).  Atoms of one tile meet in all 31 ordered steps instead.  The
+// partial rows of I and J go to part (as adjoint_sym_kernel's) and
+// adjoint_reduce_kernel adds them in a fixed order.
+// Bound by the shared-memory pipe: the two 16-byte reads of the table at 32
+// unrelated cells take about ten cycles each.  They come from two planes: one
+// of 32-byte cells has only every second bank group at a time and took 14.
+// TAB_SMEM: the key's table is staged in shared memory; else it is read
+// through L1 (it does not fit for more than about 850 bins, and an item of one
+// tile pair does not earn the copy).  A pair at r = 0 gives NaN, as the closed
+// form does.
+// 64 x 1,000 atoms, 330 bins: 173 us and 9 for the reduction, after 20 us for
+// the tables (adjoint_sym_kernel and its reduction: 2,470 us; with each
+// ordered pair evaluated 244); the gradient is 1.1e-7 off the FP64 one
+// (2.3e-7).
 template <bool TAB_SMEM>
 __global__ void __launch_bounds__(kAdjBlock)
     adjoint_grid_kernel(const float *__restrict__ pos,
                         const int *__restrict__ perm,
                         const int4 *__restrict__ tiles,
-                        const int2 *__restrict__ cfg_tiles, GridScale gs,
+                        const int4 *__restrict__ items,
+                        const int *__restrict__ order, GridScale gs,
                         int n_cells, const float4 *__restrict__ tab,
-                        int n_spairs, float *__restrict__ grad) {
-  extern __shared__ float4 stab[];
-  __shared__ float4 sB[2][kAdjBlock];  // (hx, hy, hz, lx), (ly, lz, 0, 0)
-  __shared__ float sred[kAdjBlock / kTile][kTile][3];
-  const int4 ti = tiles[blockIdx.x];
-  const int2 ct = cfg_tiles[ti.z];
+                        const int *__restrict__ ioff,
+                        const int *__restrict__ joff, float *__restrict__ part) {
+  extern __shared__ float4 stab[];  // [2][n_cells]
+  constexpr int W = kAdjBlock / 32;
+  __shared__ float4 sJ[W][kTile][2];  // (hx, hy, hz, lx), (ly, lz, 0, 0)
+  __shared__ float sred[W][kTile][3];
+  __shared__ float sjac[W][kTile][3];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int ia = ti.x + min(lane, ti.y - 1);  // sorted index of this atom
-  const float4 pa = load_atom(pos, perm, ia);
-  const SplitAtom a = split_atom(pa.x, pa.y, pa.z);
+  const int item = order[blockIdx.x];
+  const int4 it = items[item];
+  const int4 ti = tiles[it.x];
+  const int len = it.z - it.y;
+  const float4 *src = tab + (size_t)it.w * n_cells * 2;
+  if (TAB_SMEM)
+    for (int i = threadIdx.x; i < 2 * n_cells; i += kAdjBlock)
+      stab[(i & 1) * n_cells + (i >> 1)] = src[i];
+  const bool here = lane < ti.y;
+  const float4 pa = load_atom(pos, perm, ti.x + min(lane, ti.y - 1));
+  SplitAtom a = split_atom(pa.x, pa.y, pa.z);
+  if (!here) a.hx += 1.0f;  // counts nothing; any place of its own
+  if (TAB_SMEM) __syncthreads();
+  // tasks: (tile of the run, share of its steps)
+  const int shares = len > 4 ? 1 : len > 2 ? 2 : len == 2 ? 4 : 8;
+  const int per = kTile / shares;
+  float *const pj = part + joff[item];
   float gx = 0.f, gy = 0.f, gz = 0.f;
-  for (int tj = ct.x; tj < ct.y;) {
-    // the run of tiles of one species: atoms [b0, b1) in sorted order
-    const int sb = tiles[tj].w, b0 = tiles[tj].x;
-    int b1 = b0;
-    for (; tj < ct.y && tiles[tj].w == sb; ++tj) b1 += tiles[tj].y;
-    const int hi = max(ti.w, sb), lo = min(ti.w, sb);
-    const size_t key = (size_t)ti.z * n_spairs + hi * (hi + 1) / 2 + lo;
-    const float4 *src = tab + key * n_cells * 2;
-    __syncthreads();
-    if (TAB_SMEM)
-      for (int i = threadIdx.x; i < 2 * n_cells; i += kAdjBlock)
-        stab[i] = src[i];
-    for (int c0 = b0; c0 < b1; c0 += kAdjBlock) {
-      const int nb = min(kAdjBlock, b1 - c0);
-      __syncthreads();
-      if ((int)threadIdx.x < nb) {
-        const float4 q = load_atom(pos, perm, c0 + threadIdx.x);
-        const SplitAtom s = split_atom(q.x, q.y, q.z);
-        sB[0][threadIdx.x] = make_float4(s.hx, s.hy, s.hz, s.lx);
-        sB[1][threadIdx.x] = make_float4(s.ly, s.lz, 0.f, 0.f);
-      }
-      __syncthreads();
-      auto sweep = [&](auto checked) {
-        constexpr bool CHECK = decltype(checked)::value;
+  for (int task = warp; task < len * shares; task += W) {
+    const int jl = task / shares, tj = it.y + jl;
+    const int4 tJ = tiles[tj];
+    const bool diag = tj == it.x;
+    const float4 q = load_atom(pos, perm, tJ.x + min(lane, tJ.y - 1));
+    SplitAtom mine = split_atom(q.x, q.y, q.z);
+    if (lane >= tJ.y) mine.hx += 2.0f;
+    __syncwarp();
+    sJ[warp][lane][0] = make_float4(mine.hx, mine.hy, mine.hz, mine.lx);
+    sJ[warp][lane][1] = make_float4(mine.ly, mine.lz, 0.f, 0.f);
+    __syncwarp();
+    const int s0 = (task % shares) * per, s1 = s0 + per;
+    float jx = 0.f, jy = 0.f, jz = 0.f;
 #pragma unroll 2
-        for (int i = warp; i < nb; i += kAdjBlock / 32) {
-          const bool self = CHECK && c0 + i == ia;
-          const float4 q0 = sB[0][i];
-          const float2 q1 = *reinterpret_cast<const float2 *>(&sB[1][i]);
-          SplitAtom b{q0.x, q0.y, q0.z, q0.w, q1.x, q1.y};
-          if (CHECK && self) b.hx += 1.0f;  // any distance but 0
-          const PairDist p = pair_dist(a, b);
-          float uh, ul;
-          grid_pos(gs, p.r, p.rl, uh, ul);
-          const float sg = uh < 0.f ? -1.0f : 1.0f;
-          uh *= sg;
-          ul *= sg;
-          const float fj = rintf(uh);
-          const float t = (uh - fj) + ul;
-          const int j = min(max((int)fj, 0), n_cells - 1);
-          const float4 *cp = TAB_SMEM ? stab + 2 * j : src + 2 * j;
-          const float4 lo4 = cp[0], hi4 = cp[1];
-          // value and derivative together
-          float v = hi4.w, d = hi4.w;
-          v = fmaf(v, t, hi4.z);
-          d = fmaf(d, t, v);
-          v = fmaf(v, t, hi4.y);
-          d = fmaf(d, t, v);
-          v = fmaf(v, t, hi4.x);
-          d = fmaf(d, t, v);
-          v = fmaf(v, t, lo4.w);
-          d = fmaf(d, t, v);
-          v = fmaf(v, t, lo4.z);
-          d = fmaf(d, t, v);
-          v = fmaf(v, t, lo4.y);
-          d = fmaf(d, t, v);
-          v = fmaf(v, t, lo4.x);
-          float s = fmaf(gs.hi, d, -(sg * v) * p.inv_r) *
-                    (p.inv_r * p.inv_r);
-          if (CHECK && self) s = 0.f;
-          gx = fmaf(s, p.dx, gx);
-          gy = fmaf(s, p.dy, gy);
-          gz = fmaf(s, p.dz, gz);
-        }
-      };
-      if (c0 < ti.x + ti.y && ti.x < c0 + nb)
-        sweep(BoolTag<true>());
-      else
-        sweep(BoolTag<false>());
+    for (int s = s0; s < s1; ++s) {
+      const int bl = (lane + s) & (kTile - 1);
+      const float4 q0 = sJ[warp][bl][0];
+      const float2 q1 = *reinterpret_cast<const float2 *>(&sJ[warp][bl][1]);
+      SplitAtom b{q0.x, q0.y, q0.z, q0.w, q1.x, q1.y};
+      const bool self = diag && s == 0;
+      if (self) b.hx += 1.0f;  // any distance but 0
+      const PairDist p = pair_dist(a, b);
+      float uh, ul;
+      grid_pos(gs, p.r, p.rl, uh, ul);
+      const float sg = uh < 0.f ? -1.0f : 1.0f;
+      uh *= sg;
+      ul *= sg;
+      const float fj = rintf(uh);
+      const float t = (uh - fj) + ul;
+      const int j = min(max((int)fj, 0), n_cells - 1);
+      const float4 lo4 = TAB_SMEM ? stab[j] : src[2 * j];
+      const float4 hi4 = TAB_SMEM ? stab[n_cells + j] : src[2 * j + 1];
+      // value and derivative together
+      float v = hi4.w, d = hi4.w;
+      v = fmaf(v, t, hi4.z);
+      d = fmaf(d, t, v);
+      v = fmaf(v, t, hi4.y);
+      d = fmaf(d, t, v);
+      v = fmaf(v, t, hi4.x);
+      d = fmaf(d, t, v);
+      v = fmaf(v, t, lo4.w);
+      d = fmaf(d, t, v);
+      v = fmaf(v, t, lo4.z);
+      d = fmaf(d, t, v);
+      v = fmaf(v, t, lo4.y);
+      d = fmaf(d, t, v);
+      v = fmaf(v, t, lo4.x);
+      float f = fmaf(gs.hi, d, -(sg * v) * p.inv_r) * (p.inv_r * p.inv_r);
+      if (!here || bl >= tJ.y || self) f = 0.f;
+      gx = fmaf(f, p.dx, gx);
+      gy = fmaf(f, p.dy, gy);
+      gz = fmaf(f, p.dz, gz);
+      jx = fmaf(-f, p.dx, jx);
+      jy = fmaf(-f, p.dy, jy);
+      jz = fmaf(-f, p.dz, jz);
+      if (s + 1 < s1) {
+        const int from = (lane + 1) & (kTile - 1);
+        jx = __shfl_sync(0xffffffffu, jx, from);
+        jy = __shfl_sync(0xffffffffu, jy, from);
+        jz = __shfl_sync(0xffffffffu, jz, from);
+      }
     }
+    // (in its own tile every atom has its row on the i side already)
+    if (diag) jx = jy = jz = 0.f;
+    const int bl = (lane + s1 - 1) & (kTile - 1);
+    float *o = shares == 1 ? pj + (size_t)jl * kTile * 3 : &sjac[task][0][0];
+    o[bl * 3] = jx;
+    o[bl * 3 + 1] = jy;
+    o[bl * 3 + 2] = jz;
   }
   sred[warp][lane][0] = gx;
   sred[warp][lane][1] = gy;
   sred[warp][lane][2] = gz;
   __syncthreads();
-  if ((int)threadIdx.x < ti.y * 3) {
-    const int al = threadIdx.x / 3, c = threadIdx.x % 3;
+  float *pi = part + ioff[item];
+  for (int i = threadIdx.x; i < kTile * 3; i += kAdjBlock) {
     float sum = 0.f;
-    for (int g = 0; g < kAdjBlock / kTile; ++g) sum += sred[g][al][c];
-    grad[(size_t)perm[ti.x + al] * 3 + c] = sum;
+    for (int g = 0; g < W; ++g) sum += (&sred[g][0][0])[i];
+    pi[i] = sum;
   }
+  if (shares > 1)
+    for (int i = threadIdx.x; i < len * kTile * 3; i += kAdjBlock) {
+      const int jl = i / (kTile * 3), c = i % (kTile * 3);
+      float sum = 0.f;
+      for (int g = 0; g < shares; ++g)
+        sum += (&sjac[jl * shares + g][0][0])[c];
+      pj[i] = sum;
+    }
 }
 
 }  // namespace pyiid

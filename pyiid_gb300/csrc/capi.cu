@@ -2164,17 +2164,25 @@ int pyiid_batch_potential_grad(pyiid_ctx *ctx, const float *positions,
       LAUNCH_CHECK(ctx);
     }
     const GridScale gs = grid_scale(qstep, m);
+    TRY(ensure(ctx, "b_adjpart", std::max<size_t>(L->adj_total, 1) * sizeof(float),
+               &p));
+    float *part = static_cast<float *>(p);
     const size_t smem = (size_t)n_cells * 2 * sizeof(float4);
-    if (smem <= kAdjTabSmem)
-      adjoint_grid_kernel<true>
-          <<<(unsigned)L->tiles.size(), kAdjBlock, smem, ctx->stream>>>(
-              positions, L->d_perm, L->d_tiles, L->d_cfg_tiles, gs, n_cells,
-              gtab, L->n_spairs, grad);
-    else
-      adjoint_grid_kernel<false>
-          <<<(unsigned)L->tiles.size(), kAdjBlock, 0, ctx->stream>>>(
-              positions, L->d_perm, L->d_tiles, L->d_cfg_tiles, gs, n_cells,
-              gtab, L->n_spairs, grad);
+    // Staged where an item has several tile pairs to share its copy of the
+    // table (64 x 1,000 atoms, runs of up to 32: the call takes 501 us, through
+    // L1 530; 16 x 1,000: 183 and 196).  Where every item is one tile pair
+    // the copy costs what it saves or more (16 x 309: 93.5 us, through L1
+    // 91.7; one 1,000-atom particle 67.2 and 65.8).
+    const size_t tile_pairs = L->adj_total / (kTile * 3) - L->items.size();
+    const bool staged = smem <= kAdjTabSmem && tile_pairs > L->items.size();
+    (staged ? adjoint_grid_kernel<true> : adjoint_grid_kernel<false>)<<<
+        (unsigned)L->items.size(), kAdjBlock, staged ? smem : 0, ctx->stream>>>(
+        positions, L->d_perm, L->d_tiles, L->d_items, L->d_item_order, gs,
+        n_cells, gtab, L->d_adj_ioff, L->d_adj_joff, part);
+    LAUNCH_CHECK(ctx);
+    adjoint_reduce_kernel<<<(unsigned)L->tiles.size(), 96, 0, ctx->stream>>>(
+        part, L->d_adj_tile_ptr, L->d_adj_entries, L->d_tiles, L->d_perm,
+        (int)L->tiles.size(), grad);
     LAUNCH_CHECK(ctx);
     return PYIID_OK;
   }

@@ -81,6 +81,40 @@ def test_pair_force_table_matches_oracle(D, sizes, species, exp, shift, kind):
         assert rel(g[a:b], tg) <= TOL_G, (i, rel(g[a:b], tg))
 
 
+# The length of an item's run of tiles grows with the tile pairs of the call
+# (about four items per SM: one tile up to 1,215 pairs; here also two, three,
+# five and nine), and with it how the warps share its steps and where the
+# table is read.  Copies of one configuration need one oracle evaluation.
+@pytest.mark.parametrize('n,species,copies,exp', [
+    (165, 1, 40, {}),
+    (165, 1, 64, {}),
+    (240, 2, 40, {}),
+    (193, 1, 70, {}),
+    (290, 2, 64, {}),
+    (290, 1, 100, {}),
+    (290, 1, 64, {'rmax': 110.0, 'rstep': 0.05}),
+])
+def test_pair_force_of_longer_runs_matches_oracle(D, n, species, copies, exp):
+    import torch
+    e = O.update_experiment(dict({'rstep': 0.02, 'rmax': 40.0}, **exp))
+    qb, rg = O.pdf_qbin(e), O.r_grid(e)
+    nb = int(np.floor(e['qmax'] / qb))
+    pos, nums = cluster(n, 11 + n, species)
+    sp, tab = tables(nums, qb, nb)
+    gobs = O.pdf_fft(O.fq(S.fcc_nearest(4.0, 50), np.repeat(tab[:1], 50, 0),
+                          qb), e['rstep'], qb, rg, e['qmin'])
+    out = D.batch_potential_grad(
+        np.tile(pos, (copies, 1)), np.tile(sp, copies),
+        np.arange(copies + 1) * n, tab, qb, e['rstep'], rg, e['qmin'],
+        torch.as_tensor(gobs))
+    g = out['grad'].cpu().numpy().reshape(copies, n, 3)
+    val, tg = O.true_grad_potential(pos, tab[sp], e, gobs)
+    energy = out['energy'][:, 0].cpu().numpy()
+    assert np.all(np.abs(energy - val) <= TOL_F * abs(val))
+    for i in range(copies):
+        assert rel(g[i], tg) <= TOL_G, (i, rel(g[i], tg))
+
+
 def test_pair_force_table_close_and_coincident_pairs(D):
     """Pairs nearer than the split coordinates resolve (0.1 A) take the
     general distance; coincident atoms give NaN rows, the others' stay."""
