@@ -33,13 +33,6 @@ sys.path.insert(0, REPO)
 METRIC = 'exact F(Q)+grad evals/s'
 N_ATOMS, A_PT, SIGMA, SEED = 20000, 3.92, 0.02, 2
 QMIN, QMAX, QBIN = 0.5, 30.0, 0.02
-FLOPS_GRAD_TERM = 20   # flop-equivalents per unordered pair-bin of dF/dx
-FLOPS_F_TERM = 10      # ... of F(Q)
-# FP32 lane operations the packed dF/dx inner loop issues per ordered
-# pair-bin: per two bins 4 FFMA2/FADD2 of the recurrence and the derivative
-# factor plus 3 FFMA2 of the x, y, z accumulation, plus 1 FADD2 of the bin
-# factor (8 packed instructions = 16 lane operations per two bins).
-LANE_OPS_GRAD_LOOP = 8
 FP32_LANES_PER_SM = 128
 
 
@@ -309,23 +302,25 @@ def run_gpu(args, rank, world, local):
         return None
     g_ms = float(np.mean(t_g))
     f_ms = float(np.mean(t_f))
+    # both paths go through the phase-grid kernels at this size: F and dF/dx
+    # from one spreading launch, or one each
     if one_pass:
-        # the F and dF/dx of a step come from one launch: its time is t_f
-        kernel = 'fqgrad2_kernel'
-        k_ms = f_ms
+        kernel, k_ms = 'grad_spread_kernel', f_ms
         kernel_ms = {'fq_grad': f_ms}
-        flops_term = FLOPS_GRAD_TERM + FLOPS_F_TERM
-        # F(Q) adds 1 lane op per ordered pair-bin on the tiles J >= I
-        lane_ops = LANE_OPS_GRAD_LOOP + 0.5
     else:
-        kernel = ('gradfq2_kernel' if (tuned is None or
-                                       tuned['grad_fq']['pairs_per_thread']
-                                       <= 0) else 'gradfq_kernel')
-        k_ms = g_ms
+        kernel, k_ms = 'grad_spread_kernel', g_ms
         kernel_ms = {'fq': f_ms, 'grad_fq': g_ms}
-        flops_term = FLOPS_GRAD_TERM
-        lane_ops = LANE_OPS_GRAD_LOOP
-    achieved = pairs * k_ret * flops_term / (k_ms * 1e-3) / 1e12
+    sm_mhz = clk.summary().get('sm_mhz') or 2070.0
+    roofline = grid_roofline(torch, [(kernel, 2 * pairs)], k_ms, sm_mhz)
+    out_bytes = 4 * (3 * n * n_bins + n_bins)
+    hbm = measured_hbm_gbs()
+    if hbm:
+        gbs = (out_bytes + 12 * n) / (ms_step * 1e-3) / 1e9
+        roofline['hbm'] = {
+            'achieved': gbs, 'peak': hbm, 'unit': 'GB/s', 'frac': gbs / hbm,
+            'counted': 'positions read and F, dF/dx written once',
+            'peak_source': 'MEASURED_PEAKS.json hbm_gbs (measured copy)'}
+    roofline['fp32_peak_tflops'] = peak
     line = {
         'metric': METRIC, 'value': value, 'unit': 'evals/s', 'n_gpus': world,
         'steps': args.steps, 'warmup': args.warmup, 'ms_per_step': ms_step,
@@ -345,27 +340,9 @@ def run_gpu(args, rank, world, local):
                 'd2h_bytes_per_step': int(h_fq.numel() * 4 + h_grad.numel() * 4),
                 'path': e2e_path,
                 'ms_copy_out': e2e_copy_ms, 'ms_kernels_write_host': e2e_host_ms},
-        'roofline': {
-            'bound': 'fp32',
-            'kernel': kernel,
-            'achieved': achieved, 'peak': peak, 'unit': 'TFLOP/s',
-            'frac': achieved / peak if peak else None,
-            'peak_source': 'measured live: cuBLAS SGEMM 8192^3 (TF32 off)',
-            'algorithmic_flops_per_launch': pairs * k_ret * flops_term,
-            'traffic': traffic_from_profile(kernel),
-        },
+        'roofline': roofline,
         'clocks': clk.summary(),
     }
-    line['roofline']['issue'] = issue_roofline(
-        torch, dev, pairs, k_ret, k_ms, line['clocks'].get('sm_mhz'), kernel,
-        lane_ops)
-    # the same launch against HBM: its ncu DRAM bytes over its time
-    hbm, traffic = measured_hbm_gbs(), line['roofline']['traffic']
-    if hbm and traffic:
-        gbs = traffic / (k_ms * 1e-3) / 1e9
-        line['roofline']['hbm'] = {
-            'achieved': gbs, 'peak': hbm, 'unit': 'GB/s', 'frac': gbs / hbm,
-            'peak_source': 'MEASURED_PEAKS.json hbm_gbs (measured copy)'}
     if workloads:
         hmc, nuts = (workloads.get('hmc_64_chains_au1000'),
                      workloads.get('nuts_64_chains_au1000'))
@@ -489,23 +466,30 @@ def run_gpu_sharded(args, rank, world, local):
     }
 
 
-def issue_roofline(torch, dev, pairs, k_ret, k_ms, sm_mhz, kernel, lane_ops):
-    """FP32 issue roofline of the dF/dx (or one-pass F + dF/dx) launch:
-    lane operations its inner loop issues per second (each unordered
-    pair-bin is evaluated for both atoms) over the SMs' FP32 lane capacity
-    at the median SM clock sampled during the timed region.  Seeds and pair
-    records are not counted."""
-    if kernel not in ('gradfq2_kernel', 'fqgrad2_kernel') or not sm_mhz:
-        return None
-    sms = torch.cuda.get_device_properties(dev).multi_processor_count
-    achieved = 2 * pairs * k_ret * lane_ops / (k_ms * 1e-3) / 1e12
-    peak = sms * FP32_LANES_PER_SM * sm_mhz * 1e6 / 1e12
-    return {'lane_ops_per_ordered_pair_bin': lane_ops,
-            'achieved': achieved, 'peak': peak, 'unit': 'T lane-op/s',
+# warp instructions per pair of the pair kernels (ncu, smsp__inst_executed over
+# the pairs): unordered pairs of F(Q) and of the force table (64 x 1,000 atoms),
+# ordered pairs of the gradient (2,001 atoms; counted without F, so low for the
+# pass that sums F beside it)
+GRID_INST_PER_PAIR = {'fq_spread_kernel': 4.95, 'adjoint_grid_kernel': 3.87,
+                      'grad_spread_kernel': 16.4}
+
+
+def grid_roofline(torch, counted, ms, sm_mhz=2070.0):
+    """Issue roofline of calls through the phase-grid kernels: the warp
+    instructions of their pair loops ([(kernel, pairs)]; transforms and
+    reductions not counted) per second of the whole call, over four a cycle
+    and SM.  The work of a pair does not grow with the bins there, so pair-bin
+    operations no longer measure it."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    inst = sum(GRID_INST_PER_PAIR[k] * n for k, n in counted)
+    achieved = inst / (ms * 1e-3) / 1e12
+    peak = sms * 4 * sm_mhz * 1e6 / 1e12
+    return {'bound': 'instruction issue',
+            'kernel': ' + '.join(k for k, _ in counted),
+            'achieved': achieved, 'peak': peak, 'unit': 'T warp-inst/s',
             'frac': achieved / peak,
-            'peak_source': f'{sms} SMs x {FP32_LANES_PER_SM} FP32 lanes x '
-                           f'{sm_mhz:.0f} MHz (median sampled clock)',
-            'counted': 'inner loop only (per-pair seeds and records excluded)'}
+            'peak_source': f'{sms} SMs x 4 schedulers x {sm_mhz:.0f} MHz',
+            'counted': 'pair loops only, over the whole call'}
 
 
 def time_ms(torch, fn, reps):
@@ -556,8 +540,8 @@ def batched_workload():
 
 def run_batched(torch, steps=5):
     """Configuration 3: F(Q) of all 256 configurations per step, one graph
-    replay (one pair-sum launch + one finishing launch), with the F(Q) launch
-    shape tuned on this batch."""
+    replay, with the F(Q) launch shape of the small alloys' direct kernels
+    tuned on this batch."""
     from pyiid_gb300 import autotune
     with autotune.variant_scope():
         return _run_batched(torch, steps)
@@ -613,28 +597,21 @@ def _run_batched(torch, steps):
     persistent = info['pairs_per_thread'] == -13
     pairs = int(np.sum(sizes.astype(np.int64) * (sizes - 1) // 2))
     assert torch.isfinite(out).all()
-    # FP32 issue roofline: the F(Q) loop issues 3 lane-ops per unordered
-    # pair-bin (per two bins: FFMA2 + FFMA2 recurrence, FADD2/FFMA2 sum)
-    sms = torch.cuda.get_device_properties(0).multi_processor_count
-    lane_peak = sms * FP32_LANES_PER_SM * 2.07e9 / 1e12
-    lane = pairs * 498 * 3 / (ms * 1e-3) / 1e12
     return {'workload': '256 fcc Au/Pt alloys, N~U{55..2000}, Q 0.1-25 step 0.05',
             'atoms': int(sizes.sum()), 'pairs': pairs,
-            'roofline': {'bound': 'fp32 issue', 'kernel': 'fq_pair3_kernel',
-                         'achieved': lane, 'peak': lane_peak,
-                         'unit': 'T lane-op/s', 'frac': lane / lane_peak,
-                         'counted': '3 lane-ops per unordered pair-bin, '
-                                    'whole batch (pair sums and finish)'},
+            'roofline': dict(
+                grid_roofline(torch, [('fq_spread_kernel', pairs)], ms),
+                note='pairs of the small alloys, which take the direct '
+                     'kernels, counted as the others'),
             'ms_per_batch': ms, 'configs_per_s': len(sizes) / (ms * 1e-3),
             'pair_bin_terms_per_s': pairs * 498 / (ms * 1e-3),
             'fq_variant': best,
             'fq_shape': {'bins_per_thread': info['bins_per_thread'],
                          'persistent': persistent},
             'launch_forms': forms,
-            'launch': ('CUDA graph replay: counter reset + 1 persistent '
-                       'pair-sum + 1 finishing kernel') if persistent else
-                      ('CUDA graph replay: 1 pair-sum (one CTA per work '
-                       'unit) + 1 finishing kernel')}
+            'launch': 'CUDA graph replay: extents, spreading, sums and '
+                      'transform of the larger alloys, pair sums and finish '
+                      'of the smallest'}
 
 
 def run_fq_grad_au1000(torch, reps=100, cpu_reps=2):
@@ -735,20 +712,7 @@ def _run_fq_grad_au1000(torch, reps, cpu_reps):
     cpu = 1.0 / float(np.mean(t))
     gpu = 1e3 / ms
     single = single_config_au1000(torch)
-    # the one-pass kernel's FP32 issue roofline at this size: lane operations
-    # of its inner loop (8.5 per ordered pair-bin) over 152 SMs x 128 lanes
-    # at the maximum SM clock, with the whole call's time (kernel, part
-    # combine and finish)
-    k_ret = n_bins - k_begin
-    sms = torch.cuda.get_device_properties(0).multi_processor_count
-    lane_peak = sms * FP32_LANES_PER_SM * 2.07e9 / 1e12
-    lane = 2 * pairs * k_ret * (LANE_OPS_GRAD_LOOP + 0.5) / (ms * 1e-3) / 1e12
-    roof = {'bound': 'fp32 issue', 'kernel': 'fqgrad2_kernel',
-            'achieved': lane, 'peak': lane_peak, 'unit': 'T lane-op/s',
-            'frac': lane / lane_peak,
-            'peak_source': f'{sms} SMs x {FP32_LANES_PER_SM} lanes x 2070 MHz',
-            'flop_eq_tflops': pairs * k_ret * (FLOPS_GRAD_TERM +
-                                               FLOPS_F_TERM) / (ms * 1e-3) / 1e12}
+    roof = grid_roofline(torch, [('grad_spread_kernel', 2 * pairs)], ms)
     return {'workload': '1000-atom fcc Au, exact F(Q) + full dF/dx, '
                         'Q 0.1-25 step 0.05 (498 bins returned)',
             'pairs': pairs, 'ms_per_eval': ms, 'evals_per_s': gpu,
@@ -946,21 +910,11 @@ def _run_hmc(torch, iters):
     e1.record()
     e1.synchronize()
     ev_ms = e0.elapsed_time(e1) / 3
-    # one evaluation = F(Q) of the 64 configurations (3 lane-ops per unordered
-    # pair-bin) + the symmetric adjoint (5 lane-ops per unordered pair-bin)
-    # on the PDF grid
-    k_pdf = pot.n_bins
     pairs64 = 64 * 1000 * 999 // 2
-    sms = torch.cuda.get_device_properties(0).multi_processor_count
-    lane_peak = sms * FP32_LANES_PER_SM * 2.07e9 / 1e12
-    lane = pairs64 * k_pdf * (3 + 5) / (ev_ms * 1e-3) / 1e12
     return {'workload': '1000-atom fcc Au, 64 chains, 10 leapfrog x dt 1e-3, 300 K, E = 100 Rw',
-            'roofline': {'bound': 'fp32 issue',
-                         'kernel': 'fq_pair3_kernel + adjoint_sym_kernel',
-                         'achieved': lane, 'peak': lane_peak,
-                         'unit': 'T lane-op/s', 'frac': lane / lane_peak,
-                         'counted': '3 (F) + 5 (adjoint) lane-ops per '
-                                    'unordered pair-bin, whole evaluation'},
+            'roofline': grid_roofline(
+                torch, [('fq_spread_kernel', pairs64),
+                        ('adjoint_grid_kernel', pairs64)], ev_ms),
             'hmc_iterations_per_s': iters / s,
             'accepted_steps_per_s': acc / s,
             'acceptance': acc / (iters * 64),
