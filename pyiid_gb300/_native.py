@@ -181,7 +181,7 @@ class Context:
         """Call entry point ``name`` on the given (or torch's current) stream."""
         if stream is None:
             import torch
-            stream = torch.cuda.current_stream(self.device).cuda_stream
+            stream = torch._C._cuda_getCurrentRawStream(self.device)
         with self._call_lock:
             self.check(self._lib.pyiid_set_stream(self.handle, _vp(stream)),
                        'pyiid_set_stream')
@@ -209,6 +209,9 @@ _contexts = {}
 
 def context(device=None):
     """The per-device shared :class:`Context` (created on first use)."""
+    ctx = _contexts.get(device)  # (None is never a key)
+    if ctx is not None:
+        return ctx
     import torch
     if not torch.cuda.is_available():
         raise NativeError('no CUDA device is visible; pyiid_gb300 runs only '

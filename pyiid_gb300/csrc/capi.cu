@@ -167,21 +167,35 @@ size_t fq_smem(const FqVariant &v, int n_chunks = -1) {
 }
 
 // Cache key of host arrays (r grids, species, form-factor tables) that are
-// hashed on every call: eight bytes per step (an FNV-style multiply followed
-// by an xor-shift so that high bits reach the low ones), then the tail byte
-// by byte.  A 4,000-point r grid takes a few microseconds.
+// hashed on every call: four FNV-style streams of eight-byte words (a multiply
+// followed by an xor-shift so that high bits reach the low ones; one stream
+// alone waits for its multiply, 9 us for a 4,000-point r grid), joined at the
+// end, then the tail byte by byte.
 uint64_t fnv1a(const void *data, size_t n, uint64_t h = 1469598103934665603ull) {
+  constexpr uint64_t kPrime = 1099511628211ull;
   const unsigned char *p = static_cast<const unsigned char *>(data);
   size_t i = 0;
-  for (; i + 8 <= n; i += 8) {
+  auto step = [&](uint64_t s, size_t at) {
     uint64_t w;
-    std::memcpy(&w, p + i, 8);
-    h = (h ^ w) * 1099511628211ull;
-    h ^= h >> 29;
+    std::memcpy(&w, p + at, 8);
+    s = (s ^ w) * kPrime;
+    return s ^ (s >> 29);
+  };
+  if (n >= 64) {
+    uint64_t s[4] = {h, h ^ 0x9e3779b97f4a7c15ull, h ^ 0xbf58476d1ce4e5b9ull,
+                     h ^ 0x94d049bb133111ebull};
+    for (; i + 32 <= n; i += 32)
+      for (int q = 0; q < 4; ++q) s[q] = step(s[q], i + 8 * q);
+    for (int q = 1; q < 4; ++q) {
+      s[0] = (s[0] ^ s[q]) * kPrime;
+      s[0] ^= s[0] >> 29;
+    }
+    h = s[0];
   }
+  for (; i + 8 <= n; i += 8) h = step(h, i);
   for (; i < n; ++i) {
     h ^= p[i];
-    h *= 1099511628211ull;
+    h *= kPrime;
   }
   return h;
 }

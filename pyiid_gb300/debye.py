@@ -22,12 +22,17 @@ _f32p = None
 
 
 def _np(a, dtype):
+    if type(a) is np.ndarray and a.ndim and a.dtype == dtype and \
+            a.flags.c_contiguous:  # (0-d becomes [1] below)
+        return a
     return np.ascontiguousarray(np.asarray(a, dtype=dtype))
 
 
 def _ptr(a, ctype):
-    import ctypes
-    return a.ctypes.data_as(ctypes.POINTER(ctype))
+    """The first element of ``a``, which ctypes passes by reference (the
+    caller holds the array while the library reads it; a third of the time
+    of ndarray.ctypes.data_as)."""
+    return ctype.from_address(a.__array_interface__['data'][0])
 
 
 _cuda_seen = False
@@ -61,6 +66,7 @@ def _check_packed(n_rows, sp, off, tab):
         raise NativeError(f'offsets cover {total} atoms: positions has '
                           f'{n_rows} rows, species {list(sp.shape)}, '
                           f'scatter must be [S, K] (got {list(tab.shape)})')
+    return total
 
 
 def _require_cuda():
@@ -76,6 +82,10 @@ def _dev_tensor(t, dtype, device=None):
     """Contiguous CUDA tensor of ``dtype`` from a tensor or an array.  Host
     data is copied to the device: the library dereferences device
     pointers only."""
+    if type(t) is torch.Tensor and t.is_cuda and t.dtype == dtype and \
+            not t.requires_grad and t.is_contiguous() and \
+            (device is None or t.device == device):
+        return t
     _require_cuda()
     if not isinstance(t, torch.Tensor):
         t = torch.as_tensor(np.asarray(t))
@@ -93,6 +103,10 @@ def _check_len(t, n, name):
 def as_positions(x, device=None):
     """float32 contiguous CUDA tensor [N, 3] from an array or tensor (any
     leading shape with x, y, z last, e.g. [B, N, 3], is flattened)."""
+    if type(x) is torch.Tensor and x.is_cuda and x.dim() == 2 and \
+            x.shape[1] == 3 and x.dtype == torch.float32 and \
+            not x.requires_grad and x.is_contiguous():
+        return x
     _positions_shape(x)
     _require_cuda()
     if isinstance(x, torch.Tensor):
@@ -403,7 +417,7 @@ def batch_potential_grad(positions, species, offsets, scatter, qstep, rstep,
     sp = _np(species, np.int32)
     off = _np(offsets, np.int32)
     tab = _np(scatter, np.float32)
-    _check_packed(pos.numel() // 3, sp, off, tab)
+    total = _check_packed(pos.numel() // 3, sp, off, tab)
     rg = _np(rgrid, np.float64)
     b = len(off) - 1
     dev = pos.device
@@ -427,9 +441,9 @@ def batch_potential_grad(positions, species, offsets, scatter, qstep, rstep,
             _check_len(out[key], size, key)
         if want_grad and out.get('grad') is not None:
             _check_dev(out['grad'], 'grad', torch.float32)
-            if out['grad'].numel() < 3 * int(off.max()):
+            if out['grad'].numel() < 3 * total:
                 raise NativeError(f'grad has {out["grad"].numel()} values, '
-                                  f'the offsets cover {int(off.max())} atoms')
+                                  f'the offsets cover {total} atoms')
     ctx = context(dev.index)
     g = out.get('grad') if want_grad else None
     ctx.call('pyiid_batch_potential_grad', ctypes.c_void_p(pos.data_ptr()),

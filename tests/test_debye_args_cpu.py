@@ -150,3 +150,22 @@ def test_surrogate_checks_its_device_buffers(monkeypatch):
     assert calls == []
     g = sur.backward(np.array([0.5, -1.0]))   # host values are accepted
     assert calls == ['pyiid_mlp_backward'] and set(g) == set(sur.params)
+
+
+@pytest.mark.parametrize('a', [
+    np.arange(6, dtype=np.int32), np.arange(6, dtype=np.int64),
+    np.arange(6, dtype='>i4'), np.arange(12, dtype=np.int32)[::2],
+    np.asfortranarray(np.arange(6, dtype=np.int32).reshape(2, 3)),
+    np.array(3, dtype=np.int32), np.empty(0, np.int32), [1, 2, 3], 4])
+def test_host_arrays_as_the_library_reads_them(a):
+    """Any array or sequence arrives as ascontiguousarray gives it (0-d as
+    [1]), and its pointer reads and writes that array."""
+    import ctypes
+    from pyiid_gb300 import debye
+    want = np.ascontiguousarray(np.asarray(a, dtype=np.int32))
+    got = debye._np(a, np.int32)
+    assert got.dtype == want.dtype and got.shape == want.shape
+    assert got.flags.c_contiguous and np.array_equal(got, want)
+    p = ctypes.byref(debye._ptr(got, ctypes.c_int32))
+    p = ctypes.cast(p, ctypes.POINTER(ctypes.c_int32))
+    assert [p[i] for i in range(got.size)] == want.ravel().tolist()
