@@ -2399,30 +2399,45 @@ static int mh_step_reset(pyiid_ctx *ctx, const MhStep &S) {
   return PYIID_OK;
 }
 
-static int mh_step_launch(pyiid_ctx *ctx, const MhStep &S, float *positions,
+// chained: the stream's last launch is move_gram_kernel of the step before,
+// so that move_delta_kernel may start while it drains; anything else
+// (uploads, counters just cleared) is waited for in full.
+static int mh_step_launch(pyiid_ctx *ctx, const MhStep &S, bool chained,
+                          float *positions,
                           uint64_t *counter, uint64_t seed, float sigma,
                           HostMoves hm, int potential, double beta,
                           double *energy, int64_t *accepted, double *trace,
                           double *eval_out) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.stream = ctx->stream;
+  cfg.attrs = &attr;
   if (S.n_mi > 0) {
-    dim3 g1(S.n_mi, S.n_cb);
-    move_delta_kernel<<<g1, kBlock, S.smem, ctx->stream>>>(
-        positions, S.L->d_perm, S.L->d_tiles, S.L->d_mitems,
-        S.L->d_mitem_begin, S.L->d_offsets, S.L->d_species,
-        reinterpret_cast<const unsigned long long *>(counter), (uint32_t)seed,
-        (uint32_t)(seed >> 32), sigma, S.dq_hi, S.dq_lo, S.kb0, S.kmin,
-        S.n_chunks, S.n_groups, S.n_bins, S.ftab, S.na, S.st, S.n_configs,
-        S.kp, hm, S.prop, S.part, S.done, S.fsum, S.fdif);
-    LAUNCH_CHECK(ctx);
+    cfg.gridDim = dim3(S.n_mi, S.n_cb);
+    cfg.blockDim = dim3(kBlock);
+    cfg.dynamicSmemBytes = S.smem;
+    cfg.numAttrs = chained ? 1 : 0;
+    CUDA_TRY(ctx, cudaLaunchKernelEx(
+        &cfg, move_delta_kernel, (const float *)positions, S.L->d_perm,
+        S.L->d_tiles, S.L->d_mitems, S.L->d_mitem_begin, S.L->d_offsets,
+        S.L->d_species, reinterpret_cast<const unsigned long long *>(counter),
+        (uint32_t)seed, (uint32_t)(seed >> 32), sigma, S.dq_hi, S.dq_lo, S.kb0,
+        S.kmin, S.n_chunks, S.n_groups, S.n_bins, S.ftab, S.na, S.st,
+        S.n_configs, S.kp, hm, S.prop, S.part, S.done, S.fsum, S.fdif));
+    chained = true;
   }
-  dim3 gg(S.n_rb, S.n_cg);
-  move_gram_kernel<<<gg, 256, S.gram_smem, ctx->stream>>>(
-      S.T->d_M32, S.fsum, S.fdif, S.kp, S.L->d_offsets, S.prop, S.st,
-      S.n_configs, S.n_bins, S.kmin, potential, beta, S.gpart,
-      S.done + S.n_configs, positions, energy,
+  cfg.gridDim = dim3(S.n_rb, S.n_cg);
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = S.gram_smem;
+  cfg.numAttrs = chained ? 1 : 0;
+  CUDA_TRY(ctx, cudaLaunchKernelEx(
+      &cfg, move_gram_kernel, S.T->d_M32, S.fsum, S.fdif, S.kp,
+      S.L->d_offsets, S.prop, S.st, S.n_configs, S.n_bins, S.kmin, potential,
+      beta, S.gpart, S.done + S.n_configs, positions, energy,
       reinterpret_cast<unsigned long long *>(counter),
-      reinterpret_cast<long long *>(accepted), trace, eval_out);
-  LAUNCH_CHECK(ctx);
+      reinterpret_cast<long long *>(accepted), trace, eval_out));
   return PYIID_OK;
 }
 
@@ -2448,7 +2463,7 @@ int pyiid_mh_steps(pyiid_ctx *ctx, float *positions, const int32_t *species,
   TRY(mh_step_reset(ctx, S));
   const double beta = conv / kT;
   for (int step = 0; step < n_steps; ++step)
-    TRY(mh_step_launch(ctx, S, positions, counter, seed, sigma, HostMoves{},
+    TRY(mh_step_launch(ctx, S, step > 0, positions, counter, seed, sigma, HostMoves{},
                        potential, beta, energy, accepted,
                        trace ? trace + (size_t)step * n_configs * 8 : nullptr,
                        nullptr));
@@ -2518,7 +2533,7 @@ int pyiid_mc_propose(pyiid_ctx *ctx, const float *positions,
                                 cudaMemcpyHostToDevice, ctx->stream));
   TRY(mh_step_reset(ctx, S));
   HostMoves hm{d_hp, d_hx, d_na};
-  TRY(mh_step_launch(ctx, S, const_cast<float *>(positions), nullptr, 0, 0.f,
+  TRY(mh_step_launch(ctx, S, false, const_cast<float *>(positions), nullptr, 0, 0.f,
                      hm, potential, 1.0, nullptr, nullptr, nullptr, eval));
   // the host arrays above are read by the copies: wait before returning
   CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));

@@ -145,6 +145,36 @@ def test_graph_replay_equals_eager():
     assert a.state['accepted'].sum().item() > 0
 
 
+# Steps of one call overlap the launches of their kernels, the first of a call
+# does not: the chains are the same bits either way.  One chain and eight or
+# nine (a group of the Gram kernel, and one more), empty and one-atom chains,
+# more than 384 bins (a second block of columns), CTAs beyond one wave.
+@pytest.mark.parametrize('sizes,alloy,exp', [
+    ([64], False, {}),
+    ([40] * 8, True, {}),
+    ([70, 0, 1, 2, 33, 128, 129, 5, 31], True, {}),
+    ([150] * 6, False, {'rmax': 60.0}),
+    ([600] * 48, True, {}),
+])
+def test_steps_of_one_call_equal_single_steps(sizes, alloy, exp):
+    from pyiid_gb300.sampling import SingleAtomMC
+    pot, x0, _, _ = make_potential(sizes, alloy, seed=9,
+                                   exp_dict=dict(EXP, **exp))
+    a = SingleAtomMC(pot, x0, temperature=600, sigma=0.1, seed=4,
+                     resync_every=None)
+    b = SingleAtomMC(pot, x0, temperature=600, sigma=0.1, seed=4,
+                     resync_every=None)
+    a.step(40)
+    for _ in range(40):
+        b.step(1)
+    assert np.array_equal(a.positions().cpu().numpy(),
+                          b.positions().cpu().numpy())
+    for k in ('energy', 'accepted', 'counter'):
+        assert np.array_equal(a.state[k].cpu().numpy(),
+                              b.state[k].cpu().numpy(), equal_nan=k == 'energy')
+    assert a.state['accepted'].sum().item() > 0
+
+
 def test_running_sums_do_not_drift():
     """3000 steps without re-synchronisation: the running sums and energies
     equal a fresh full evaluation of the final positions."""
