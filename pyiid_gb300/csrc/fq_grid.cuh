@@ -216,11 +216,11 @@ __device__ __forceinline__ bool finish_rows(const HistRows &out, int wi,
 // instructions per eight pairs.  Bound by instruction issue and the latency
 // of its dependent chains (0.60 issued per cycle and scheduler): two columns
 // go side by side, and as many warps run as have room for a histogram, 8 per
-// SM at 650 cells.  163 instructions per column; four slots of one tap per
+// SM at 650 cells.  158 instructions per 32 pairs; four slots of one tap per
 // lane, at half the memory per warp, took 248.
-// 64 x 1,000 atoms at 330 bins: 253 us (fq_pair3_kernel 1,451); 256 alloys of
-// 55 to 2,000 atoms at 500 bins 1.45 ms (11.5); 10,007 atoms at 1,500 bins
-// 0.60 ms (9.5).
+// 64 x 1,000 atoms at 330 bins: 224 us (fq_pair3_kernel 1,451); 256 alloys of
+// 55 to 2,000 atoms at 500 bins 1.22 ms (11.5); 10,007 atoms at 1,500 bins
+// 0.49 ms (9.5).
 constexpr int kSpreadSlots = 8;
 constexpr int kSpreadCols = 2;
 constexpr PlanShape kFqPlan{4 * kSpreadSlots, 8};

@@ -102,10 +102,13 @@ __device__ __forceinline__ void sts(int addr, float x) {
 // the 8 cells x (x, y, z, F) of a pair are 32 consecutive words.  What a warp
 // waits for is the chain read - add - write, so four pairs go together when
 // no two of them are within 8 cells (found for all groups of four by three
-// shuffles), one by one otherwise.  Bound by the shared-memory pipe (five
-// passes per pair) and instruction issue (about 14 per pair).
+// shuffles), one by one otherwise.  Bound by the shared-memory pipe (83 %
+// busy; 16.4 instructions per ordered pair fill 64 % of the issue slots).
+// 2,001 atoms, 4.0 M ordered pairs, without F: 90 us; 20,000 atoms with F,
+// 400 M pairs: 9.8 ms (gradfq2_kernel 2,056 us, fqgrad2_kernel 205 ms, whose
+// work grows with the bins too).
 // With WITH_F the fourth word collects sin(Q r)/r (half of each ordered
-// pair) over all units of a block, one partial histogram per warp and block.
+// pair) over all units of a block; finish_rows joins a CTA's partial sums.
 //
 // X needs the true distance of a pair, not the one folded into half a
 // period, r = s r_folded + n P: the rows hold s w, and where any n is not 0
