@@ -160,7 +160,8 @@ struct HostMoves {
 // __restrict__: read-only loads need not stay below the wait.
 // A step is bound by this chain of two kernels, not by a unit (move_delta
 // keeps 23 % of the SM's throughput busy): 64 chains of 1,000 atoms, 330
-// bins, 16 steps take 494 us, with plain launches 569.
+// bins, 16 steps take 494 us, with plain launches 569.  Replayed from a
+// graph a step takes 29.3 us either way.
 __device__ __forceinline__ void await_previous_grid() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
