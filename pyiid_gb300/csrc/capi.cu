@@ -1223,7 +1223,6 @@ int run_fq_grid(pyiid_ctx *ctx, const Layout *L, const FqGridWork *W,
   TRY(hist_rows(ctx, "fqg", W->n_keys, grid_words(m / 2), &rows));
   void *p;
   TRY(ensure(ctx, "fqg_sum",
-  out->low = nullptr;
              (size_t)W->n_keys * fq_sum_floats(m) * sizeof(float), &p));
   float *hsum = static_cast<float *>(p);
   TRY(ensure(ctx, "fqg_ext", (size_t)W->n_cfgs * sizeof(int), &p));
@@ -1277,10 +1276,6 @@ int run_fq(pyiid_ctx *ctx, Layout *L, const float *positions,
       order = W->d_direct_order;
       skip = W->d_skip;
     }
-  TRY(ensure(ctx, "fqg_low",
-             (size_t)kSpreadWarps * n_ctas * rows.row_words * sizeof(float),
-             &p));
-  rows.low = static_cast<float *>(p);
   }
   if (n_items > 0 && kb0 < n_bins) {
     const FqEntry &E = kFqTable[ctx->fq_variant];

@@ -162,7 +162,6 @@ struct HistRows {
   float *rows;  // [n_ctas] rows of the CTAs, then those of the slots
   int *flag;    // [slots]
   int2 *cta;    // [n_ctas]
-  float *low;   // [warps], for sums in float pairs (fq_spread_kernel only)
   int n_ctas, row_words;
   __device__ __forceinline__ float *cta_row(int b) const {
     return rows + (size_t)b * row_words;
@@ -170,19 +169,7 @@ struct HistRows {
   __device__ __forceinline__ float *warp_row(int slot) const {
     return rows + ((size_t)n_ctas + slot) * row_words;
   }
-  // what the additions to a warp's row have rounded away so far
-  __device__ __forceinline__ float *low_row(int warp) const {
-    return low + (size_t)warp * row_words;
-  }
 };
-
-// x into the float pair (s, c)
-__device__ __forceinline__ void pair_add(float x, float &s, float &c) {
-  const float y = __fadd_rn(x, c);
-  const float t = __fadd_rn(s, y);
-  c = __fsub_rn(y, __fsub_rn(t, s));
-  s = t;
-}
 
 // End of a spreading CTA (all threads call it): whether this warp has to
 // write its last key itself.  Else, if s[0] >= 0, the CTA's warps 0 .. s[1]-1
@@ -237,32 +224,6 @@ __device__ __forceinline__ bool finish_rows(const HistRows &out, int wi,
 constexpr int kSpreadSlots = 8;
 constexpr int kSpreadCols = 2;
 constexpr PlanShape kFqPlan{4 * kSpreadSlots, 8};
-
-// the eight copies of word i
-__device__ __forceinline__ float sum_copies(const float4 *hist4, int i) {
-  const float4 v = hist4[2 * i], w = hist4[2 * i + 1];
-  return ((v.x + v.y) + (v.z + v.w)) + ((w.x + w.y) + (w.z + w.w));
-}
-
-// Moves a warp's cells to its row, the float pair (row, low) until `last`.
-// Not inlined: in line it costs the spreading loop 8 registers and 3 to 6 % of
-// its time.
-static __device__ __noinline__ void spill_cells(float4 *hist4, float *row,
-                                                float *low, int words,
-                                                bool add, bool last) {
-  __syncwarp();
-#pragma unroll 4
-  for (int i = threadIdx.x & 31; i < words; i += 32) {
-    float s = add ? row[i] : 0.f, c = add ? low[i] : 0.f;
-    pair_add(sum_copies(hist4, i), s, c);
-    row[i] = last ? s + c : s;
-    if (!last) low[i] = c;
-    hist4[2 * i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    hist4[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  __syncwarp();
-}
-
 __global__ void __launch_bounds__(32 * kSpreadWarps)
     fq_spread_kernel(const float *__restrict__ pos,
                      const int *__restrict__ perm,
@@ -273,7 +234,6 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
                      const float *__restrict__ taps, HistRows out) {
   extern __shared__ float4 smem4[];
   __shared__ int splan[32];
-  __shared__ bool sspill[kSpreadWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const SpreadPlan plan =
       spread_plan(ext, n_cfgs, gridDim.x, kFqPlan, total, splan);
@@ -304,19 +264,20 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
   }
   // tap p of cell j is cell j - 3 + p
   float *const base = hist + (8 + tp) * kSpreadSlots + slot;
-  // The cells go to the warp's row when it leaves a key, and after every
-  // spill_cols columns: a copy of a cell has then taken about 128 values,
-  // where one that grows without limit loses the window's tails.  The row is
-  // a float pair, so the sums do not depend on how many columns a warp gets.
-  const int spill_cols = 4 * words;
-  int since = 0;
-  bool spilled = false;
-  auto spill = [&](int key, bool last) {
-    spill_cells(hist4, out.warp_row(wi + key), out.low_row(wi), words, spilled,
-                last);
-    if (last && lane == 0) out.flag[wi + key] = 1;
-    since = 0;
-    spilled = !last;
+  auto word = [](const float4 *h, int i) {  // the eight copies of word i
+    const float4 v = h[2 * i], w = h[2 * i + 1];
+    return ((v.x + v.y) + (v.z + v.w)) + ((w.x + w.y) + (w.z + w.w));
+  };
+  auto flush = [&](int key) {
+    __syncwarp();
+    float *row = out.warp_row(wi + key);
+    for (int i = lane; i < words; i += 32) {
+      row[i] = word(hist4, i);
+      hist4[2 * i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      hist4[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (lane == 0) out.flag[wi + key] = 1;
+    __syncwarp();
   };
   int cur = -1;
   bool alone = false;
@@ -326,7 +287,7 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
     const int begin = seg_begin[sgi], end = min(seg_begin[sgi + 1], c1);
     if (sg.key != cur) {
       if (cur >= 0) {
-        spill(cur, true);
+        flush(cur);
         alone = true;
       }
       cur = sg.key;
@@ -434,29 +395,19 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
           __syncwarp();
         }
       }
-      since += nb;
-      if (since >= spill_cols) spill(cur, false);
     }
     c = end;
   }
-  if (lane == 0) sspill[warp] = spilled;
   if (finish_rows(out, wi, works ? cur : -1, alone, splan))
-    spill(cur, true);
+    flush(cur);
   else if (splan[0] >= 0)
     for (int i = threadIdx.x; i < words; i += blockDim.x) {
-      float s = 0.f, c = 0.f;
-      for (int w = 0; w < splan[1]; ++w) {
-        if (sspill[w]) {
-          const int wj = blockIdx.x * plan.per_cta + w;
-          pair_add(out.warp_row(wj + splan[0])[i], s, c);
-          pair_add(out.low_row(wj)[i], s, c);
-        }
-        pair_add(sum_copies(smem4 + w * (kSpreadStage / 16 + 2 * words) +
-                                kSpreadStage / 16,
-                            i),
-                 s, c);
-      }
-      out.cta_row(blockIdx.x)[i] = s + c;
+      float s = 0.f;
+      for (int w = 0; w < splan[1]; ++w)
+        s += word(smem4 + w * (kSpreadStage / 16 + 2 * words) +
+                      kSpreadStage / 16,
+                  i);
+      out.cta_row(blockIdx.x)[i] = s;
     }
 }
 
@@ -504,11 +455,17 @@ __device__ __forceinline__ void fq_grid_reduce(
   // the cells that meet in (G-_j, G+_j): j, its mirror images at 0 and M/2
   float hs = 0.f, hc = 0.f, ms = 0.f, mc = 0.f;
   const bool on = j <= quarter, near = j > quarter && j <= quarter + kNearTerms;
+  auto add = [](float x, float &s, float &c) {
+    const float y = __fadd_rn(x, c);
+    const float t = __fadd_rn(s, y);
+    c = __fsub_rn(y, __fsub_rn(t, s));
+    s = t;
+  };
   if (ty < ny && (on || near)) {
     const int j1 = half - j, last = plan.used + 4;
     auto take = [&](const float *r) {
       if (near) {
-        pair_add(r[j - quarter - 1], hs, hc);
+        add(r[j - quarter - 1], hs, hc);
         return;
       }
       r += kGridCell0;
@@ -516,8 +473,8 @@ __device__ __forceinline__ void fq_grid_reduce(
       float x = j <= last ? r[j] : 0.f, y = j1 <= last ? r[j1] : 0.f;
       if (j >= 1 && j <= 3) x -= r[-j];
       if (j >= 1 && half + j <= last) y -= r[half + j];
-      pair_add(x, hs, hc);
-      pair_add(y, ms, mc);
+      add(x, hs, hc);
+      add(y, ms, mc);
     };
     auto own = [&](int w, int key) {
       if (in.cta[w / plan.per_cta].y && in.flag[w + key])
@@ -552,9 +509,9 @@ __device__ __forceinline__ void fq_grid_reduce(
   if (ty != 0 || !(on || near)) return;
   for (int y = 1; y < ny; ++y) {
     const float *sh = sred + y * nx + tx;
-    pair_add(sh[0], hs, hc);
+    add(sh[0], hs, hc);
     hc += sh[st];
-    pair_add(sh[2 * st], ms, mc);
+    add(sh[2 * st], ms, mc);
     mc += sh[3 * st];
   }
   if (near) {
