@@ -215,6 +215,7 @@ struct DevBuf {
 struct FqGridWork {
   int n_bins = 0;
   int n_segs = 0, total = 0, n_keys = 0, n_cfgs = 0;  // n_cfgs 0: no work
+  int n_wide = 0;    // the last of them take the transform in FP64
   int n_direct = 0;  // work items of the other configurations
   GridSeg *d_segs = nullptr;
   int *d_seg_begin = nullptr;
@@ -808,6 +809,10 @@ int set_attrs(pyiid_ctx *ctx) {
                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                     (int)(fq_dft_float4(kFqCellsPerBin * kFqGridMaxBins) *
                           sizeof(float4))));
+  CUDA_TRY(ctx, cudaFuncSetAttribute(
+                    fq_grid_finish_wide_kernel,
+                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                    fq_wide_smem(kFqCellsPerBin * kFqGridMaxBins)));
   // (partial sums of 12,288 bins beside the staged F)
   CUDA_TRY(ctx, cudaFuncSetAttribute(pdf_kernel<1>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -993,6 +998,15 @@ std::vector<int> fq_grid_configs(const Layout *L, int n_bins) {
   return on;
 }
 
+// Whether configuration c's sums are transformed in FP64
+// (fq_grid_finish_wide_kernel).
+bool wide_sums(const Layout *L, int c) {
+  double pairs = 0;
+  for (int s = 0; s < L->n_spairs; ++s)
+    pairs += L->pair_counts[(size_t)c * L->n_spairs + s];
+  return pairs > 1e8;
+}
+
 // The grid path's share of a layout (n_cfgs == 0: none of it).
 int get_fq_grid_work(pyiid_ctx *ctx, Layout *L, int n_bins,
                      FqGridWork **out) {
@@ -1009,7 +1023,11 @@ int get_fq_grid_work(pyiid_ctx *ctx, Layout *L, int n_bins,
   std::vector<KeyCols> cols;  // columns of each key
   std::vector<unsigned char> skip(L->n_configs, 0);
   long long total = 0;
-  for (int c : fq_grid_configs(L, n_bins)) {
+  std::vector<int> on = fq_grid_configs(L, n_bins);
+  const auto wide = std::stable_partition(
+      on.begin(), on.end(), [&](int c) { return !wide_sums(L, c); });
+  W->n_wide = (int)(on.end() - wide);
+  for (int c : on) {
     skip[c] = 1;
     const int first_key = (int)key_spair.size();
     const int t0 = L->cfg_tiles[c].x, t1 = L->cfg_tiles[c].y;
@@ -1205,8 +1223,45 @@ int hist_rows(pyiid_ctx *ctx, const std::string &name, int n_keys,
   out->flag = static_cast<int *>(p);
   TRY(ensure(ctx, (name + "_cta").c_str(), n_ctas * sizeof(int2), &p));
   out->cta = static_cast<int2 *>(p);
+  out->low = nullptr;
   out->n_ctas = n_ctas;
   out->row_words = row_words;
+  return PYIID_OK;
+}
+
+// The transform of the sums to F(Q).
+struct FqFinish {
+  const float *hsum;
+  const int4 *cfg_keys;
+  const int *key_spair;
+  const int2 *spair;
+  const float *ftab;
+  const double *na, *inv_phi;
+  int m, n_bins, kb_out;
+  double qbin;
+  float *fq;
+  double *fq_raw;
+};
+
+// ... of configurations [first, first + n) of a.cfg_keys.
+int launch_fq_finish(pyiid_ctx *ctx, const FqFinish &a, int first, int n,
+                     bool wide) {
+  if (n == 0) return PYIID_OK;
+  const dim3 grid((a.n_bins + 31) / 32, n);
+  const float near_unit = 1.0f / (float)a.n_bins;
+  if (wide)
+    fq_grid_finish_wide_kernel<<<grid, 32 * kFqDftWarps, fq_wide_smem(a.m),
+                                 ctx->stream>>>(
+        a.hsum, a.cfg_keys + first, a.key_spair, a.spair, a.ftab, a.na,
+        a.inv_phi, a.m, a.n_bins, a.kb_out, a.qbin, near_unit, a.fq, a.fq_raw);
+  else
+    fq_grid_finish_kernel<<<grid, 32 * kFqDftWarps,
+                            fq_dft_float4(a.m) * sizeof(float4),
+                            ctx->stream>>>(
+        a.hsum, a.cfg_keys + first, a.key_spair, a.spair, a.ftab, a.na,
+        a.inv_phi, a.m, 1.0f / (float)a.m, a.n_bins, a.kb_out, a.qbin,
+        near_unit, a.fq, a.fq_raw);
+  LAUNCH_CHECK(ctx);
   return PYIID_OK;
 }
 
@@ -1222,6 +1277,10 @@ int run_fq_grid(pyiid_ctx *ctx, const Layout *L, const FqGridWork *W,
   HistRows rows;
   TRY(hist_rows(ctx, "fqg", W->n_keys, grid_words(m / 2), &rows));
   void *p;
+  TRY(ensure(ctx, "fqg_low",
+             (size_t)kSpreadWarps * n_ctas * rows.row_words * sizeof(float),
+             &p));
+  rows.low = static_cast<float *>(p);
   TRY(ensure(ctx, "fqg_sum",
              (size_t)W->n_keys * fq_sum_floats(m) * sizeof(float), &p));
   float *hsum = static_cast<float *>(p);
@@ -1244,13 +1303,10 @@ int run_fq_grid(pyiid_ctx *ctx, const Layout *L, const FqGridWork *W,
       (double)n_ctas / W->n_keys * (W->n_keys > n_ctas / 4 ? kSpreadWarps : 1);
   TRY(launch_grid_reduce(ctx, rows, W->d_key_cols, ext, W->n_cfgs, kFqPlan,
                          W->total, m, W->n_keys, most, hsum));
-  fq_grid_finish_kernel<<<dim3((n_bins + 31) / 32, W->n_cfgs),
-                          32 * kFqDftWarps, fq_dft_float4(m) * sizeof(float4),
-                          ctx->stream>>>(
-      hsum, W->d_cfg_keys, W->d_key_spair, L->d_spair, d_ftab, d_na,
-      G->d_inv_phi, m, 1.0f / (float)m, n_bins, kb_out, qbin,
-      1.0f / (float)n_bins, fq, fq_raw);
-  LAUNCH_CHECK(ctx);
+  const FqFinish fin{hsum, W->d_cfg_keys, W->d_key_spair, L->d_spair, d_ftab,
+                     d_na, G->d_inv_phi, m, n_bins, kb_out, qbin, fq, fq_raw};
+  TRY(launch_fq_finish(ctx, fin, 0, W->n_cfgs - W->n_wide, false));
+  TRY(launch_fq_finish(ctx, fin, W->n_cfgs - W->n_wide, W->n_wide, true));
   return PYIID_OK;
 }
 
@@ -1505,13 +1561,9 @@ int run_grad_grid(pyiid_ctx *ctx, Layout *L, const float *positions,
                                      fsum});
   LAUNCH_CHECK(ctx);
   if (!fq) return PYIID_OK;
-  fq_grid_finish_kernel<<<dim3((n_bins + 31) / 32, 1), 32 * kFqDftWarps,
-                          fq_dft_float4(m) * sizeof(float4), ctx->stream>>>(
-      fsum, W->d_cfg_keys, W->d_key_spair, L->d_spair, d_ftab, d_na,
-      G->d_inv_phi, m, 1.0f / (float)m, n_bins, kbo, qbin,
-      1.0f / (float)n_bins, fq, nullptr);
-  LAUNCH_CHECK(ctx);
-  return PYIID_OK;
+  const FqFinish fin{fsum, W->d_cfg_keys, W->d_key_spair, L->d_spair, d_ftab,
+                     d_na, G->d_inv_phi, m, n_bins, kbo, qbin, fq, nullptr};
+  return launch_fq_finish(ctx, fin, 0, 1, wide_sums(L, 0));
 }
 
 // One cluster per configuration, of as many CTAs (8, 2 or 1) as leave an SM

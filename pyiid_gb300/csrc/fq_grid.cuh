@@ -162,6 +162,7 @@ struct HistRows {
   float *rows;  // [n_ctas] rows of the CTAs, then those of the slots
   int *flag;    // [slots]
   int2 *cta;    // [n_ctas]
+  float *low;   // [warps], for sums in float pairs (fq_spread_kernel only)
   int n_ctas, row_words;
   __device__ __forceinline__ float *cta_row(int b) const {
     return rows + (size_t)b * row_words;
@@ -169,7 +170,19 @@ struct HistRows {
   __device__ __forceinline__ float *warp_row(int slot) const {
     return rows + ((size_t)n_ctas + slot) * row_words;
   }
+  // what the additions to a warp's row have rounded away so far
+  __device__ __forceinline__ float *low_row(int warp) const {
+    return low + (size_t)warp * row_words;
+  }
 };
+
+// x into the float pair (s, c)
+__device__ __forceinline__ void pair_add(float x, float &s, float &c) {
+  const float y = __fadd_rn(x, c);
+  const float t = __fadd_rn(s, y);
+  c = __fsub_rn(y, __fsub_rn(t, s));
+  s = t;
+}
 
 // End of a spreading CTA (all threads call it): whether this warp has to
 // write its last key itself.  Else, if s[0] >= 0, the CTA's warps 0 .. s[1]-1
@@ -224,6 +237,32 @@ __device__ __forceinline__ bool finish_rows(const HistRows &out, int wi,
 constexpr int kSpreadSlots = 8;
 constexpr int kSpreadCols = 2;
 constexpr PlanShape kFqPlan{4 * kSpreadSlots, 8};
+
+// the eight copies of word i
+__device__ __forceinline__ float sum_copies(const float4 *hist4, int i) {
+  const float4 v = hist4[2 * i], w = hist4[2 * i + 1];
+  return ((v.x + v.y) + (v.z + v.w)) + ((w.x + w.y) + (w.z + w.w));
+}
+
+// Moves a warp's cells to its row, the float pair (row, low) until `last`.
+// Not inlined: in line it costs the spreading loop 8 registers and 3 to 6 % of
+// its time.
+static __device__ __noinline__ void spill_cells(float4 *hist4, float *row,
+                                                float *low, int words,
+                                                bool add, bool last) {
+  __syncwarp();
+#pragma unroll 4
+  for (int i = threadIdx.x & 31; i < words; i += 32) {
+    float s = add ? row[i] : 0.f, c = add ? low[i] : 0.f;
+    pair_add(sum_copies(hist4, i), s, c);
+    row[i] = last ? s + c : s;
+    if (!last) low[i] = c;
+    hist4[2 * i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    hist4[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  __syncwarp();
+}
+
 __global__ void __launch_bounds__(32 * kSpreadWarps)
     fq_spread_kernel(const float *__restrict__ pos,
                      const int *__restrict__ perm,
@@ -234,6 +273,7 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
                      const float *__restrict__ taps, HistRows out) {
   extern __shared__ float4 smem4[];
   __shared__ int splan[32];
+  __shared__ bool sspill[kSpreadWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const SpreadPlan plan =
       spread_plan(ext, n_cfgs, gridDim.x, kFqPlan, total, splan);
@@ -264,20 +304,19 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
   }
   // tap p of cell j is cell j - 3 + p
   float *const base = hist + (8 + tp) * kSpreadSlots + slot;
-  auto word = [](const float4 *h, int i) {  // the eight copies of word i
-    const float4 v = h[2 * i], w = h[2 * i + 1];
-    return ((v.x + v.y) + (v.z + v.w)) + ((w.x + w.y) + (w.z + w.w));
-  };
-  auto flush = [&](int key) {
-    __syncwarp();
-    float *row = out.warp_row(wi + key);
-    for (int i = lane; i < words; i += 32) {
-      row[i] = word(hist4, i);
-      hist4[2 * i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      hist4[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    if (lane == 0) out.flag[wi + key] = 1;
-    __syncwarp();
+  // The cells go to the warp's row when it leaves a key, and after every
+  // spill_cols columns: a copy of a cell has then taken about 128 values,
+  // where one that grows without limit loses the window's tails.  The row is
+  // a float pair, so the sums do not depend on how many columns a warp gets.
+  const int spill_cols = 4 * words;
+  int since = 0;
+  bool spilled = false;
+  auto spill = [&](int key, bool last) {
+    spill_cells(hist4, out.warp_row(wi + key), out.low_row(wi), words, spilled,
+                last);
+    if (last && lane == 0) out.flag[wi + key] = 1;
+    since = 0;
+    spilled = !last;
   };
   int cur = -1;
   bool alone = false;
@@ -287,7 +326,7 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
     const int begin = seg_begin[sgi], end = min(seg_begin[sgi + 1], c1);
     if (sg.key != cur) {
       if (cur >= 0) {
-        flush(cur);
+        spill(cur, true);
         alone = true;
       }
       cur = sg.key;
@@ -395,19 +434,29 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
           __syncwarp();
         }
       }
+      since += nb;
+      if (since >= spill_cols) spill(cur, false);
     }
     c = end;
   }
+  if (lane == 0) sspill[warp] = spilled;
   if (finish_rows(out, wi, works ? cur : -1, alone, splan))
-    flush(cur);
+    spill(cur, true);
   else if (splan[0] >= 0)
     for (int i = threadIdx.x; i < words; i += blockDim.x) {
-      float s = 0.f;
-      for (int w = 0; w < splan[1]; ++w)
-        s += word(smem4 + w * (kSpreadStage / 16 + 2 * words) +
-                      kSpreadStage / 16,
-                  i);
-      out.cta_row(blockIdx.x)[i] = s;
+      float s = 0.f, c = 0.f;
+      for (int w = 0; w < splan[1]; ++w) {
+        if (sspill[w]) {
+          const int wj = blockIdx.x * plan.per_cta + w;
+          pair_add(out.warp_row(wj + splan[0])[i], s, c);
+          pair_add(out.low_row(wj)[i], s, c);
+        }
+        pair_add(sum_copies(smem4 + w * (kSpreadStage / 16 + 2 * words) +
+                                kSpreadStage / 16,
+                            i),
+                 s, c);
+      }
+      out.cta_row(blockIdx.x)[i] = s + c;
     }
 }
 
@@ -455,17 +504,11 @@ __device__ __forceinline__ void fq_grid_reduce(
   // the cells that meet in (G-_j, G+_j): j, its mirror images at 0 and M/2
   float hs = 0.f, hc = 0.f, ms = 0.f, mc = 0.f;
   const bool on = j <= quarter, near = j > quarter && j <= quarter + kNearTerms;
-  auto add = [](float x, float &s, float &c) {
-    const float y = __fadd_rn(x, c);
-    const float t = __fadd_rn(s, y);
-    c = __fsub_rn(y, __fsub_rn(t, s));
-    s = t;
-  };
   if (ty < ny && (on || near)) {
     const int j1 = half - j, last = plan.used + 4;
     auto take = [&](const float *r) {
       if (near) {
-        add(r[j - quarter - 1], hs, hc);
+        pair_add(r[j - quarter - 1], hs, hc);
         return;
       }
       r += kGridCell0;
@@ -473,8 +516,8 @@ __device__ __forceinline__ void fq_grid_reduce(
       float x = j <= last ? r[j] : 0.f, y = j1 <= last ? r[j1] : 0.f;
       if (j >= 1 && j <= 3) x -= r[-j];
       if (j >= 1 && half + j <= last) y -= r[half + j];
-      add(x, hs, hc);
-      add(y, ms, mc);
+      pair_add(x, hs, hc);
+      pair_add(y, ms, mc);
     };
     auto own = [&](int w, int key) {
       if (in.cta[w / plan.per_cta].y && in.flag[w + key])
@@ -509,9 +552,9 @@ __device__ __forceinline__ void fq_grid_reduce(
   if (ty != 0 || !(on || near)) return;
   for (int y = 1; y < ny; ++y) {
     const float *sh = sred + y * nx + tx;
-    add(sh[0], hs, hc);
+    pair_add(sh[0], hs, hc);
     hc += sh[st];
-    add(sh[2 * st], ms, mc);
+    pair_add(sh[2 * st], ms, mc);
     mc += sh[3 * st];
   }
   if (near) {
@@ -541,6 +584,19 @@ __global__ void fq_grid_reduce_kernel(HistRows in,
   fq_grid_reduce(in, key_cols[blockIdx.y], ext, n_cfgs, shape, total, m,
                  blockIdx.x, nx, ny,
                  out + (size_t)blockIdx.y * fq_sum_floats(m), sred, splan);
+}
+
+// Sum over a key's near pairs of sin(Q r)/r = Q sum_n (-1)^n (Q r)^2n /
+// (2n + 1)!; nr[n] = sum (Q_max r)^2n, near_unit = 1 / n_bins.
+__device__ __forceinline__ double near_sum(const float *nr, int k,
+                                           float near_unit, double dq) {
+  if (nr[0] == 0.f) return 0.0;
+  const float z = -(k * near_unit) * (k * near_unit);
+  const float v =
+      nr[0] + z * (nr[1] / 6.f +
+                   z * (nr[2] / 120.f +
+                        z * (nr[3] / 5040.f + z * (nr[4] / 362880.f))));
+  return (double)k * dq * (double)v;
 }
 
 // F(Q) of the configurations on the grid.  CTA = (32 bins, configuration),
@@ -636,10 +692,7 @@ __global__ void __launch_bounds__(32 * kFqDftWarps, 3)
           u = fmaf(cn[n], x.x, u);
           v = fmaf(sn[n], x.y, v);
         }
-        const float y = __fadd_rn(fmaf(sc, u, cc * v), c);
-        const float t = __fadd_rn(s, y);
-        c = __fsub_rn(y, __fsub_rn(t, s));
-        s = t;
+        pair_add(fmaf(sc, u, cc * v), s, c);
       }
       red[q][0][warp][lane] = s;
       red[q][1][warp][lane] = c;
@@ -653,20 +706,10 @@ __global__ void __launch_bounds__(32 * kFqDftWarps, 3)
         c = __fsub_rn(y, __fsub_rn(t, s)) + red[warp][1][w][lane];
         s = t;
       }
-      double d = ((double)s + (double)c) * inv_phi[k];
-      const float *nr =
-          hq + (size_t)warp * fq_sum_floats(m) + 2 * (quarter + 1);
-      if (nr[0] != 0.f) {
-        // sum over near pairs of sin(Q r)/r = Q sum_n (-1)^n (Q r)^2n /
-        // (2n + 1)!; nr[n] = sum (Q_max r)^2n
-        const float z = -(k * near_unit) * (k * near_unit);
-        const float v =
-            nr[0] +
-            z * (nr[1] / 6.f +
-                 z * (nr[2] / 120.f +
-                      z * (nr[3] / 5040.f + z * (nr[4] / 362880.f))));
-        d += (double)k * dq * (double)v;
-      }
+      const double d =
+          ((double)s + (double)c) * inv_phi[k] +
+          near_sum(hq + (size_t)warp * fq_sum_floats(m) + 2 * (quarter + 1), k,
+                   near_unit, dq);
       const int2 ss = spair_species[key_spair[ck.y + q0 + warp]];
       terms[warp][lane] = (double)ftab[ss.x * n_bins + k] *
                           (double)ftab[ss.y * n_bins + k] * d;
@@ -674,6 +717,95 @@ __global__ void __launch_bounds__(32 * kFqDftWarps, 3)
     __syncthreads();
     if (warp == 0)
       for (int q = 0; q < nq; ++q) sum += terms[q][lane];
+  }
+  const int kk = blockIdx.x * 32 + lane;
+  if (warp != 0 || kk >= n_bins) return;
+  const size_t o = (size_t)ck.x * n_bins + kk;
+  const bool on = kk >= kb_out;
+  if (fq) fq[o] = on ? fq_value(sum, na[o]) : 0.f;
+  if (fq_raw) fq_raw[o] = on ? sum : 0.0;
+}
+
+// The same transform in FP64 for configurations of many pairs.  The rotations
+// by n cells are common to all blocks of a bin, so what FP32 rounds off them
+// multiplies every 33rd cell's sum, which sees the small-angle peak of F (its
+// height grows with the atoms) at the bins near multiples of M / 33.
+// One key at a time; warps share the blocks, each centre one rotation by
+// kFqDftWarps blocks from the one before.  FP64 bound.
+__host__ __device__ constexpr int fq_wide_smem(int m) {
+  return fq_dft_blocks(m) * (kFqDftReach + 1) * 4 * (int)sizeof(double);
+}
+__global__ void __launch_bounds__(32 * kFqDftWarps)
+    fq_grid_finish_wide_kernel(const float *__restrict__ hsum,
+                               const int4 *__restrict__ cfg_keys,
+                               const int *__restrict__ key_spair,
+                               const int2 *__restrict__ spair_species,
+                               const float *__restrict__ ftab,
+                               const double *__restrict__ na,
+                               const double *__restrict__ inv_phi, int m,
+                               int n_bins, int kb_out, double dq,
+                               float near_unit, float *__restrict__ fq,
+                               double *__restrict__ fq_raw) {
+  constexpr int R = kFqDftReach, B = 2 * R + 1;
+  extern __shared__ double2 sh2[];  // [block][n][even, odd bins]
+  __shared__ double red[kFqDftWarps][32];
+  const int4 ck = cfg_keys[blockIdx.y];  // configuration, first key, keys
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int k = min((int)(blockIdx.x * 32 + lane), n_bins - 1);
+  const int quarter = m / 4, blocks = fq_dft_blocks(m);
+  auto turn = [&](int n, double &s, double &c) {  // of 2 pi k n / m
+    sincospi(2.0 * (double)((unsigned)n * (unsigned)k % (unsigned)m) /
+                 (double)m,
+             &s, &c);
+  };
+  double s1, c1, sw, cw, s0, c0;
+  turn(1, s1, c1);
+  turn(B * kFqDftWarps % m, sw, cw);
+  turn((1 + warp * B + R) % m, s0, c0);
+  double sum = 0.0;
+  for (int q = 0; q < ck.z; ++q) {
+    const float *h = hsum + (size_t)(ck.y + q) * fq_sum_floats(m);
+    __syncthreads();
+    for (int i = threadIdx.x; i < blocks * (R + 1); i += blockDim.x) {
+      const int b = i / (R + 1), n = i - b * (R + 1);
+      const int jp = 1 + b * B + R + n, jm = 1 + b * B + R - n;
+      float2 p = make_float2(0.f, 0.f), o = p;
+      if (jp <= quarter) p = *reinterpret_cast<const float2 *>(h + 2 * jp);
+      if (n > 0 && jm <= quarter)
+        o = *reinterpret_cast<const float2 *>(h + 2 * jm);
+      sh2[2 * i] = make_double2((double)p.x + o.x, (double)p.x - o.x);
+      sh2[2 * i + 1] = make_double2((double)p.y + o.y, (double)p.y - o.y);
+    }
+    __syncthreads();
+    const double2 *hk = sh2 + (k & 1);
+    double s = 0.0, sc = s0, cc = c0;
+    for (int b = warp; b < blocks; b += kFqDftWarps) {
+      double u = 0.0, v = 0.0, sn = 0.0, cn = 1.0;
+#pragma unroll
+      for (int n = 0; n <= R; ++n) {
+        const double2 x = hk[2 * (b * (R + 1) + n)];
+        u = fma(cn, x.x, u);
+        v = fma(sn, x.y, v);
+        const double t = fma(sn, c1, cn * s1);
+        cn = fma(cn, c1, -sn * s1);
+        sn = t;
+      }
+      s += fma(sc, u, cc * v);
+      const double t = fma(sc, cw, cc * sw);
+      cc = fma(cc, cw, -sc * sw);
+      sc = t;
+    }
+    red[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0) {
+      s = 0.0;
+      for (int w = 0; w < kFqDftWarps; ++w) s += red[w][lane];
+      const int2 ss = spair_species[key_spair[ck.y + q]];
+      sum += (double)ftab[ss.x * n_bins + k] *
+             (double)ftab[ss.y * n_bins + k] *
+             (s * inv_phi[k] +
+              near_sum(h + 2 * (quarter + 1), k, near_unit, dq));
+    }
   }
   const int kk = blockIdx.x * 32 + lane;
   if (warp != 0 || kk >= n_bins) return;

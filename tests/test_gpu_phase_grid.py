@@ -342,3 +342,44 @@ def test_transform_and_potential_of_batches(D, n_configs, exp):
         v = 1.0 if a <= 0 else np.sqrt((wn * (gobs - a * want[i]) ** 2).sum() /
                                        (wn * gobs ** 2).sum())
         assert abs(got[i, 0] - v) <= 1e-12 * abs(v)
+
+
+def sampled_fq(pos, sp, tab, qb, bins):
+    """F on `bins` from FP64 pair sums."""
+    from oracle import debye_c as C
+    bins = np.asarray(bins, np.int32)
+    return 2 * C.pair_sums(pos, sp, tab, qb, bins) / \
+        O.normalization(tab[sp])[bins]
+
+
+# A warp's share of a key's columns grows with the batch: thousands of values
+# per copy of a cell here.  Their error must not: the bound
+# is twice what the direct kernels, which add short FP32 sums in FP64, leave
+# for one such particle (2e-7); sums held in FP32 alone leave 1.2e-6.
+def test_sums_of_a_large_batch_keep_their_precision(D):
+    n, copies, qb, nb = 20000, 16, 0.02, 1500
+    pos, nums = cluster(n, 3)
+    sp, tab = tables(nums, qb, nb)
+    f = D.batch_fq(np.tile(pos, (copies, 1)), np.tile(sp, copies),
+                   np.arange(copies + 1) * n, tab, qb).cpu().numpy()
+    bins = np.arange(41, nb, 97)
+    want = sampled_fq(pos, sp, tab, qb, bins)
+    for row in f:
+        assert rel(row[bins], want) <= 4e-7, rel(row[bins], want)
+
+
+# The transform of many pairs at the bins where FP32 rotations would see the
+# small-angle peak of F (multiples of M / 33 of M = 5 n_bins cells).  Bound:
+# the rounding of the sums handed to it (4e-8), the window (2e-8) and the
+# distances (5e-8), added and rounded up.
+@pytest.mark.parametrize('grad', [False, True])
+def test_transform_of_a_large_particle(D, grad):
+    n, qb, nb = 30000, 0.02, 1500
+    pos, nums = cluster(n, 4)
+    sp, tab = tables(nums, qb, nb)
+    m = 6144 if grad else 5 * nb
+    bins = np.round(m / 33 * np.arange(1, 6)).astype(int)
+    f = D.fq_grad(pos, sp, tab, qb)[0] if grad else D.fq(pos, sp, tab, qb)
+    want = sampled_fq(pos, sp, tab, qb, bins)
+    assert rel(f.cpu().numpy()[bins], want) <= 1.5e-7, \
+        rel(f.cpu().numpy()[bins], want)
