@@ -263,6 +263,74 @@ static __device__ __noinline__ void spill_cells(float4 *hist4, float *row,
   __syncwarp();
 }
 
+// The pairs of a column that the fast distance does not cover (on: the
+// lane's is one).  Beyond 128 A they can be most of a call's, so they go
+// together as the others do; only those nearer than near_r and those without
+// a distance go one at a time.  Not inlined: in line, or as a branch ahead of
+// the others' spreading, it costs every call 6 to 24 %.
+// 4,000 atoms in two clusters 400 A apart, 500 bins: 426 us (one at a time
+// 5,830; fq_pair3_kernel 710).
+static __device__ __noinline__ void spread_rest(
+    float ahx, float ahy, float ahz, float alx, float aly, float alz,
+    float bhx, float bhy, float bhz, float blx, float bly, float blz, bool on,
+    float ghi, float glo, float gm, float ginv, float near_r, float near_scale,
+    const float *__restrict__ taps, float *hist, int used) {
+  if (!__any_sync(0xffffffffu, on)) return;
+  const GridScale gs{ghi, glo, gm, ginv};
+  const int lane = threadIdx.x & 31, slot = lane >> 2, tp = lane & 3;
+  PairDist p{};
+  bool wide = on;
+  if (on) {
+    p = pair_dist_general(ahx + alx, ahy + aly, ahz + alz, bhx + blx,
+                          bhy + bly, bhz + blz);
+    wide = p.r >= near_r && p.r < 3e38f;
+  }
+  float uh, ul;
+  grid_pos(gs, p.r, p.rl, uh, ul);
+  float w = uh < 0.f ? -p.inv_r : p.inv_r;
+  ul = uh < 0.f ? -ul : ul;
+  uh = fabsf(uh);
+  const float fj = floorf(uh);
+  // (NaN: the middle of a cell)
+  const float t = fminf(fmaxf((uh - fj) + (ul - 0.5f), -0.5f), 0.5f);
+  const int j = min(max((int)fj, 0), used);
+  if (!wide) w = 0.f;
+  for (int src = slot; src < 32; src += 8) {
+    float *h = hist + (8 + tp + __shfl_sync(0xffffffffu, j, src)) *
+                          kSpreadSlots + slot;
+    const float ts = __shfl_sync(0xffffffffu, t, src);
+    const float ws = __shfl_sync(0xffffffffu, w, src);
+    float f0 = taps[tp * kTapCoef + 7], f1 = taps[(tp + 4) * kTapCoef + 7];
+#pragma unroll
+    for (int n = 6; n >= 0; --n) {
+      f0 = fmaf(f0, ts, taps[tp * kTapCoef + n]);
+      f1 = fmaf(f1, ts, taps[(tp + 4) * kTapCoef + n]);
+    }
+    const float x = h[0], y = h[4 * kSpreadSlots];
+    h[0] = x + ws * f0;
+    h[4 * kSpreadSlots] = y + ws * f1;
+    __syncwarp();
+  }
+  if (!__any_sync(0xffffffffu, on && !wide)) return;
+  for (int l = 0; l < 32; ++l) {
+    if (lane == l && on && !wide) {
+      if (p.r > 0.f && p.r < near_r) {
+        // far below the resolution of Q (Q_max r < 0.6): the power sums of
+        // r^2 give sin(Q r)/r, which the window would only give to 1e-7 / r
+        const float z = (p.r * near_scale) * (p.r * near_scale);
+        float x = 1.f;
+        for (int n = 0; n < kNearTerms; ++n, x *= z)
+          hist[n * kSpreadSlots] += x;
+      } else {
+        // r = 0, infinite or NaN: NaN for every bin, as sin(Q r)/r is
+        for (int n = 0; n < kTaps; ++n)
+          hist[(8 + j + n) * kSpreadSlots] = __int_as_float(0x7fffffff);
+      }
+    }
+    __syncwarp();
+  }
+}
+
 __global__ void __launch_bounds__(32 * kSpreadWarps)
     fq_spread_kernel(const float *__restrict__ pos,
                      const int *__restrict__ perm,
@@ -396,43 +464,12 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
 #pragma unroll
         for (int q = 0; q < kSpreadCols; ++q) left |= on[q] && !ok[q];
         if (!__any_sync(0xffffffffu, left)) continue;
-        // pairs that the fast distance does not cover, one at a time
-        for (int l = 0; l < 32; ++l) {
-          for (int q = 0; q < kSpreadCols; ++q) {
-            if (lane != l || !on[q] || ok[q]) continue;
-            const PairDist g = pair_dist_general(
-                a.hx + a.lx, a.hy + a.ly, a.hz + a.lz, b[q].hx + b[q].lx,
-                b[q].hy + b[q].ly, b[q].hz + b[q].lz);
-            if (g.r > 0.f && g.r < near_r) {
-              // far below the resolution of Q (Q_max r < 0.6): the power
-              // sums of r^2 give sin(Q r)/r, which the window would only
-              // give to 1e-7 / r
-              const float z = (g.r * near_scale) * (g.r * near_scale);
-              float x = 1.f;
-              for (int n = 0; n < kNearTerms; ++n, x *= z)
-                hist[n * kSpreadSlots] += x;
-            } else {
-              float uh, ul;
-              grid_pos(gs, g.r, g.rl, uh, ul);
-              float wg = uh < 0.f ? -g.inv_r : g.inv_r;
-              ul = uh < 0.f ? -ul : ul;
-              uh = fabsf(uh);
-              // r = 0, infinite or NaN: NaN for every bin, as sin(Q r)/r is
-              if (!(g.r > 0.f && g.r < 3e38f)) wg = __int_as_float(0x7fffffff);
-              const float fg = floorf(uh);
-              const float tg =
-                  fminf(fmaxf((uh - fg) + (ul - 0.5f), -0.5f), 0.5f);
-              const int j = min(max((int)fg, 0), plan.used);
-              for (int n = 0; n < kTaps; ++n) {
-                float f = taps[n * kTapCoef + 7];
-                for (int m = 6; m >= 0; --m)
-                  f = fmaf(f, tg, taps[n * kTapCoef + m]);
-                hist[(8 + j + n) * kSpreadSlots] += wg * f;
-              }
-            }
-          }
-          __syncwarp();
-        }
+#pragma unroll
+        for (int q = 0; q < kSpreadCols; ++q)
+          spread_rest(a.hx, a.hy, a.hz, a.lx, a.ly, a.lz, b[q].hx, b[q].hy,
+                      b[q].hz, b[q].lx, b[q].ly, b[q].lz, on[q] && !ok[q],
+                      gs.hi, gs.lo, gs.m, gs.inv_m, near_r, near_scale, taps,
+                      hist, plan.used);
       }
       since += nb;
       if (since >= spill_cols) spill(cur, false);

@@ -91,6 +91,145 @@ __device__ __forceinline__ void sts(int addr, float x) {
   asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(x) : "memory");
 }
 
+// A staged column: weights [4][32 + 4] (x, y, z, F; the four rows on different
+// banks), shared-memory words of the cells [32], positions [32].
+__device__ __forceinline__ void stage_column(float *sw, int hbase, int cell,
+                                             float t, float x, float y, float z,
+                                             float f) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  sw[lane] = x;
+  sw[36 + lane] = y;
+  sw[72 + lane] = z;
+  sw[108 + lane] = f;
+  reinterpret_cast<int *>(sw)[144 + lane] = hbase + cell * 16;
+  sw[176 + lane] = t;
+  __syncwarp();
+}
+
+// Bit of each lane whose group of four has cells that overlap.
+__device__ __forceinline__ unsigned tied_groups(int cell) {
+  bool near4 = false;
+#pragma unroll
+  for (int x = 1; x < 4; ++x)
+    near4 |= abs(__shfl_xor_sync(0xffffffffu, cell, x) - cell) < kTaps;
+  return __ballot_sync(0xffffffffu, near4);
+}
+
+// Adds a staged column to the warp's cells, lane = (tap, component).
+__device__ __forceinline__ void spread_column(const float *sw, unsigned tied,
+                                              const float2 (&cf)[kTapCoef]) {
+  const int lane = threadIdx.x & 31;
+  const int4 *so4 = reinterpret_cast<const int4 *>(sw + 144);
+  const float4 *st4 = reinterpret_cast<const float4 *>(sw + 176);
+  const float4 *sw4 = reinterpret_cast<const float4 *>(sw) + 9 * (lane & 3);
+  int4 no = so4[0];
+  float4 nt = st4[0], nv = sw4[0];
+#pragma unroll 2
+  for (int g = 0; g < 8; ++g) {
+    const int4 o = no;
+    const float4 t4 = nt, v = nv;
+    // (the last one reads what lies behind, inside the warp's stage)
+    no = so4[g + 1];
+    nt = st4[g + 1];
+    nv = sw4[g + 1];
+    const float2 t01 = make_float2(t4.x, t4.y);
+    const float2 t23 = make_float2(t4.z, t4.w);
+    float2 f01 = cf[7], f23 = cf[7];
+#pragma unroll
+    for (int m = 6; m >= 0; --m) {
+      f01 = __ffma2_rn(f01, t01, cf[m]);
+      f23 = __ffma2_rn(f23, t23, cf[m]);
+    }
+    const int h0 = o.x + 4 * lane, h1 = o.y + 4 * lane;
+    const int h2 = o.z + 4 * lane, h3 = o.w + 4 * lane;
+    if ((tied >> (4 * g)) & 0xfu) {
+      sts(h0, fmaf(v.x, f01.x, lds(h0)));
+      __syncwarp();
+      sts(h1, fmaf(v.y, f01.y, lds(h1)));
+      __syncwarp();
+      sts(h2, fmaf(v.z, f23.x, lds(h2)));
+      __syncwarp();
+      sts(h3, fmaf(v.w, f23.y, lds(h3)));
+    } else {
+      const float x0 = lds(h0), x1 = lds(h1), x2 = lds(h2), x3 = lds(h3);
+      sts(h0, fmaf(v.x, f01.x, x0));
+      sts(h1, fmaf(v.y, f01.y, x1));
+      sts(h2, fmaf(v.z, f23.x, x2));
+      sts(h3, fmaf(v.w, f23.y, x3));
+    }
+    __syncwarp();
+  }
+}
+
+// The pairs of a column that the fast distance does not cover, as spread_rest
+// of fq_grid.cuh; returns whether the lane's pair is a period or more away.
+// The two clusters named there, F and dF/dx: 1,807 us (one at a time 8,076,
+// fqgrad2_kernel 3,352).
+// stage: the warp's, as grad_spread_kernel lays it out.
+template <bool WITH_F>
+static __device__ __noinline__ bool grad_spread_rest(
+    float ahx, float ahy, float ahz, float alx, float aly, float alz,
+    float bhx, float bhy, float bhz, float blx, float bly, float blz, bool on,
+    int sweep, float ghi, float glo, float gm, float ginv, float near_r,
+    float near_scale, const float *__restrict__ taps, float4 *stage,
+    float4 *hist4, int used) {
+  const GridScale gs{ghi, glo, gm, ginv};
+  const int lane = threadIdx.x & 31;
+  PairDist p{};
+  bool use = on;
+  if (on) {
+    p = pair_dist_general(ahx + alx, ahy + aly, ahz + alz, bhx + blx,
+                          bhy + bly, bhz + blz);
+    use = p.r >= near_r && p.r < 3e38f;
+  }
+  float uh, ul;
+  const float n = grid_pos(gs, p.r, p.rl, uh, ul);
+  const float s = uh < 0.f ? -1.0f : 1.0f;
+  const float ua = fabsf(uh), fj = floorf(ua);
+  // (NaN: the middle of a cell)
+  const float t = fminf(fmaxf((ua - fj) + (s * ul - 0.5f), -0.5f), 0.5f);
+  const int j = min(max((int)fj, 0), used);
+  const float w =
+      (p.inv_r * p.inv_r) * (sweep ? gs.m * n * p.inv_r : s * p.inv_r);
+  float2 cf[kTapCoef];
+#pragma unroll
+  for (int i = 0; i < kTapCoef; ++i)
+    cf[i] = f2(taps[(lane >> 2) * kTapCoef + i]);
+  float *const sw = reinterpret_cast<float *>(stage);
+  stage_column(sw, (int)__cvta_generic_to_shared(hist4 + 8), j, t,
+               use ? w * p.dx : 0.f, use ? w * p.dy : 0.f,
+               use ? w * p.dz : 0.f,
+               use && WITH_F && !sweep ? 0.5f * s * p.inv_r : 0.f);
+  spread_column(sw, tied_groups(j), cf);
+  for (unsigned rest = __ballot_sync(0xffffffffu, on && !use); rest;
+       rest &= rest - 1) {
+    if (lane == __ffs(rest) - 1) {
+      if (p.r > 0.f && p.r < near_r) {
+        // far below the resolution of Q: power sums of r^2
+        const float z = (p.r * near_scale) * (p.r * near_scale);
+        float x = sweep ? 0.f : 1.f;
+        for (int m = 0; m < kNearTerms; ++m, x *= z) {
+          hist4[m].x += x * p.dx;
+          hist4[m].y += x * p.dy;
+          hist4[m].z += x * p.dz;
+          if (WITH_F) hist4[m].w += 0.5f * x;
+        }
+      } else {
+        // r = 0, infinite or NaN: NaN for every bin
+        const float bad = __int_as_float(0x7fffffff);
+        for (int m = 0; m < kTaps; ++m) {
+          float4 &x = hist4[8 + j + m];
+          x.x = x.y = x.z = bad;
+          if (WITH_F) x.w = bad;
+        }
+      }
+    }
+    __syncwarp();
+  }
+  return use && n != 0.f;
+}
+
 // One CTA per SM, each warp with a private histogram; the columns of all
 // units, in order, are dealt out evenly to the warps (spread_plan), so a unit
 // may be cut between warps: warp i writes its part of unit u at row i + u,
@@ -134,13 +273,8 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
   const int c1 = (int)((long long)(wi + 1) * total / plan.n);
   const bool works = warp < plan.per_cta && wi < plan.n;
   const int words = grid_words(plan.used);
-  // staged column: weights [4][32 + 4] (the four rows on different banks),
-  // words of the cells [32], positions [32]
   float4 *const stage = smem4 + warp * (kSpreadStage / 16 + words);
   float *const sw = reinterpret_cast<float *>(stage);
-  int *const so = reinterpret_cast<int *>(sw + 144);
-  float *const st = sw + 176;
-  const float4 *const sw4 = stage + 9 * (lane & 3);
   float4 *const hist4 = stage + kSpreadStage / 16;  // [word]
   const int hbase = (int)__cvta_generic_to_shared(hist4 + 8);
   float2 cf[kTapCoef];
@@ -221,103 +355,14 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
         const float ua = fabsf(uh), fj = floorf(ua);
         const float t = ok ? (ua - fj) + (sg * ul - 0.5f) : 0.f;
         const int cell = ok ? min((int)fj, plan.used) : 0;
-        // groups of four lanes whose cells overlap
-        bool near4 = false;
-#pragma unroll
-        for (int x = 1; x < 4; ++x)
-          near4 |= abs(__shfl_xor_sync(0xffffffffu, cell, x) - cell) < kTaps;
-        const unsigned tied = __ballot_sync(0xffffffffu, near4);
-        __syncwarp();
-        sw[lane] = ok ? w * p.dx : 0.f;
-        sw[36 + lane] = ok ? w * p.dy : 0.f;
-        sw[72 + lane] = ok ? w * p.dz : 0.f;
-        sw[108 + lane] = ok ? wf : 0.f;
-        so[lane] = hbase + cell * 16;
-        st[lane] = t;
-        __syncwarp();
-        int4 no = reinterpret_cast<const int4 *>(so)[0];
-        float4 nt = reinterpret_cast<const float4 *>(st)[0], nv = sw4[0];
-#pragma unroll 2
-        for (int g = 0; g < 8; ++g) {
-          const int4 o = no;
-          const float4 t4 = nt, v = nv;
-          // (the last one reads what lies behind, inside the warp's stage)
-          no = reinterpret_cast<const int4 *>(so)[g + 1];
-          nt = reinterpret_cast<const float4 *>(st)[g + 1];
-          nv = sw4[g + 1];
-          const float2 t01 = make_float2(t4.x, t4.y);
-          const float2 t23 = make_float2(t4.z, t4.w);
-          float2 f01 = cf[7], f23 = cf[7];
-#pragma unroll
-          for (int m = 6; m >= 0; --m) {
-            f01 = __ffma2_rn(f01, t01, cf[m]);
-            f23 = __ffma2_rn(f23, t23, cf[m]);
-          }
-          const int h0 = o.x + 4 * lane, h1 = o.y + 4 * lane;
-          const int h2 = o.z + 4 * lane, h3 = o.w + 4 * lane;
-          if ((tied >> (4 * g)) & 0xfu) {
-            sts(h0, fmaf(v.x, f01.x, lds(h0)));
-            __syncwarp();
-            sts(h1, fmaf(v.y, f01.y, lds(h1)));
-            __syncwarp();
-            sts(h2, fmaf(v.z, f23.x, lds(h2)));
-            __syncwarp();
-            sts(h3, fmaf(v.w, f23.y, lds(h3)));
-          } else {
-            const float x0 = lds(h0), x1 = lds(h1), x2 = lds(h2), x3 = lds(h3);
-            sts(h0, fmaf(v.x, f01.x, x0));
-            sts(h1, fmaf(v.y, f01.y, x1));
-            sts(h2, fmaf(v.z, f23.x, x2));
-            sts(h3, fmaf(v.w, f23.y, x3));
-          }
-          __syncwarp();
-        }
+        stage_column(sw, hbase, cell, t, ok ? w * p.dx : 0.f,
+                     ok ? w * p.dy : 0.f, ok ? w * p.dz : 0.f, ok ? wf : 0.f);
+        spread_column(sw, tied_groups(cell), cf);
         if (!__any_sync(0xffffffffu, on && !ok)) continue;
-        // pairs that the fast distance does not cover, one at a time
-        for (int l = 0; l < 32; ++l) {
-          if (lane == l && on && !ok) {
-            const PairDist d = pair_dist_general(
-                a.hx + a.lx, a.hy + a.ly, a.hz + a.lz, b.hx + b.lx,
-                b.hy + b.ly, b.hz + b.lz);
-            if (d.r > 0.f && d.r < near_r) {
-              // far below the resolution of Q: power sums of r^2
-              const float z = (d.r * near_scale) * (d.r * near_scale);
-              float x = sweep ? 0.f : 1.f;
-              for (int m = 0; m < kNearTerms; ++m, x *= z) {
-                hist4[m].x += x * d.dx;
-                hist4[m].y += x * d.dy;
-                hist4[m].z += x * d.dz;
-                if (WITH_F) hist4[m].w += 0.5f * x;
-              }
-            } else {
-              float gh, gl;
-              const float gn = grid_pos(gs, d.r, d.rl, gh, gl);
-              wide |= gn != 0.f;
-              const float s = gh < 0.f ? -1.0f : 1.0f;
-              float k = (d.inv_r * d.inv_r) *
-                        (sweep ? gs.m * gn * d.inv_r : s * d.inv_r);
-              float kf = WITH_F && !sweep ? 0.5f * s * d.inv_r : 0.f;
-              // r = 0, infinite or NaN: NaN for every bin
-              if (!(d.r > 0.f && d.r < 3e38f))
-                k = kf = __int_as_float(0x7fffffff);
-              const float ga = fabsf(gh), fg = floorf(ga);
-              const float tg =
-                  fminf(fmaxf((ga - fg) + (s * gl - 0.5f), -0.5f), 0.5f);
-              const int j = min(max((int)fg, 0), plan.used);
-              for (int m = 0; m < kTaps; ++m) {
-                float f = taps[m * kTapCoef + 7];
-                for (int o = 6; o >= 0; --o)
-                  f = fmaf(f, tg, taps[m * kTapCoef + o]);
-                float4 &x = hist4[8 + j + m];
-                x.x = fmaf(k * d.dx, f, x.x);
-                x.y = fmaf(k * d.dy, f, x.y);
-                x.z = fmaf(k * d.dz, f, x.z);
-                if (WITH_F) x.w = fmaf(kf, f, x.w);
-              }
-            }
-          }
-          __syncwarp();
-        }
+        wide |= grad_spread_rest<WITH_F>(
+            a.hx, a.hy, a.hz, a.lx, a.ly, a.lz, b.hx, b.hy, b.hz, b.lx, b.ly,
+            b.lz, on && !ok, sweep, gs.hi, gs.lo, gs.m, gs.inv_m, near_r,
+            near_scale, taps, stage, hist4, plan.used);
       }
       __syncwarp();
       float *out = (sweep ? rows2 : rows) + row;

@@ -103,12 +103,16 @@ __device__ __forceinline__ bool pair_dist_fast(const SplitAtom &a,
   return s > 0.01f && n < 16384.0f;
 }
 
+__device__ __forceinline__ PairDist pair_dist_general(const SplitAtom &a,
+                                                      const SplitAtom &b) {
+  return pair_dist_general(a.hx + a.lx, a.hy + a.ly, a.hz + a.lz, b.hx + b.lx,
+                           b.hy + b.ly, b.hz + b.lz);
+}
+
 __device__ __forceinline__ PairDist pair_dist(const SplitAtom &a,
                                               const SplitAtom &b) {
   PairDist p;
-  if (!pair_dist_fast(a, b, p))
-    p = pair_dist_general(a.hx + a.lx, a.hy + a.ly, a.hz + a.lz, b.hx + b.lx,
-                          b.hy + b.ly, b.hz + b.lz);
+  if (!pair_dist_fast(a, b, p)) p = pair_dist_general(a, b);
   return p;
 }
 

@@ -383,3 +383,63 @@ def test_transform_of_a_large_particle(D, grad):
     want = sampled_fq(pos, sp, tab, qb, bins)
     assert rel(f.cpu().numpy()[bins], want) <= 1.5e-7, \
         rel(f.cpu().numpy()[bins], want)
+
+
+# Most pairs beyond 128 A, where the split coordinates no longer give the
+# distance: a rod, and two clusters far apart.
+@pytest.mark.parametrize('shape', ['rod', 'halves'])
+def test_far_pairs_match_oracle(D, shape):
+    from oracle import debye_c as C
+    n, qb, nb, kb = 700, 0.05, 500, 2
+    if shape == 'rod':
+        pos = np.zeros((n, 3), np.float32)
+        pos[:, 0] = 2.9 * np.arange(n)
+        pos += np.random.default_rng(6).normal(0, 0.05, pos.shape)
+        pos = pos.astype(np.float32)
+        nums = np.full(n, 79)
+    else:
+        pos, nums = cluster(n, 8, 2)
+        pos[::2] += np.float32([300.0, -250.0, 100.0])
+    sp, tab = tables(nums, qb, nb)
+    bins = np.arange(kb, nb, 11)
+    want = sampled_fq(pos, sp, tab, qb, bins)
+    f = D.fq(pos, sp, tab, qb, kb).cpu().numpy()
+    f2, g = (t.cpu().numpy() for t in D.fq_grad(pos, sp, tab, qb, kb))
+    assert rel(f[bins], want) <= TOL_F and rel(f2[bins], want) <= TOL_F
+    rows = np.array([0, 1, n // 2, n - 1], np.int32)
+    want_g = -C.grad_rows(pos, sp, tab, qb, rows) / O.normalization(tab[sp])
+    for i, a in enumerate(rows):
+        assert rel(g[a, :, kb:], want_g[i, :, kb:]) <= TOL_G
+
+
+# ... which are no rare case to be done one at a time: the same two clusters
+# 400 A apart instead of 100 take about one distance in full more per pair,
+# not twice as long.
+def test_far_pairs_cost_what_near_ones_cost(D):
+    import torch
+    n, qb, nb = 4000, 0.05, 500
+    pos, nums = cluster(n, 12)
+    sp, tab = tables(nums, qb, nb)
+
+    def ms(fn):
+        fn()
+        t = []
+        for _ in range(9):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            for _ in range(4):
+                fn()
+            b.record()
+            b.synchronize()
+            t.append(a.elapsed_time(b))
+        return np.median(t)
+
+    def times(apart):
+        p = pos.copy()
+        p[::2, 0] += np.float32(apart)
+        p = torch.as_tensor(p, device='cuda')
+        return (ms(lambda: D.fq(p, sp, tab, qb)),
+                ms(lambda: D.fq_grad(p, sp, tab, qb)))
+
+    near, far = times(100.0), times(400.0)
+    assert far[0] <= 2 * near[0] and far[1] <= 2 * near[1], (near, far)
