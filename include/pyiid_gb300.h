@@ -537,6 +537,12 @@ int pyiid_variant_info(int kernel, int variant, int *params, int n_params);
 int pyiid_set_variant(pyiid_ctx *ctx, int kernel, int variant);
 int pyiid_get_variant(const pyiid_ctx *ctx, int kernel);
 
+/* Number of launches so far of the kernels that `kernel` selects the shape of
+ * (-1: no such kernel).  A call that leaves it as it was took another path, on
+ * which the variants have no effect: F(Q), its gradient and the gradient of
+ * the potential go to kernels on a grid of phases where these are faster. */
+int64_t pyiid_variant_launches(const pyiid_ctx *ctx, int kernel);
+
 #ifdef __cplusplus
 }
 #endif

@@ -95,6 +95,7 @@ _SIGNATURES = {
     'pyiid_variant_info': (_c_int, [_c_int, _c_int, _i32p, _c_int]),
     'pyiid_set_variant': (_c_int, [_vp, _c_int, _c_int]),
     'pyiid_get_variant': (_c_int, [_vp, _c_int]),
+    'pyiid_variant_launches': (ctypes.c_int64, [_vp, _c_int]),
 }
 
 KERNELS = {'fq': 0, 'grad_fq': 1, 'adjoint': 2, 'fq_grad': 3, 'mlp': 4}
@@ -198,6 +199,11 @@ class Context:
 
     def get_variant(self, kernel):
         return int(self._lib.pyiid_get_variant(self.handle, KERNELS[kernel]))
+
+    def variant_launches(self, kernel):
+        """Launches so far of the kernels whose shape a variant selects."""
+        return int(self._lib.pyiid_variant_launches(self.handle,
+                                                    KERNELS[kernel]))
 
     @property
     def launches(self):

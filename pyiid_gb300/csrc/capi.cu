@@ -324,6 +324,7 @@ struct pyiid_ctx {
   cudaStream_t stream = nullptr;
   std::string err;
   int64_t launches = 0;
+  int64_t variant_launches[5] = {};  // by PYIID_KERNEL_*
   std::unordered_map<std::string, DevBuf> bufs;
   std::vector<std::unique_ptr<Layout>> layouts;  // small LRU (front = newest)
   std::vector<std::unique_ptr<TMatrix>> tmats;
@@ -382,6 +383,13 @@ int fail(pyiid_ctx *ctx, int code, const char *fmt, ...) {
     if (e_ != cudaSuccess)                                                    \
       return fail(ctx, PYIID_ERR_CUDA, "kernel launch failed: %s (%s:%d)",    \
                   cudaGetErrorString(e_), __FILE__, __LINE__);                \
+  } while (0)
+
+// after a launch of a kernel with variants
+#define VARIANT_LAUNCH_CHECK(ctx, kernel)  \
+  do {                                     \
+    LAUNCH_CHECK(ctx);                     \
+    ++(ctx)->variant_launches[kernel];     \
   } while (0)
 
 #define TRY(expr)              \
@@ -1370,7 +1378,7 @@ int run_fq(pyiid_ctx *ctx, Layout *L, const float *positions,
           positions, L->d_perm, L->d_tiles, L->d_items, order, dq_hi, dq_lo,
           kb0, n_chunks, n_groups, n_bins, partial);
     }
-    LAUNCH_CHECK(ctx);
+    VARIANT_LAUNCH_CHECK(ctx, PYIID_KERNEL_FQ);
   }
   dim3 g2((n_bins + 127) / 128, L->n_configs);
   const int kb_out = (n_items > 0) ? std::min(k_begin, n_bins) : n_bins;
@@ -1738,6 +1746,11 @@ int64_t pyiid_launch_count(const pyiid_ctx *ctx) {
   return ctx ? ctx->launches : -1;
 }
 
+int64_t pyiid_variant_launches(const pyiid_ctx *ctx, int kernel) {
+  if (!ctx || kernel < 0 || kernel > PYIID_KERNEL_MLP) return -1;
+  return ctx->variant_launches[kernel];
+}
+
 int pyiid_fq(pyiid_ctx *ctx, const float *positions, const int32_t *species,
              int n_atoms, const float *scatter, int n_species, int n_bins,
              double qbin, int k_begin, float *fq) {
@@ -1812,7 +1825,7 @@ int pyiid_grad_fq(pyiid_ctx *ctx, const float *positions,
         positions, L->d_perm, L->d_tiles, L->d_cfg_tiles, dq_hi, dq_lo, kb0,
         chunks_total, n_bins, coef, n_species, gout,
         make_jsplit(n_split, n_tiles, gsize, 0));
-    LAUNCH_CHECK(ctx);
+    VARIANT_LAUNCH_CHECK(ctx, PYIID_KERNEL_GRAD_FQ);
     if (n_split > 1) {
       combine_grad_parts_kernel<<<8 * std::max(1, ctx->n_sms), 256, 0,
                                   ctx->stream>>>(gout, n_split, gsize, gsize,
@@ -1893,7 +1906,7 @@ int pyiid_fq_grad(pyiid_ctx *ctx, const float *positions,
         positions, L->d_perm, L->d_tiles, L->d_cfg_tiles, dq_hi, dq_lo, kb0,
         chunks_total, n_bins, coef, n_species, gout, d_ftab, fpart, 0,
         make_jsplit(n_split, n_tiles, gsize, (size_t)n_tiles * n_bins));
-    LAUNCH_CHECK(ctx);
+    VARIANT_LAUNCH_CHECK(ctx, PYIID_KERNEL_FQ_GRAD);
     if (n_split > 1) {
       combine_grad_parts_kernel<<<8 * std::max(1, ctx->n_sms), 256, 0,
                                   ctx->stream>>>(gout, n_split, gsize, gsize,
@@ -1981,7 +1994,7 @@ int pyiid_fq_grad_part(pyiid_ctx *ctx, const float *positions,
         positions, L->d_perm, L->d_tiles, L->d_cfg_tiles, dq_hi, dq_lo, kb0,
         chunks_total, n_bins, coef, n_species, grad, d_ftab, fpart, t0,
         make_jsplit(1, 1, 0, 0));
-    LAUNCH_CHECK(ctx);
+    VARIANT_LAUNCH_CHECK(ctx, PYIID_KERNEL_FQ_GRAD);
   }
   fqgrad_finish_kernel<<<(n_bins + 3) / 4, 128, 0, ctx->stream>>>(
       fpart, t0, fpart ? t1 : t0, d_na, n_bins, kbo, nullptr, sums);
@@ -2273,7 +2286,7 @@ int pyiid_batch_potential_grad(pyiid_ctx *ctx, const float *positions,
                              ctx->stream>>>(positions, L->d_perm, L->d_tiles,
                                             L->d_cfg_tiles, dq_hi, dq_lo, kb0,
                                             kp, tabs, n_species, grad);
-    LAUNCH_CHECK(ctx);
+    VARIANT_LAUNCH_CHECK(ctx, PYIID_KERNEL_ADJOINT);
   } else if (!L->tiles.empty()) {
     TRY(ensure(ctx, "b_adjpart", std::max<size_t>(L->adj_total, 1) * sizeof(float),
                &p));
@@ -2283,7 +2296,7 @@ int pyiid_batch_potential_grad(pyiid_ctx *ctx, const float *positions,
                                    (kp / 2) * sizeof(float4), ctx->stream>>>(
           positions, L->d_perm, L->d_tiles, L->d_items, L->d_item_order, dq_hi,
           dq_lo, kb0, kp, tabs, n_species, L->d_adj_ioff, L->d_adj_joff, part);
-      LAUNCH_CHECK(ctx);
+      VARIANT_LAUNCH_CHECK(ctx, PYIID_KERNEL_ADJOINT);
     }
     adjoint_reduce_kernel<<<(unsigned)L->tiles.size(), 96, 0, ctx->stream>>>(
         part, L->d_adj_tile_ptr, L->d_adj_entries, L->d_tiles, L->d_perm,
@@ -2942,7 +2955,7 @@ extern "C" int pyiid_fq_noalloc(pyiid_ctx *ctx, const float *positions,
     E.k<<<grid, kBlock, fq_smem(E.v, n_chunks), st>>>(
         positions, d_perm, d_tiles, d_items, nullptr, dq_hi, dq_lo, kb0,
         n_chunks, n_groups, n_bins, d_part);
-    LAUNCH_CHECK(ctx);
+    VARIANT_LAUNCH_CHECK(ctx, PYIID_KERNEL_FQ);
   }
   dim3 g2((n_bins + 127) / 128, 1);
   const int kb_out = (n_items > 0) ? std::min(k_begin, n_bins) : n_bins;
@@ -3352,7 +3365,7 @@ extern "C" int pyiid_surrogate_forces(
       mlp_fused_kernel<<<blocks, 256, sizeof(FusedMlpSmem), ctx->stream>>>(
           X, n, W1, b1, W2, b2, w3, b3, y, gh);
     }
-    LAUNCH_CHECK(ctx);
+    VARIANT_LAUNCH_CHECK(ctx, PYIID_KERNEL_MLP);
     reduce_by_config_kernel<<<n_configs, 256, 0, ctx->stream>>>(
         y, d_off, n_configs, energy);
     LAUNCH_CHECK(ctx);

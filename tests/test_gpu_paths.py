@@ -1,0 +1,236 @@
+"""Which kernels a call runs, and parity of the direct pair kernels (those
+with launch variants) at sizes that the dispatch rules leave to them.
+
+Each test states the path it is about through Context.variant_launches, so a
+rule that moves its sizes elsewhere makes it fail instead of emptying it.
+Tolerances as everywhere (norm-wise relative): F(Q) and potentials 1e-5,
+gradients 1e-4.
+"""
+import numpy as np
+import pytest
+
+from oracle import debye_c as C
+from oracle import debye_np as O
+from pyiid_gb300 import structures as S
+from pyiid_gb300.scatter_factors import form_factor_array, species_tables
+
+pytestmark = pytest.mark.gpu
+
+TOL_F = 1e-5
+TOL_G = 1e-4
+
+
+def rel(a, b):
+    a = np.asarray(a, dtype=np.float64)
+    b = np.asarray(b, dtype=np.float64)
+    nb = np.linalg.norm(b)
+    return np.linalg.norm(a - b) / (nb if nb > 0 else 1.0)
+
+
+@pytest.fixture(scope='module')
+def D():
+    from pyiid_gb300 import debye
+    return debye
+
+
+@pytest.fixture
+def ctx():
+    """The shared context, its variants as they were afterwards."""
+    from pyiid_gb300 import autotune
+    with autotune.variant_scope() as c:
+        yield c
+
+
+def launched(ctx, kernel, fn):
+    """(launches of ``kernel``'s variants, result) of one call."""
+    n = ctx.variant_launches(kernel)
+    out = fn()
+    return ctx.variant_launches(kernel) - n, out
+
+
+def particle(n, seed, species=1):
+    rng = np.random.default_rng(seed)
+    pos = S.displaced(S.fcc_nearest(4.08, n), 0.05, seed)[rng.permutation(n)]
+    nums = rng.choice([46, 78, 79][:species], n) if species > 1 \
+        else np.full(n, 79)
+    return pos.astype(np.float32), nums
+
+
+def fq64(pos, sp, tab, qb, bins):
+    bins = np.asarray(bins, np.int32)
+    return 2 * C.pair_sums(pos, sp, tab, qb, bins) / \
+        O.normalization(tab[sp])[bins]
+
+
+def rows64(pos, sp, tab, qb, rows):
+    return -C.grad_rows(pos, sp, tab, qb, np.asarray(rows, np.int32)) / \
+        O.normalization(tab[sp])
+
+
+# fewer than 64 bins, and more than the grid has: several tiles per work item
+# (1,300 atoms), one element and two
+@pytest.mark.parametrize('n,species,nb', [(70, 2, 500), (1300, 1, 60),
+                                          (1300, 2, 60), (300, 2, 2900)])
+def test_direct_fq_variants_match_oracle(D, ctx, n, species, nb):
+    from pyiid_gb300 import autotune
+    pos, nums = particle(n, n, species)
+    qb, kb = 0.02 if nb > 500 else 0.1, 3
+    sp, tab, _ = species_tables(nums, qb, nb)
+    bins = np.unique(np.concatenate([np.arange(kb, nb, nb // 40 + 1),
+                                     [nb - 1]]))
+    want = fq64(pos, sp, tab, qb, bins)
+    for idx, info in autotune.variants('fq'):
+        ctx.set_variant('fq', idx)
+        ran, f = launched(ctx, 'fq', lambda: D.fq(pos, sp, tab, qb, kb))
+        f = f.cpu().numpy()
+        assert ran == 1
+        assert np.all(f[:kb] == 0)
+        assert rel(f[bins], want) <= TOL_F, (idx, info)
+
+
+def test_direct_persistent_batch_equals_one_cta_per_unit(D, ctx):
+    from pyiid_gb300 import autotune
+    rng = np.random.default_rng(31)
+    sizes = [int(n) for n in rng.integers(2, 90, 40)]
+    parts = [particle(n, 80 + i, 2) for i, n in enumerate(sizes)]
+    pos = np.concatenate([p for p, _ in parts])
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    sp, tab, _ = species_tables(np.concatenate([z for _, z in parts]), 0.05,
+                                500)
+    shapes = {(i['bins_per_thread'], i['pairs_per_thread']): idx
+              for idx, i in autotune.variants('fq')}
+    got = {}
+    for shape in ((56, -3), (56, -13), (56, -13)):
+        ctx.set_variant('fq', shapes[shape])
+        ran, f = launched(ctx, 'fq', lambda: D.batch_fq(pos, sp, off, tab,
+                                                        0.05, 2))
+        assert ran == 1
+        assert np.array_equal(got.setdefault('f', f.cpu().numpy()),
+                              f.cpu().numpy())
+    for i in (0, 7, 39):
+        a, b = off[i], off[i + 1]
+        assert rel(got['f'][i, 2:], O.fq(pos[a:b], tab[sp[a:b]], 0.05)[2:]) \
+            <= TOL_F
+
+
+# beyond the longest transform (2,007 bins); 33 and 70 atoms of two elements
+# (tile remainders), 300 of three (tiles J split over CTAs)
+@pytest.mark.parametrize('n,species', [(33, 2), (70, 2), (300, 3)])
+@pytest.mark.parametrize('kernel', ['grad_fq', 'fq_grad'])
+def test_direct_gradient_variants_match_oracle(D, ctx, kernel, n, species):
+    from pyiid_gb300 import autotune
+    pos, nums = particle(n, 2 * n, species)
+    qb, nb, kb = 0.012, 2101, 3
+    sp, tab, _ = species_tables(nums, qb, nb)
+    rows = [0, n // 3, n - 1]
+    want_g = rows64(pos, sp, tab, qb, rows)[:, :, kb:]
+    bins = np.arange(kb, nb, 53)
+    want_f = fq64(pos, sp, tab, qb, bins)
+    for idx, info in autotune.variants(kernel):
+        ctx.set_variant(kernel, idx)
+        if kernel == 'grad_fq':
+            ran, g = launched(ctx, kernel,
+                              lambda: D.grad_fq(pos, sp, tab, qb, kb))
+        else:
+            ran, (f, g) = launched(ctx, kernel,
+                                   lambda: D.fq_grad(pos, sp, tab, qb, kb))
+            f = f.cpu().numpy()
+            assert np.all(f[:kb] == 0)
+            assert rel(f[bins], want_f) <= TOL_F, (idx, info)
+        assert ran == 1
+        g = g.cpu().numpy()
+        assert np.all(g[:, :, :kb] == 0)
+        assert rel(g[rows][:, :, kb:], want_g) <= TOL_G, (idx, info)
+
+
+def test_direct_split_combine_into_an_output_at_an_odd_offset(D, ctx):
+    """A J-split gradient (coefficients, parts, their combination and F) into
+    an output 4 bytes past a 16-byte boundary equals the aligned call."""
+    import torch
+    n, qb, nb, kb = 100, 0.012, 2101, 2
+    pos, nums = particle(n, 3)
+    sp, tab, _ = species_tables(nums, qb, nb)
+    before = ctx.launches
+    ran, (f, g) = launched(ctx, 'fq_grad',
+                           lambda: D.fq_grad(pos, sp, tab, qb, kb))
+    assert ran == 1 and ctx.launches - before == 4  # 3 without a split
+    big = torch.full((n * 3 * nb + 4,), float('nan'), device='cuda')
+    out = big[1:1 + n * 3 * nb].view(n, 3, nb)
+    assert out.data_ptr() % 16 == 4
+    f2, g2 = D.fq_grad(pos, sp, tab, qb, kb, out_grad=out)
+    assert torch.equal(g2, g) and torch.equal(f2, f)
+    assert torch.isnan(big[0]) and torch.isnan(big[-3:]).all()
+
+
+# few pairs for many (configuration, species pair) tables: one element in
+# single and several tiles, two elements; both forms of the kernel
+@pytest.mark.parametrize('variant', [0, 1])
+@pytest.mark.parametrize('sizes,species,exp', [
+    ([70, 33, 97, 5, 64, 80, 31, 32, 96, 40, 75, 66], 1, {'rmax': 40.0}),
+    ([70, 33, 97], 2, {'rmax': 60.0}),
+    ([130] * 24, 2, {'rmax': 20.0, 'qmin': 0.9}),
+])
+def test_direct_adjoint_variants_match_oracle(D, ctx, sizes, species, exp,
+                                              variant):
+    import torch
+    e = O.update_experiment(dict({'rstep': 0.02, 'rmax': 30.0}, **exp))
+    qb, rg = O.pdf_qbin(e), O.r_grid(e)
+    nb = int(np.floor(e['qmax'] / qb))
+    parts = [particle(n, 200 + i, species) for i, n in enumerate(sizes)]
+    pos = np.concatenate([p for p, _ in parts])
+    nums = np.concatenate([z for _, z in parts])
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    uniq, sp = np.unique(nums, return_inverse=True)
+    sp = sp.reshape(-1).astype(np.int32)
+    tab = np.stack([form_factor_array(z, np.arange(nb) * qb)
+                    for z in uniq]).astype(np.float32)
+    gobs = O.pdf_fft(O.fq(S.random_cube(50, 9.0, 3), np.repeat(tab[:1], 50, 0),
+                          qb), e['rstep'], qb, rg, e['qmin'])
+    ctx.set_variant('adjoint', variant)
+    ran, out = launched(ctx, 'adjoint', lambda: D.batch_potential_grad(
+        pos, sp, off, tab, qb, e['rstep'], rg, e['qmin'],
+        torch.as_tensor(gobs)))
+    assert ran == 1
+    g = out['grad'].cpu().numpy()
+    for i in range(min(3, len(sizes))):
+        a, b = off[i], off[i + 1]
+        _, tg = O.true_grad_potential(pos[a:b], tab[sp[a:b]], e, gobs)
+        assert rel(g[a:b], tg) <= TOL_G, (variant, i, rel(g[a:b], tg))
+
+
+# either side of the rules, far from the line
+@pytest.mark.parametrize('n,species,nb,kb,direct', [
+    (55, 1, 250, 0, True), (250, 2, 500, 2, True), (700, 1, 500, 2, False),
+    (900, 2, 500, 2, False), (2000, 1, 63, 0, True),
+])
+def test_fq_path(D, ctx, n, species, nb, kb, direct):
+    pos, nums = particle(n, n, species)
+    sp, tab, _ = species_tables(nums, 0.05, nb)
+    ran, _ = launched(ctx, 'fq', lambda: D.fq(pos, sp, tab, 0.05, kb))
+    assert ran == direct
+
+
+def test_grid_fq_close_coincident_and_far_pairs(D, ctx):
+    """Pairs at tiny distances (power sums), under 0.1 A and beyond 128 A
+    (general distance) against the oracle; a coincident pair makes every bin
+    0, and so does a NaN position, in its own configuration only."""
+    qb, nb, n = 0.05, 500, 700
+    pos, nums = particle(n, 9, 2)
+    pos[30] = pos[7] + np.float32([1e-3, 0, 0])
+    pos[31] = pos[8] + np.float32([0.02, 0.03, 0.01])
+    pos[32] += np.float32([150.0, 0, 0])
+    sp, tab, _ = species_tables(nums, qb, nb)
+    bins = np.arange(0, nb, 9)
+    want = fq64(pos, sp, tab, qb, bins)
+    ran, f = launched(ctx, 'fq', lambda: D.fq(pos, sp, tab, qb))
+    assert ran == 0 and rel(f.cpu().numpy()[bins], want) <= TOL_F
+    bad, nan, inf = pos.copy(), pos.copy(), pos.copy()
+    bad[30] = bad[7]
+    nan[5, 1] = np.nan
+    inf[6, 2] = np.inf
+    ran, f = launched(ctx, 'fq', lambda: D.batch_fq(
+        np.concatenate([bad, pos, nan, pos, inf]), np.tile(sp, 5),
+        np.arange(6) * n, tab, qb))
+    f = f.cpu().numpy()
+    assert ran == 0 and np.all(f[[0, 2, 4]] == 0)
+    assert rel(f[1, bins], want) <= TOL_F and rel(f[3, bins], want) <= TOL_F
