@@ -209,11 +209,11 @@ struct DevBuf {
   size_t bytes = 0;
 };
 
-// Work of the F(Q) grid path for one layout and bin count: the rows of
+// Work of the F(Q) grid path for one layout and range of bins: the rows of
 // columns of the configurations that take it, and what is left to the direct
 // kernels.
 struct FqGridWork {
-  int n_bins = 0;
+  int n_bins = 0, k_begin = 0;
   int n_segs = 0, total = 0, n_keys = 0, n_cfgs = 0;  // n_cfgs 0: no work
   int n_wide = 0;    // the last of them take the transform in FP64
   int n_direct = 0;  // work items of the other configurations
@@ -272,7 +272,7 @@ struct Layout {
   int *d_item_order = nullptr;
   int *d_key_item_begin = nullptr;
   int2 *d_spair = nullptr;
-  std::vector<std::unique_ptr<FqGridWork>> fq_grid;  // by n_bins, newest first
+  std::vector<std::unique_ptr<FqGridWork>> fq_grid;  // newest first
   std::unique_ptr<GradGridWork> grad_grid;
 };
 
@@ -968,41 +968,59 @@ int get_phase_grid(pyiid_ctx *ctx, int n_bins, int m, bool with_grad,
 }
 
 // Which configurations of a layout take the F(Q) grid path (empty: none).
-// Times in us of both paths, fitted to single configurations of 60 to 2,000
-// atoms and batches of 16 to 256 x 40 to 320 atoms, each of one to three
-// elements at 250, 500 and 1,500 bins: the grid path spends four launches,
-// and on each (configuration, species pair) a transform of 2.8e-4 n_bins,
-// but 1.5e-5 per pair where the direct kernels spend 1.3e-7 n_bins (2e-7
-// while the pairs do not fill the GPU).  A configuration takes it if its own
-// pairs pay for its transforms, and all of those do if together they pay for
-// the launches.  Either side of the line, direct / grid: 300 atoms at 500
-// bins 22.3 / 23.5, 420 26.6 / 26.0, 1,000 91.6 / 44.1; 420 of three elements
-// at 1,500 bins 49 / 67, 600 80 / 69; 64 x 80 of two elements at 500 bins
-// 28 / 54, 64 x 160 70 / 61, 256 x 320 859 / 234.
-std::vector<int> fq_grid_configs(const Layout *L, int n_bins) {
+// Times in us of both paths, fitted to 2,600 calls of each: 1 to 256
+// configurations of 16 to 4,000 atoms, one to three elements, 64 to 2,500
+// bins of which the last 2 % to all are returned.  The direct kernels skip
+// the bins below k_begin (though a pair never costs less than about 56 of
+// them); few pairs leave them with the time of one work item, and their finish
+// adds a configuration's items one by one.  The grid path spends four
+// launches, a transform of 2.2e-7 n_bins^2 on each (configuration, species
+// pair) and the same on a pair whatever its bins.  A configuration of a batch
+// takes it if its own pairs pay for its transforms, and all of those do if
+// together they pay for the launches, with 10 % to spare for what the fit does
+// not see.  Either side of the line, direct / grid: 300 atoms at 500 bins
+// 25.1 / 27.4, 420 29.1 / 27.0, 900 72.4 / 31.2; 250 of two elements at 1,500
+// bins 45.4 / 37.3, the last 30 of them 17.1 / 36.3; 64 x 90 of two elements at
+// 500 bins 31.8 / 54.0, 64 x 160 74.2 / 59.8, the last 50 of them 31.3 / 57.9.
+std::vector<int> fq_grid_configs(const Layout *L, int n_bins, int k_begin) {
   std::vector<int> on;
   if (n_bins < 64 || n_bins > kFqGridMaxBins) return on;
-  const double k = n_bins;
-  double pairs = 0, keys = 0, most_keys = 0;
+  const int S = L->n_spairs;
+  const double k = n_bins, ke = n_bins - (k_begin & ~1);
+  const double direct_pair = 1.4e-5 + 1.15e-7 * std::max(ke, 56.0);
+  const double grid_pair = 7.4e-6;
+  double pairs = 0, keys = 0, most_pairs = 0, most_keys = 0, most_items = 0;
+  bool rest = false;
   for (int c = 0; c < L->n_configs; ++c) {
     double p = 0, n = 0;
-    for (int s = 0; s < L->n_spairs; ++s) {
-      const double ps = L->pair_counts[(size_t)c * L->n_spairs + s];
+    for (int s = 0; s < S; ++s) {
+      const double ps = L->pair_counts[(size_t)c * S + s];
       p += ps;
       n += ps > 0;
     }
-    if (p * (1.3e-7 * k - 1.5e-5) <= 2.8e-4 * k * n) continue;
+    if (L->n_configs > 1 &&
+        p * (direct_pair - grid_pair) <= 1.4e-4 * k + 2.2e-7 * k * k * n) {
+      rest |= p > 0;
+      continue;
+    }
     on.push_back(c);
     pairs += p;
     keys += n;
+    most_pairs = std::max(most_pairs, p);
     most_keys = std::max(most_keys, n);
+    most_items = std::max<double>(
+        most_items, L->key_item_begin[(size_t)(c + 1) * S] -
+                        L->key_item_begin[(size_t)c * S]);
   }
-  const double pk = pairs * k;
+  // (the launches of the direct kernels stay if they have other work)
   const double direct =
-      10 + k / 60 + (pk < 3e8 ? 2e-7 * pk : 18 + 1.4e-7 * pk);
-  const double grid = 19.5 + most_keys * (2 + k / 250) + 2.8e-4 * k * keys +
-                      1.5e-5 * pairs;
-  if (grid >= direct) on.clear();
+      (rest ? 0.0 : 12.7) + 0.075 * most_items +
+      std::max(0.0195 * ke * std::min(1.0, most_pairs / 1000),
+               0.0098 * ke + direct_pair * pairs);
+  const double grid = 25 + 0.002 * k + most_keys * (0.3 + 0.0012 * k) +
+                      1.4e-4 * k * on.size() + 2.2e-7 * k * k * keys +
+                      grid_pair * pairs;
+  if (grid >= 0.9 * direct) on.clear();
   return on;
 }
 
@@ -1016,22 +1034,23 @@ bool wide_sums(const Layout *L, int c) {
 }
 
 // The grid path's share of a layout (n_cfgs == 0: none of it).
-int get_fq_grid_work(pyiid_ctx *ctx, Layout *L, int n_bins,
+int get_fq_grid_work(pyiid_ctx *ctx, Layout *L, int n_bins, int k_begin,
                      FqGridWork **out) {
   for (auto &W : L->fq_grid)
-    if (W->n_bins == n_bins) {
+    if (W->n_bins == n_bins && W->k_begin == k_begin) {
       *out = W.get();
       return PYIID_OK;
     }
   auto W = std::make_unique<FqGridWork>();
   W->n_bins = n_bins;
+  W->k_begin = k_begin;
   std::vector<GridSeg> segs;
   std::vector<int> begin, key_spair, direct;
   std::vector<int4> cfg_keys;
   std::vector<KeyCols> cols;  // columns of each key
   std::vector<unsigned char> skip(L->n_configs, 0);
   long long total = 0;
-  std::vector<int> on = fq_grid_configs(L, n_bins);
+  std::vector<int> on = fq_grid_configs(L, n_bins, k_begin);
   const auto wide = std::stable_partition(
       on.begin(), on.end(), [&](int c) { return !wide_sums(L, c); });
   W->n_wide = (int)(on.end() - wide);
@@ -1331,7 +1350,7 @@ int run_fq(pyiid_ctx *ctx, Layout *L, const float *positions,
   double *partial = nullptr;
   if (n_items > 0 && kb0 < n_bins) {
     FqGridWork *W;
-    TRY(get_fq_grid_work(ctx, L, n_bins, &W));
+    TRY(get_fq_grid_work(ctx, L, n_bins, k_begin, &W));
     if (W->n_cfgs > 0) {
       TRY(run_fq_grid(ctx, L, W, positions, d_ftab, d_na, n_bins, qbin,
                       std::min(k_begin, n_bins), fq, fq_raw));
@@ -1439,29 +1458,47 @@ const GradTransformEntry *grad_transform_for(int n_bins) {
 }
 
 // Whether a gradient (with_f: and F(Q) beside it) goes through the grid.
-// Times in us of both paths, fitted to 16 to 640 atoms of one to three
-// elements at 250, 500 and 1,500 bins.  Direct: a tile's 32 partners one
-// after the other while the pairs do not fill the GPU, then 5.1e-7 per pair
-// and bin.  Grid: its launches, and per species pair of F a transform or per
-// species the sums of the rows.  Measured, direct / grid: 16 atoms at 500
-// bins 20.7 / 24.2 (gradient alone 18.6 / 13.3), 32 35.2 / 21.5, 249
-// 52.8 / 26.5, 1,000 276 / 77; of two elements 64 36.1 / 36.3, 249
-// 53.4 / 40.8; of three 160 37.8 / 50.1, 400 79.2 / 73.9; of two at 1,500
-// bins 160 54.9 / 65.8, 249 78.7 / 75.3, 2,001 (gradient) 2,050 / 374.
-bool grad_on_grid(const Layout *L, int n_bins, bool with_f) {
+// Times in us of both paths, fitted to 1,350 calls of each: 16 to 4,000 atoms,
+// one to three elements, 16 to 1,500 bins of which the last 2 % to all are
+// returned.  Direct: a tile's 32 partners one after the other while the pairs
+// do not fill the GPU, then so much per pair (of full tiles) and bin from
+// k_begin on, 56 of them at least.  Grid: its launches, the transforms (per
+// atom and species; of F per species pair) and the pairs, whatever the bins
+// returned.  Measured, direct / grid: 16 atoms at 1,500 bins 23.6 / 47.9
+// (gradient alone 21.0 / 20.7), 32 at 500 36.0 / 24.9, 250 55.9 / 29.7, 900
+// 247 / 68, 250 at 16 29.3 / 33.5; of two elements 64 39.7 / 33.3, 250
+// 58.8 / 40.3; of three 160 40.2 / 45.9, 300 75.0 / 57.3; of two at 1,500 bins
+// 160 59.1 / 68.1, 250 83.3 / 79.9; of three 900 589 / 277, the last 30 of
+// them 127 / 261.
+bool grad_on_grid(const Layout *L, int n_bins, int k_begin, bool with_f) {
   const GradTransformEntry *E = grad_transform_for(n_bins);
   if (!E || L->n_configs != 1 || L->total < 2) return false;
   std::vector<int> count(L->n_species, 0);
   for (const int4 &t : L->tiles) count[t.w] += t.y;
   double s = 0;
   for (int c : count) s += c > 0;
-  const double n = L->total, k = n_bins, x = n * n * k;
-  double direct = x > 2.5e7 ? 37.7 + 5.1e-7 * x
-                            : 9.5 + 0.78 * std::min(32.0, n / s);
-  if (!with_f) direct *= 0.85;
-  const double grid =
-      (with_f ? 18 + s * (s + 1) / 2 * (2.5 + k / 165) : 12 + s * (4 + k / 300)) +
-      5e-5 * s * k * std::max(0.0, n - 100);
+  const double n = L->total, k = n_bins, ke = n_bins - (k_begin & ~1);
+  const double np = (double)kTile * L->tiles.size();
+  const double km = std::max(ke, 56.0), k1 = std::min(ke, 250.0) / 250;
+  const double len = std::min(32.0, n / s), sp = s * (s + 1) / 2;
+  const double kt = 1e-4 * std::min(km, 500.0);
+  const double rows_t = s * std::max(0.0, n - 100) * E->len;
+  double direct, grid;
+  if (with_f) {
+    direct = std::max(12.7 + len * (0.47 + 0.43 * k1),
+                      16 + np * (0.034 + 1.3 * kt) +
+                          np * np * (4.1e-5 + 2.8e-7 * km));
+    // (short transforms of many atoms do not cover F's sums beside them)
+    const double few = n < 100 ? 0 : std::max(0.0, 5 - k / 100);
+    grid = 24.3 + few + sp * (1.1 + 0.0054 * k) + 0.0018 * s * k +
+           2.1e-5 * n * n + 2.6e-5 * rows_t;
+  } else {
+    direct = std::max(8.7 + len * (0.47 + 0.46 * k1),
+                      11.5 + np * (0.033 + 1.35 * kt) +
+                          np * np * (5.2e-5 + 2.1e-7 * km));
+    grid = 13.1 + 0.039 * std::min(n, 100.0) + 1.3 * sp + 0.0035 * s * k +
+           1.95e-5 * n * n + 2.7e-5 * rows_t;
+  }
   // the rows of all units (and those of far pairs) stay under 24 GB, and the
   // columns under 2^31
   const double rows = 6.0 * 4.0 * (n * s + 1e4) * grid_words(E->len);
@@ -1788,7 +1825,7 @@ int pyiid_grad_fq(pyiid_ctx *ctx, const float *positions,
   TRY(get_na(ctx, L, scatter, n_bins, &d_na));
   const int kbo = std::min(k_begin, n_bins);
   const int kb0 = kbo & ~1;
-  if (kbo < n_bins && grad_on_grid(L, n_bins, false))
+  if (kbo < n_bins && grad_on_grid(L, n_bins, kbo, false))
     return run_grad_grid(ctx, L, positions, d_ftab, d_na, n_bins, qbin, kbo,
                          nullptr, grad);
   void *p;
@@ -1869,7 +1906,7 @@ int pyiid_fq_grad(pyiid_ctx *ctx, const float *positions,
   const int kbo = std::min(k_begin, n_bins);
   const int kb0 = kbo & ~1;
   const int n_tiles = (int)L->tiles.size();
-  if (kbo < n_bins && grad_on_grid(L, n_bins, true))
+  if (kbo < n_bins && grad_on_grid(L, n_bins, kbo, true))
     return run_grad_grid(ctx, L, positions, d_ftab, d_na, n_bins, qbin, kbo,
                          fq, grad);
   double *fpart = nullptr;

@@ -210,6 +210,41 @@ def test_fq_path(D, ctx, n, species, nb, kb, direct):
     assert ran == direct
 
 
+# the direct kernels skip the bins below k_begin, the grid does not: (two
+# elements) the same call for all bins and for the last few
+@pytest.mark.parametrize('n,copies,nb,kb', [(160, 64, 500, 450),
+                                            (200, 64, 1500, 1490),
+                                            (300, 1, 2500, 2450)])
+def test_fq_path_of_the_last_bins(D, ctx, n, copies, nb, kb):
+    pos, nums = particle(n, n, 2)
+    sp, tab, _ = species_tables(nums, 0.02, nb)
+    pos, sp = np.tile(pos, (copies, 1)), np.tile(sp, copies)
+    off = np.arange(copies + 1) * n
+    all_bins = launched(ctx, 'fq',
+                        lambda: D.batch_fq(pos, sp, off, tab, 0.02))
+    last = launched(ctx, 'fq',
+                    lambda: D.batch_fq(pos, sp, off, tab, 0.02, kb))
+    assert all_bins[0] == 0 and last[0] == 1
+    f, g = all_bins[1].cpu().numpy(), last[1].cpu().numpy()
+    assert np.all(g[:, :kb] == 0)
+    assert rel(g[:, kb:], f[:, kb:]) <= TOL_F
+
+
+@pytest.mark.parametrize('kernel', ['grad_fq', 'fq_grad'])
+def test_gradient_path_of_the_last_bins(D, ctx, kernel):
+    n, nb, kb = 900, 1500, 1470
+    pos, nums = particle(n, n, 3)
+    sp, tab, _ = species_tables(nums, 0.02, nb)
+    call = getattr(D, kernel)
+    all_bins = launched(ctx, kernel, lambda: call(pos, sp, tab, 0.02))
+    last = launched(ctx, kernel, lambda: call(pos, sp, tab, 0.02, kb))
+    assert all_bins[0] == 0 and last[0] == 1
+    g, g1 = ((x[1] if kernel == 'fq_grad' else x).cpu().numpy()
+             for x in (all_bins[1], last[1]))
+    assert np.all(g1[:, :, :kb] == 0)
+    assert rel(g1[:, :, kb:], g[:, :, kb:]) <= TOL_G
+
+
 def test_grid_fq_close_coincident_and_far_pairs(D, ctx):
     """Pairs at tiny distances (power sums), under 0.1 A and beyond 128 A
     (general distance) against the oracle; a coincident pair makes every bin
