@@ -74,6 +74,15 @@ int pyiid_synchronize(pyiid_ctx *ctx);
  * NULL).  The string stays valid until the next call on the same context. */
 const char *pyiid_last_error(const pyiid_ctx *ctx);
 
+/* Most device memory (bytes) that the per-atom rows of a gradient may take
+ * where pyiid_grad_fq and pyiid_fq_grad go through their phase grid (24
+ * bytes x 2 to 3 n_bins per atom and element, and 2,432 times as much); 2 GiB
+ * at first.  A gradient that needs more runs in parts.  One that
+ * the limit leaves no room for, or for which the device has no memory, runs
+ * the kernels that need none.  What a call has allocated stays with the
+ * context. */
+int pyiid_set_workspace_limit(pyiid_ctx *ctx, size_t bytes);
+
 /* Number of kernels this context has launched so far (for launch accounting). */
 int64_t pyiid_launch_count(const pyiid_ctx *ctx);
 

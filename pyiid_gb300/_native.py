@@ -30,6 +30,7 @@ _SIGNATURES = {
     'pyiid_destroy': (_c_int, [_vp]),
     'pyiid_set_stream': (_c_int, [_vp, _vp]),
     'pyiid_synchronize': (_c_int, [_vp]),
+    'pyiid_set_workspace_limit': (_c_int, [_vp, ctypes.c_size_t]),
     'pyiid_last_error': (ctypes.c_char_p, [_vp]),
     'pyiid_launch_count': (ctypes.c_int64, [_vp]),
     'pyiid_fq': (_c_int, [_vp, _vp, _i32p, _c_int, _f32p, _c_int, _c_int,
@@ -199,6 +200,12 @@ class Context:
 
     def get_variant(self, kernel):
         return int(self._lib.pyiid_get_variant(self.handle, KERNELS[kernel]))
+
+    def set_workspace_limit(self, n_bytes):
+        """Most device memory of a gradient's rows (2 GiB at first)."""
+        self.check(self._lib.pyiid_set_workspace_limit(self.handle,
+                                                       int(n_bytes)),
+                   'pyiid_set_workspace_limit')
 
     def variant_launches(self, kernel):
         """Launches so far of the kernels whose shape a variant selects."""

@@ -226,12 +226,17 @@ struct FqGridWork {
   unsigned char *d_skip = nullptr;
 };
 
-// Work of the gradient's grid path for a layout of one configuration.
+// Work of the gradient's grid path for a layout of one configuration, in
+// parts of its atoms that use the workspace one after the other.
 struct GradGridWork {
-  int total = 0, units = 0, staged = 0;
-  GradBlock *d_blocks = nullptr;   // [n_species][n_species]
-  KeyCols *d_key_cols = nullptr;   // columns of each species pair
-  int *d_key_spair = nullptr;
+  struct Part {
+    int a_first = 0, n = 0, total = 0;  // atoms, columns
+  };
+  std::vector<Part> parts;
+  int units = 0, staged = 0;       // units of the largest part
+  GradBlock *d_blocks = nullptr;   // [part][n_species][n_species]
+  KeyCols *d_key_cols = nullptr;   // [part] columns of each species pair
+  int *d_key_spair = nullptr;      // [part][n_spairs]
   int4 *d_cfg_keys = nullptr;
 };
 
@@ -273,7 +278,7 @@ struct Layout {
   int *d_key_item_begin = nullptr;
   int2 *d_spair = nullptr;
   std::vector<std::unique_ptr<FqGridWork>> fq_grid;  // newest first
-  std::unique_ptr<GradGridWork> grad_grid;
+  std::vector<std::unique_ptr<GradGridWork>> grad_grid;  // by parts
 };
 
 // Phase grid of n_bins bins (independent of their step): the window's
@@ -341,6 +346,9 @@ struct pyiid_ctx {
   // two tiles in flight per CTA (default: 57 against 70 us for mma.sync)
   int mlp_variant = 2;
   int n_sms = 0;  // streaming multiprocessors of the device
+  // most bytes of the rows of a gradient on the phase grid (20,000 atoms of
+  // one element at 1,500 bins: 1.66 GB, in one part)
+  size_t workspace_limit = (size_t)2 << 30;
   // device word a kernel sets when one of its bounded waits gave up
   // (reported and cleared by pyiid_synchronize)
   int *d_status = nullptr;
@@ -413,6 +421,12 @@ int ensure(pyiid_ctx *ctx, const char *name, size_t bytes, void **out) {
   return PYIID_OK;
 }
 
+void release(pyiid_ctx *ctx, const char *name) {
+  DevBuf &b = ctx->bufs[name];
+  cudaFree(b.p);
+  b = DevBuf{};
+}
+
 template <class T>
 int upload(pyiid_ctx *ctx, T **dst, const std::vector<T> &src) {
   if (*dst) CUDA_TRY(ctx, cudaFree(*dst));
@@ -435,6 +449,13 @@ void free_fq_grid(FqGridWork *W) {
   cudaFree(W->d_skip);
 }
 
+void free_grad_grid(GradGridWork *W) {
+  cudaFree(W->d_blocks);
+  cudaFree(W->d_key_cols);
+  cudaFree(W->d_key_spair);
+  cudaFree(W->d_cfg_keys);
+}
+
 void free_phase_grid(PhaseGrid *G) {
   cudaFree(G->d_taps);
   cudaFree(G->d_inv_phi);
@@ -444,12 +465,7 @@ void free_phase_grid(PhaseGrid *G) {
 
 void free_layout(Layout *L) {
   for (auto &W : L->fq_grid) free_fq_grid(W.get());
-  if (L->grad_grid) {
-    cudaFree(L->grad_grid->d_blocks);
-    cudaFree(L->grad_grid->d_key_cols);
-    cudaFree(L->grad_grid->d_key_spair);
-    cudaFree(L->grad_grid->d_cfg_keys);
-  }
+  for (auto &W : L->grad_grid) free_grad_grid(W.get());
   cudaFree(L->d_perm);
   cudaFree(L->d_tiles);
   cudaFree(L->d_cfg_tiles);
@@ -1292,7 +1308,29 @@ int launch_fq_finish(pyiid_ctx *ctx, const FqFinish &a, int first, int n,
   return PYIID_OK;
 }
 
+// Device memory of F(Q) on the grid.
+struct FqGridBuffers {
+  HistRows rows;
+  float *hsum;
+  int *ext;
+};
+
+int ensure_fq_grid_buffers(pyiid_ctx *ctx, const FqGridWork *W, int m,
+                           FqGridBuffers *b) {
+  TRY(hist_rows(ctx, "fqg", W->n_keys, grid_words(m / 2), &b->rows));
+  TRY(ensure(ctx, "fqg_low",
+             (size_t)kSpreadWarps * ctx->n_sms * b->rows.row_words *
+                 sizeof(float),
+             (void **)&b->rows.low));
+  TRY(ensure(ctx, "fqg_sum",
+             (size_t)W->n_keys * fq_sum_floats(m) * sizeof(float),
+             (void **)&b->hsum));
+  return ensure(ctx, "fqg_ext", (size_t)W->n_cfgs * sizeof(int),
+                (void **)&b->ext);
+}
+
 // F(Q) of the configurations of W (fq_grid.cuh): spread, sum, transform.
+// PYIID_ERR_OOM without any of it if there is no memory for it.
 int run_fq_grid(pyiid_ctx *ctx, const Layout *L, const FqGridWork *W,
                 const float *positions, const float *d_ftab,
                 const double *d_na, int n_bins, double qbin, int kb_out,
@@ -1300,37 +1338,27 @@ int run_fq_grid(pyiid_ctx *ctx, const Layout *L, const FqGridWork *W,
   PhaseGrid *G;
   const int m = (kFqCellsPerBin * n_bins + 3) & ~3;
   TRY(get_phase_grid(ctx, n_bins, m, false, &G));
+  FqGridBuffers b;
+  TRY(ensure_fq_grid_buffers(ctx, W, m, &b));
   const int n_ctas = ctx->n_sms;
-  HistRows rows;
-  TRY(hist_rows(ctx, "fqg", W->n_keys, grid_words(m / 2), &rows));
-  void *p;
-  TRY(ensure(ctx, "fqg_low",
-             (size_t)kSpreadWarps * n_ctas * rows.row_words * sizeof(float),
-             &p));
-  rows.low = static_cast<float *>(p);
-  TRY(ensure(ctx, "fqg_sum",
-             (size_t)W->n_keys * fq_sum_floats(m) * sizeof(float), &p));
-  float *hsum = static_cast<float *>(p);
-  TRY(ensure(ctx, "fqg_ext", (size_t)W->n_cfgs * sizeof(int), &p));
-  int *ext = static_cast<int *>(p);
   const GridScale gs = grid_scale(qbin, m);
   // (about twenty atoms per thread, but small CTAs for batches)
   grid_extent_kernel<<<W->n_cfgs, W->n_cfgs > 8 ? 256 : 1024, 0,
                        ctx->stream>>>(positions, L->d_offsets, W->d_cfg_keys,
-                                      gs.hi, m / 2, ext);
+                                      gs.hi, m / 2, b.ext);
   LAUNCH_CHECK(ctx);
   fq_spread_kernel<<<n_ctas, 32 * kSpreadWarps, kSpreadSmem, ctx->stream>>>(
       positions, L->d_perm, W->d_segs, W->d_seg_begin, W->n_segs, W->total,
-      ext, W->n_cfgs, gs, (float)(kNearPhase / (n_bins * qbin)),
-      (float)(n_bins * qbin), G->d_taps, rows);
+      b.ext, W->n_cfgs, gs, (float)(kNearPhase / (n_bins * qbin)),
+      (float)(n_bins * qbin), G->d_taps, b.rows);
   LAUNCH_CHECK(ctx);
   // partial histograms of a key: one per CTA, or per warp where the keys are
   // so many that CTAs hold several
   const double most =
       (double)n_ctas / W->n_keys * (W->n_keys > n_ctas / 4 ? kSpreadWarps : 1);
-  TRY(launch_grid_reduce(ctx, rows, W->d_key_cols, ext, W->n_cfgs, kFqPlan,
-                         W->total, m, W->n_keys, most, hsum));
-  const FqFinish fin{hsum, W->d_cfg_keys, W->d_key_spair, L->d_spair, d_ftab,
+  TRY(launch_grid_reduce(ctx, b.rows, W->d_key_cols, b.ext, W->n_cfgs, kFqPlan,
+                         W->total, m, W->n_keys, most, b.hsum));
+  const FqFinish fin{b.hsum, W->d_cfg_keys, W->d_key_spair, L->d_spair, d_ftab,
                      d_na, G->d_inv_phi, m, n_bins, kb_out, qbin, fq, fq_raw};
   TRY(launch_fq_finish(ctx, fin, 0, W->n_cfgs - W->n_wide, false));
   TRY(launch_fq_finish(ctx, fin, W->n_cfgs - W->n_wide, W->n_wide, true));
@@ -1351,9 +1379,16 @@ int run_fq(pyiid_ctx *ctx, Layout *L, const float *positions,
   if (n_items > 0 && kb0 < n_bins) {
     FqGridWork *W;
     TRY(get_fq_grid_work(ctx, L, n_bins, k_begin, &W));
-    if (W->n_cfgs > 0) {
-      TRY(run_fq_grid(ctx, L, W, positions, d_ftab, d_na, n_bins, qbin,
-                      std::min(k_begin, n_bins), fq, fq_raw));
+    const int rc =
+        W->n_cfgs == 0
+            ? PYIID_OK
+            : run_fq_grid(ctx, L, W, positions, d_ftab, d_na, n_bins, qbin,
+                          std::min(k_begin, n_bins), fq, fq_raw);
+    if (rc == PYIID_ERR_OOM) {
+      cudaGetLastError();  // the direct kernels need less
+    } else if (rc != PYIID_OK) {
+      return rc;
+    } else if (W->n_cfgs > 0) {
       if (W->n_cfgs == L->n_configs) return PYIID_OK;
       n_items = W->n_direct;
       order = W->d_direct_order;
@@ -1410,7 +1445,7 @@ int run_fq(pyiid_ctx *ctx, Layout *L, const float *positions,
 
 // ------------------------------------------------ gradient on the grid
 using GradTransform = void (*)(const float *, const float *, const int *,
-                               const int2 *, const GradBlock *, int,
+                               const int2 *, const GradBlock *, int, int,
                                const int *, const int *, const float2 *,
                                const float2 *, const float *, int, int, float,
                                float, float *, FqReduceArgs);
@@ -1499,114 +1534,170 @@ bool grad_on_grid(const Layout *L, int n_bins, int k_begin, bool with_f) {
     grid = 13.1 + 0.039 * std::min(n, 100.0) + 1.3 * sp + 0.0035 * s * k +
            1.95e-5 * n * n + 2.7e-5 * rows_t;
   }
-  // the rows of all units (and those of far pairs) stay under 24 GB, and the
-  // columns under 2^31
-  const double rows = 6.0 * 4.0 * (n * s + 1e4) * grid_words(E->len);
-  return grid < direct && rows < 24e9 && n * (n / 32 + s) < 2e9;
+  // (columns are counted in int)
+  return grid < direct && n * (n / 32 + s) < 2e9;
 }
 
-int get_grad_grid_work(pyiid_ctx *ctx, Layout *L, GradGridWork **out) {
-  if (!L->grad_grid) {
-    const int S = L->n_species;
-    std::vector<int> start(S, 0), count(S, 0), staged(S + 1, 0);
-    for (const int4 &t : L->tiles) count[t.w] += t.y;
-    for (int s = 1; s < S; ++s) start[s] = start[s - 1] + count[s - 1];
-    for (int s = 0; s < S; ++s)
-      staged[s + 1] = staged[s] + (count[s] + 31) / 32 * 32;
-    auto W = std::make_unique<GradGridWork>();
-    W->staged = staged[S];
-    std::vector<GradBlock> blocks;
+int get_grad_grid_work(pyiid_ctx *ctx, Layout *L, int n_parts,
+                       GradGridWork **out) {
+  for (auto &W : L->grad_grid)
+    if ((int)W->parts.size() == n_parts) {
+      *out = W.get();
+      return PYIID_OK;
+    }
+  const int S = L->n_species, N = L->total;
+  std::vector<int> start(S + 1, 0), staged(S + 1, 0);
+  for (const int4 &t : L->tiles) start[t.w + 1] += t.y;
+  for (int s = 0; s < S; ++s) {
+    staged[s + 1] = staged[s] + (start[s + 1] + 31) / 32 * 32;
+    start[s + 1] += start[s];
+  }
+  auto W = std::make_unique<GradGridWork>();
+  W->staged = staged[S];
+  std::vector<GradBlock> blocks;
+  std::vector<KeyCols> keys;
+  std::vector<int> spair;
+  for (int part = 0; part < n_parts; ++part) {
+    const int lo = (int)((long long)part * N / n_parts);
+    const int hi = (int)((long long)(part + 1) * N / n_parts);
     std::vector<int2> cols;
-    long long total = 0;
-    for (int sa = 0; sa < S; ++sa)
+    int total = 0, units = 0;
+    for (int sa = 0; sa < S; ++sa) {
+      const int a0 = std::min(std::max(start[sa], lo), hi);
+      const int na = std::min(std::max(start[sa + 1], lo), hi) - a0;
+      const int cols_a = (start[sa + 1] - start[sa] + 31) / 32;
       for (int sb = 0; sb < S; ++sb) {
-        const int nc = (count[sb] + 31) / 32;
-        blocks.push_back(GradBlock{(int)total, count[sa] ? nc : 0, W->units,
-                                   start[sa], count[sa], start[sb], count[sb],
-                                   staged[sa], staged[sb]});
-        const long long end = total + (long long)nc * count[sa];
-        cols.push_back(make_int2((int)total, (int)end));
-        total = end;
-        if (nc) W->units += count[sa];
+        const int nb = start[sb + 1] - start[sb], nc = (nb + 31) / 32;
+        blocks.push_back(GradBlock{total, na ? nc : 0, units, a0, na, start[sb],
+                                   nb, staged[sa], staged[sb], a0 - start[sa],
+                                   cols_a});
+        cols.push_back(make_int2(total, total + nc * na));
+        total += nc * na;
+        if (nc) units += na;
       }
+    }
     // F(Q): both orders of a species pair together
-    std::vector<KeyCols> keys;
-    std::vector<int> spair;
     for (int sa = 0; sa < S; ++sa)
       for (int sb = 0; sb <= sa; ++sb) {
         const int p = sa * S + sb, q = sb * S + sa;
-        keys.push_back(KeyCols{cols[p].x, cols[p].y, p, sa == sb ? 0 : cols[q].x,
+        keys.push_back(KeyCols{cols[p].x, cols[p].y, p,
+                               sa == sb ? 0 : cols[q].x,
                                sa == sb ? 0 : cols[q].y, q});
         spair.push_back(sa * (sa + 1) / 2 + sb);
       }
-    W->total = (int)total;
-    TRY(upload(ctx, &W->d_blocks, blocks));
-    TRY(upload(ctx, &W->d_key_cols, keys));
-    TRY(upload(ctx, &W->d_key_spair, spair));
-    TRY(upload(ctx, &W->d_cfg_keys,
-               std::vector<int4>{make_int4(0, 0, (int)keys.size(), 0)}));
-    L->grad_grid = std::move(W);
+    W->parts.push_back(GradGridWork::Part{lo, hi - lo, total});
+    W->units = std::max(W->units, units);
   }
-  *out = L->grad_grid.get();
+  TRY(upload(ctx, &W->d_blocks, blocks));
+  TRY(upload(ctx, &W->d_key_cols, keys));
+  TRY(upload(ctx, &W->d_key_spair, spair));
+  TRY(upload(ctx, &W->d_cfg_keys,
+             std::vector<int4>{make_int4(0, 0, (int)keys.size(), 0)}));
+  L->grad_grid.push_back(std::move(W));
+  *out = L->grad_grid.back().get();
   return PYIID_OK;
 }
 
+// Device memory of the gradient on the grid.
+struct GradBuffers {
+  float *rows, *rows2, *fsum, *coef;
+  float4 *atoms;
+  int *flag, *ext;
+  int2 *parts;
+  HistRows frows;
+};
+
+int ensure_grad_buffers(pyiid_ctx *ctx, const Layout *L, const GradGridWork *W,
+                        int n_bins, int m, GradBuffers *b) {
+  const int S = L->n_species, row_words = grid_words(m / 2);
+  const size_t n_rows = (size_t)W->units + kSpreadWarps * ctx->n_sms;
+  const size_t row_bytes = n_rows * 3 * row_words * sizeof(float);
+  TRY(ensure(ctx, "gg_rows", row_bytes, (void **)&b->rows));
+  TRY(ensure(ctx, "gg_rows2", row_bytes, (void **)&b->rows2));
+  TRY(ensure(ctx, "gg_flag", n_rows * sizeof(int), (void **)&b->flag));
+  TRY(ensure(ctx, "gg_parts", W->units * sizeof(int2), (void **)&b->parts));
+  TRY(hist_rows(ctx, "ggf", S * S, row_words, &b->frows));
+  TRY(ensure(ctx, "gg_fsum",
+             W->parts.size() * L->n_spairs * fq_sum_floats(m) * sizeof(float),
+             (void **)&b->fsum));
+  TRY(ensure(ctx, "gg_ext", sizeof(int), (void **)&b->ext));
+  TRY(ensure(ctx, "gg_atoms", 2 * (size_t)W->staged * sizeof(float4),
+             (void **)&b->atoms));
+  return ensure(ctx, "coef", (size_t)S * S * n_bins * sizeof(float),
+                (void **)&b->coef);
+}
+
+// The parts of a gradient whose rows stay within the workspace limit, and its
+// buffers; *out = nullptr if there is no memory for them (or the limit is
+// below what one atom's takes), which leaves the call to the direct kernels.
+int plan_grad_grid(pyiid_ctx *ctx, Layout *L, int n_bins, GradGridWork **out,
+                   GradBuffers *b) {
+  *out = nullptr;
+  const int m = 2 * grad_transform_for(n_bins)->len;
+  const double row = 2.0 * 3 * grid_words(m / 2) * sizeof(float);
+  int s = 0;  // elements present: rows of an atom
+  std::vector<char> seen(L->n_species, 0);
+  for (const int4 &t : L->tiles) {
+    s += !seen[t.w];
+    seen[t.w] = 1;
+  }
+  // (a warp's share of the columns may split a unit: one row more for each)
+  for (double limit = (double)ctx->workspace_limit;; limit /= 4) {
+    const double atoms =
+        std::floor((limit / row - kSpreadWarps * ctx->n_sms) / s);
+    if (atoms < 1) return PYIID_OK;
+    const int n_parts =
+        (int)std::ceil(L->total / std::min<double>(atoms, L->total));
+    GradGridWork *W;
+    TRY(get_grad_grid_work(ctx, L, n_parts, &W));
+    const int rc = ensure_grad_buffers(ctx, L, W, n_bins, m, b);
+    if (rc == PYIID_OK) *out = W;
+    if (rc != PYIID_ERR_OOM) return rc;
+    cudaGetLastError();
+    release(ctx, "gg_rows");
+    release(ctx, "gg_rows2");
+  }
+}
+
 // grad (and fq, unless nullptr) of one configuration (grad_grid.cuh).
-int run_grad_grid(pyiid_ctx *ctx, Layout *L, const float *positions,
+int run_grad_grid(pyiid_ctx *ctx, const Layout *L, const GradGridWork *W,
+                  const GradBuffers &b, const float *positions,
                   const float *d_ftab, const double *d_na, int n_bins,
                   double qbin, int kbo, float *fq, float *grad) {
   const GradTransformEntry *E = grad_transform_for(n_bins);
-  GradGridWork *W;
-  TRY(get_grad_grid_work(ctx, L, &W));
   PhaseGrid *G;
-  const int m = 2 * E->len, S = L->n_species, n_keys = S * (S + 1) / 2;
+  const int m = 2 * E->len, S = L->n_species, n_keys = L->n_spairs;
   TRY(get_phase_grid(ctx, n_bins, m, true, &G));
-  const int n_ctas = ctx->n_sms, max_warps = kSpreadWarps * n_ctas;
-  const int row_words = grid_words(m / 2);
-  const size_t n_rows = (size_t)W->units + max_warps;
-  void *p;
-  TRY(ensure(ctx, "gg_rows", n_rows * 3 * row_words * sizeof(float), &p));
-  float *rows = static_cast<float *>(p);
-  TRY(ensure(ctx, "gg_rows2", n_rows * 3 * row_words * sizeof(float), &p));
-  float *rows2 = static_cast<float *>(p);
-  TRY(ensure(ctx, "gg_flag", n_rows * sizeof(int), &p));
-  int *flag = static_cast<int *>(p);
-  TRY(ensure(ctx, "gg_parts", W->units * sizeof(int2), &p));
-  int2 *parts = static_cast<int2 *>(p);
-  HistRows frows;
-  TRY(hist_rows(ctx, "ggf", S * S, row_words, &frows));
-  TRY(ensure(ctx, "gg_fsum",
-             (size_t)n_keys * fq_sum_floats(m) * sizeof(float), &p));
-  float *fsum = static_cast<float *>(p);
-  TRY(ensure(ctx, "gg_ext", sizeof(int), &p));
-  int *ext = static_cast<int *>(p);
   const GridScale gs = grid_scale(qbin, m);
-  TRY(ensure(ctx, "gg_atoms", 2 * (size_t)W->staged * sizeof(float4), &p));
-  float4 *atoms = static_cast<float4 *>(p);
-  TRY(ensure(ctx, "coef", (size_t)S * S * n_bins * sizeof(float), &p));
-  float *coef = static_cast<float *>(p);
-  grad_prep_kernel<<<1 + std::min(n_ctas, 1 + std::max(W->staged, S * S * n_bins) /
-                                                  kPrepBlock),
-                     kPrepBlock, 0, ctx->stream>>>(
-      positions, L->d_perm, L->total, W->d_blocks, S, gs.hi, m / 2, ext, d_na,
-      d_ftab, n_bins, coef, atoms);
+  const int n_ctas = ctx->n_sms;
+  grad_prep_kernel<<<
+      1 + std::min(n_ctas, 1 + std::max(W->staged, S * S * n_bins) / kPrepBlock),
+      kPrepBlock, 0, ctx->stream>>>(positions, L->d_perm, L->total, W->d_blocks,
+                                    S, gs.hi, m / 2, b.ext, d_na, d_ftab,
+                                    n_bins, b.coef, b.atoms);
   LAUNCH_CHECK(ctx);
   const float near_r = (float)(kNearPhase / (n_bins * qbin));
   const float near_scale = (float)(n_bins * qbin);
-  (fq ? grad_spread_kernel<true> : grad_spread_kernel<false>)<<<
-      n_ctas, 32 * kSpreadWarps, kSpreadSmem, ctx->stream>>>(
-      atoms, W->d_blocks, W->total, ext, gs, near_r, near_scale, G->d_taps, rows, rows2, flag, parts, frows);
-  LAUNCH_CHECK(ctx);
-  // (one more layer of CTAs sums F's histograms beside the transforms)
-  E->k<<<dim3(L->total, fq ? 4 : 3), E->threads, grad_transform_smem(E->len),
-         ctx->stream>>>(rows, rows2, flag, parts, W->d_blocks, S, ext,
-                        L->d_perm, G->d_tw, G->d_pr, coef, n_bins, kbo,
-                        (float)qbin, 1.0f / (float)n_bins, grad,
-                        FqReduceArgs{frows, W->d_key_cols, n_keys, W->total,
-                                     fsum});
-  LAUNCH_CHECK(ctx);
+  for (size_t i = 0; i < W->parts.size(); ++i) {
+    const GradGridWork::Part &part = W->parts[i];
+    const GradBlock *blocks = W->d_blocks + i * S * S;
+    (fq ? grad_spread_kernel<true> : grad_spread_kernel<false>)<<<
+        n_ctas, 32 * kSpreadWarps, kSpreadSmem, ctx->stream>>>(
+        b.atoms, blocks, part.total, b.ext, gs, near_r, near_scale, G->d_taps,
+        b.rows, b.rows2, b.flag, b.parts, b.frows);
+    LAUNCH_CHECK(ctx);
+    // (one more layer of CTAs sums F's histograms beside the transforms)
+    E->k<<<dim3(part.n, fq ? 4 : 3), E->threads, grad_transform_smem(E->len),
+           ctx->stream>>>(
+        b.rows, b.rows2, b.flag, b.parts, blocks, S, part.a_first, b.ext,
+        L->d_perm, G->d_tw, G->d_pr, b.coef, n_bins, kbo, (float)qbin,
+        1.0f / (float)n_bins, grad,
+        FqReduceArgs{b.frows, W->d_key_cols + i * n_keys, n_keys, part.total,
+                     b.fsum + i * n_keys * fq_sum_floats(m)});
+    LAUNCH_CHECK(ctx);
+  }
   if (!fq) return PYIID_OK;
-  const FqFinish fin{fsum, W->d_cfg_keys, W->d_key_spair, L->d_spair, d_ftab,
+  const FqFinish fin{b.fsum, W->d_cfg_keys, W->d_key_spair, L->d_spair, d_ftab,
                      d_na, G->d_inv_phi, m, n_bins, kbo, qbin, fq, nullptr};
   return launch_fq_finish(ctx, fin, 0, 1, wide_sums(L, 0));
 }
@@ -1779,6 +1870,12 @@ const char *pyiid_last_error(const pyiid_ctx *ctx) {
   return g_err.c_str();
 }
 
+int pyiid_set_workspace_limit(pyiid_ctx *ctx, size_t bytes) {
+  if (!ctx) return fail(nullptr, PYIID_ERR_INVALID_ARG, "null context");
+  ctx->workspace_limit = bytes;
+  return PYIID_OK;
+}
+
 int64_t pyiid_launch_count(const pyiid_ctx *ctx) {
   return ctx ? ctx->launches : -1;
 }
@@ -1825,9 +1922,14 @@ int pyiid_grad_fq(pyiid_ctx *ctx, const float *positions,
   TRY(get_na(ctx, L, scatter, n_bins, &d_na));
   const int kbo = std::min(k_begin, n_bins);
   const int kb0 = kbo & ~1;
-  if (kbo < n_bins && grad_on_grid(L, n_bins, kbo, false))
-    return run_grad_grid(ctx, L, positions, d_ftab, d_na, n_bins, qbin, kbo,
-                         nullptr, grad);
+  if (kbo < n_bins && grad_on_grid(L, n_bins, kbo, false)) {
+    GradGridWork *W;
+    GradBuffers b;
+    TRY(plan_grad_grid(ctx, L, n_bins, &W, &b));
+    if (W)
+      return run_grad_grid(ctx, L, W, b, positions, d_ftab, d_na, n_bins, qbin,
+                           kbo, nullptr, grad);
+  }
   void *p;
   TRY(ensure(ctx, "coef",
              (size_t)n_species * n_species * n_bins * sizeof(float), &p));
@@ -1906,9 +2008,14 @@ int pyiid_fq_grad(pyiid_ctx *ctx, const float *positions,
   const int kbo = std::min(k_begin, n_bins);
   const int kb0 = kbo & ~1;
   const int n_tiles = (int)L->tiles.size();
-  if (kbo < n_bins && grad_on_grid(L, n_bins, kbo, true))
-    return run_grad_grid(ctx, L, positions, d_ftab, d_na, n_bins, qbin, kbo,
-                         fq, grad);
+  if (kbo < n_bins && grad_on_grid(L, n_bins, kbo, true)) {
+    GradGridWork *W;
+    GradBuffers b;
+    TRY(plan_grad_grid(ctx, L, n_bins, &W, &b));
+    if (W)
+      return run_grad_grid(ctx, L, W, b, positions, d_ftab, d_na, n_bins, qbin,
+                           kbo, fq, grad);
+  }
   double *fpart = nullptr;
   int n_split = 1;
   if (n_atoms > 0 && kb0 < n_bins) {
@@ -2250,14 +2357,25 @@ int pyiid_batch_potential_grad(pyiid_ctx *ctx, const float *positions,
   if (!grad || L->total == 0) return PYIID_OK;
   TRY(ensure(ctx, "b_w", (size_t)n_configs * n_bins * sizeof(double), &p));
   double *w = static_cast<double *>(p);
-  const bool on_grid = grid_adjoint(L, n_bins);
+  bool on_grid = grid_adjoint(L, n_bins);
   const int m = kAdjCellsPerBin * n_bins, n_cells = m / 2 + 1;
   const size_t n_keys = (size_t)n_configs * L->n_spairs;
   WkArgs wa{d_na, d_ftab, L->d_spair, L->n_spairs, (float)(2.0 * M_PI / m),
             nullptr};
+  float4 *gtab = nullptr;
   if (on_grid) {
-    TRY(ensure(ctx, "b_wk", n_keys * n_bins * 2 * sizeof(float4), &p));
-    wa.wk = static_cast<float4 *>(p);
+    int rc = ensure(ctx, "b_wk", n_keys * n_bins * 2 * sizeof(float4),
+                    (void **)&wa.wk);
+    if (rc == PYIID_OK)
+      rc = ensure(ctx, "b_gtab", n_keys * n_cells * 2 * sizeof(float4),
+                  (void **)&gtab);
+    if (rc == PYIID_ERR_OOM) {  // the direct kernels need less
+      cudaGetLastError();
+      on_grid = false;
+      wa.wk = nullptr;
+    } else if (rc != PYIID_OK) {
+      return rc;
+    }
   }
   if (n_configs >= 8)
     wvec_kernel<4, 8><<<dim3((n_bins + 3) / 4, (n_configs + 7) / 8), 128, 0,
@@ -2268,8 +2386,6 @@ int pyiid_batch_potential_grad(pyiid_ctx *ctx, const float *positions,
         T->d_T, cvec, n_bins, n_r, kmin, n_configs, w, wa);
   LAUNCH_CHECK(ctx);
   if (on_grid) {
-    TRY(ensure(ctx, "b_gtab", n_keys * n_cells * 2 * sizeof(float4), &p));
-    float4 *gtab = static_cast<float4 *>(p);
     // keys in grid.y: at most 65,535 per launch
     for (size_t key0 = 0; key0 < n_keys; key0 += 32768) {
       const dim3 g((m / 4 + 32) / 32,

@@ -23,12 +23,13 @@
 
 namespace pyiid {
 
-// Units of one (species of a, species of b): unit u is atom a0 + u against
-// the n_b atoms from b0, in cols columns of 32.  Columns of all units are
-// numbered block after block from col0.
-// s_a, s_b: where the species' atoms start in the array of grad_prep_kernel.
+// Units of one (species of a, species of b) in one part of the atoms: unit u is
+// atom a0 + u against the n_b atoms from b0, in cols columns of 32.  Columns
+// of a part's units are numbered block after block from col0.
+// s_a, s_b: where the species' atoms start in the array of grad_prep_kernel;
+// atom a0 is number i_a of the cols_a x 32 there.
 struct GradBlock {
-  int col0, cols, unit0, a0, n_a, b0, n_b, s_a, s_b;
+  int col0, cols, unit0, a0, n_a, b0, n_b, s_a, s_b, i_a, cols_a;
 };
 
 __device__ __forceinline__ SplitAtom staged_atom(const float4 &p,
@@ -325,9 +326,9 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
     const int ce = min(B.cols, cb + (c1 - c));
     const int ia = B.a0 + u;
     // atom a in the order of the columns (see grad_prep_kernel)
-    const int cols_a = (B.n_a + 31) / 32;
+    const int ua = B.i_a + u;
     const float4 *pa =
-        atoms + 2 * (B.s_a + (u % cols_a) * 32 + u / cols_a);
+        atoms + 2 * (B.s_a + (ua % B.cols_a) * 32 + ua / B.cols_a);
     const SplitAtom a = staged_atom(pa[0], pa[1]);
     const size_t row = (size_t)(wi + B.unit0 + u) * 3 * words;
     bool wide = false;
@@ -595,7 +596,8 @@ struct FqReduceArgs {
   float *out;
 };
 
-// Gradient rows: CTA = (atom a in sorted order, coordinate).  X and Y of a
+// Gradient rows: CTA = (atom a of the part, in sorted order from a_first,
+// coordinate).  X and Y of a
 // row are the real and (negated) imaginary part of one real transform of
 // length M = 2 L: of r_j = (y_j + s H_j)/2, r_{M-j} = (y_j - s H_j)/2 with
 // y_j = j H_j, s = kFftScale, done as a complex transform of L points
@@ -615,7 +617,7 @@ __global__ void __launch_bounds__(fft_threads(R0 *R1 *R2),
                           const int *__restrict__ flag,
                           const int2 *__restrict__ parts,
                           const GradBlock *__restrict__ blocks, int n_species,
-                          const int *__restrict__ ext,
+                          int a_first, const int *__restrict__ ext,
                           const int *__restrict__ perm,
                           const float2 *__restrict__ tw,
                           const float2 *__restrict__ pr,
@@ -639,8 +641,8 @@ __global__ void __launch_bounds__(fft_threads(R0 *R1 *R2),
     return;
   }
   const int words = grid_words(ext[0]), last = ext[0] + 4;
-  const int ia = blockIdx.x, comp = blockIdx.y - layers;
-  int sa = 0;  // (a species without atoms starts where the next one does)
+  const int ia = a_first + blockIdx.x, comp = blockIdx.y - layers;
+  int sa = 0;  // (a species without atoms here starts where the next one does)
   while (sa + 1 < n_species && ia >= blocks[(sa + 1) * n_species].a0) ++sa;
   float acc[KT];
 #pragma unroll

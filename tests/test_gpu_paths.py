@@ -269,3 +269,74 @@ def test_grid_fq_close_coincident_and_far_pairs(D, ctx):
     f = f.cpu().numpy()
     assert ran == 0 and np.all(f[[0, 2, 4]] == 0)
     assert rel(f[1, bins], want) <= TOL_F and rel(f[3, bins], want) <= TOL_F
+
+
+# A gradient whose rows exceed the workspace limit runs in parts of its atoms:
+# parts of many and of one or two atoms, parts that begin inside a species and
+# at its edge, a species of the table without atoms, a period of Q shorter than
+# the cluster (the second rows).  F and dF/dx against one part (the sums are
+# cut differently: FP32 roundings) and against the oracle.
+@pytest.mark.parametrize('n,species,nb,qb,at_once', [
+    (300, 1, 500, 0.05, 100), (301, 2, 500, 0.05, 64), (420, 3, 301, 0.05, 17),
+    (48, 1, 500, 0.05, 1), (90, 2, 250, 0.45, 30),
+])
+def test_gradient_in_parts(D, ctx, n, species, nb, qb, at_once):
+    pos, nums = particle(n, n, species)
+    sp, tab, _ = species_tables(nums, qb, nb)
+    if species != 2:  # a species of the table has no atoms
+        sp = np.where(sp > 0, sp + 1, 0).astype(np.int32)
+        tab = np.insert(tab, 1, tab[0], axis=0)
+    kb = 2
+    half = next(x for x in (384, 512, 768, 1024) if 2 * x >= 4.08 * nb)
+    row = 24 * (half + 16)
+    rows = np.array([0, 1, n // 2, n - 1])
+    want_g = rows64(pos, sp, tab, qb, rows)
+    f, g = D.fq_grad(pos, sp, tab, qb, kb)
+    want_f = fq64(pos, sp, tab, qb, np.arange(kb, nb))
+    try:
+        # (rows of the warps besides; half a row against the rounding)
+        ctx.set_workspace_limit(int((16 * 152 + species * at_once + .5) * row))
+        before = ctx.launches
+        ran, (f2, g2) = launched(ctx, 'fq_grad',
+                                 lambda: D.fq_grad(pos, sp, tab, qb, kb))
+        assert ran == 0
+        assert ctx.launches - before == 2 + 2 * -(-n // at_once)
+        ran, g3 = launched(ctx, 'grad_fq',
+                           lambda: D.grad_fq(pos, sp, tab, qb, kb))
+        assert ran == 0
+        ctx.set_workspace_limit(0)
+        ran, (f4, g4) = launched(ctx, 'fq_grad',
+                                 lambda: D.fq_grad(pos, sp, tab, qb, kb))
+        assert ran == 1
+    finally:
+        ctx.set_workspace_limit(2 << 30)
+    for h in (f, f2, f4):
+        h = h.cpu().numpy()
+        assert np.all(h[:kb] == 0) and rel(h[kb:], want_f) <= TOL_F
+    assert rel(f2.cpu().numpy(), f.cpu().numpy()) <= 1e-6
+    for h in (g, g2, g3, g4):
+        h = h.cpu().numpy()
+        assert np.all(h[:, :, :kb] == 0)
+        assert rel(h[rows][:, :, kb:], want_g[:, :, kb:]) <= TOL_G
+    assert rel(g2.cpu().numpy(), g.cpu().numpy()) <= 1e-6
+    assert rel(g3.cpu().numpy(), g.cpu().numpy()) <= 1e-6
+
+
+def test_default_workspace_limit_bounds_a_large_gradient(D, ctx):
+    """7,000 atoms of three elements at 2,007 bins would need 2.3 GB of rows:
+    two parts within 2 GiB, sampled rows and bins against FP64."""
+    import torch
+    n, qb, nb, kb = 7000, 0.015, 2007, 3
+    pos, nums = particle(n, 7, 3)
+    sp, tab, _ = species_tables(nums, qb, nb)
+    before = ctx.launches
+    ran, (f, g) = launched(ctx, 'fq_grad',
+                           lambda: D.fq_grad(pos, sp, tab, qb, kb))
+    assert ran == 0 and ctx.launches - before == 2 + 2 * 2
+    bins = np.arange(kb, nb, 127)
+    assert rel(f.cpu().numpy()[bins], fq64(pos, sp, tab, qb, bins)) <= TOL_F
+    rows = np.array([0, 3499, 3500, n - 1])
+    want = rows64(pos, sp, tab, qb, rows)
+    got = g[torch.as_tensor(rows, device=g.device)].cpu().numpy()
+    for i in range(len(rows)):
+        assert rel(got[i, :, kb:], want[i, :, kb:]) <= TOL_G
