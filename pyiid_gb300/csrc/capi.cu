@@ -209,11 +209,11 @@ struct DevBuf {
   size_t bytes = 0;
 };
 
-// Work of the F(Q) grid path for one layout and range of bins: the rows of
-// columns of the configurations that take it, and what is left to the direct
+// Work of the F(Q) grid path for one layout and set of configurations: the
+// rows of columns of those that take it, and what is left to the direct
 // kernels.
 struct FqGridWork {
-  int n_bins = 0, k_begin = 0;
+  std::vector<unsigned char> on;  // [n_configs]
   int n_segs = 0, total = 0, n_keys = 0, n_cfgs = 0;  // n_cfgs 0: no work
   int n_wide = 0;    // the last of them take the transform in FP64
   int n_direct = 0;  // work items of the other configurations
@@ -277,7 +277,9 @@ struct Layout {
   int *d_item_order = nullptr;
   int *d_key_item_begin = nullptr;
   int2 *d_spair = nullptr;
-  std::vector<std::unique_ptr<FqGridWork>> fq_grid;  // newest first
+  std::vector<std::unique_ptr<FqGridWork>> fq_grid;  // small LRU
+  // which of them a range of bins (n_bins, k_begin) takes, small LRU
+  std::vector<std::pair<std::pair<int, int>, FqGridWork *>> fq_plans;
   std::vector<std::unique_ptr<GradGridWork>> grad_grid;  // by parts
 };
 
@@ -334,7 +336,7 @@ struct pyiid_ctx {
   std::vector<std::unique_ptr<Layout>> layouts;  // small LRU (front = newest)
   std::vector<std::unique_ptr<TMatrix>> tmats;
   std::vector<std::unique_ptr<NaTable>> nas;
-  std::vector<std::unique_ptr<PhaseGrid>> grids;
+  std::vector<std::unique_ptr<PhaseGrid>> grids;    // small LRU
   uint64_t ftab_key = 0;
   int ftab_species = 0, ftab_bins = 0;
   bool attrs_set = false;
@@ -944,9 +946,12 @@ void window_spectrum(const float *taps, int m, int n_bins, double *phi,
 // The grid of m cells for n_bins bins (with_grad: the gradient's tables too).
 int get_phase_grid(pyiid_ctx *ctx, int n_bins, int m, bool with_grad,
                    PhaseGrid **out) {
-  for (auto &G : ctx->grids)
-    if (G->n_bins == n_bins && G->m == m && (G->d_pr != nullptr) == with_grad) {
-      *out = G.get();
+  // 64 of each kind, as the normalisations
+  for (auto it = ctx->grids.begin(); it != ctx->grids.end(); ++it)
+    if ((*it)->n_bins == n_bins && (*it)->m == m &&
+        ((*it)->d_pr != nullptr) == with_grad) {
+      std::rotate(ctx->grids.begin(), it, it + 1);
+      *out = ctx->grids[0].get();
       return PYIID_OK;
     }
   auto G = std::make_unique<PhaseGrid>();
@@ -975,7 +980,7 @@ int get_phase_grid(pyiid_ctx *ctx, int n_bins, int m, bool with_grad,
     TRY(upload(ctx, &G->d_tw, tw));
   }
   ctx->grids.insert(ctx->grids.begin(), std::move(G));
-  while (ctx->grids.size() > 16) {
+  while (ctx->grids.size() > 128) {
     free_phase_grid(ctx->grids.back().get());
     ctx->grids.pop_back();
   }
@@ -1049,29 +1054,19 @@ bool wide_sums(const Layout *L, int c) {
   return pairs > 1e8;
 }
 
-// The grid path's share of a layout (n_cfgs == 0: none of it).
-int get_fq_grid_work(pyiid_ctx *ctx, Layout *L, int n_bins, int k_begin,
-                     FqGridWork **out) {
-  for (auto &W : L->fq_grid)
-    if (W->n_bins == n_bins && W->k_begin == k_begin) {
-      *out = W.get();
-      return PYIID_OK;
-    }
+// Appends the work of the configurations `on` (skip[c]: whether c is one).
+int build_fq_grid_work(pyiid_ctx *ctx, Layout *L, std::vector<int> on,
+                       const std::vector<unsigned char> &skip) {
   auto W = std::make_unique<FqGridWork>();
-  W->n_bins = n_bins;
-  W->k_begin = k_begin;
   std::vector<GridSeg> segs;
   std::vector<int> begin, key_spair, direct;
   std::vector<int4> cfg_keys;
   std::vector<KeyCols> cols;  // columns of each key
-  std::vector<unsigned char> skip(L->n_configs, 0);
   long long total = 0;
-  std::vector<int> on = fq_grid_configs(L, n_bins, k_begin);
   const auto wide = std::stable_partition(
       on.begin(), on.end(), [&](int c) { return !wide_sums(L, c); });
   W->n_wide = (int)(on.end() - wide);
   for (int c : on) {
-    skip[c] = 1;
     const int first_key = (int)key_spair.size();
     const int t0 = L->cfg_tiles[c].x, t1 = L->cfg_tiles[c].y;
     // start of each species' atoms in the sorted order
@@ -1120,12 +1115,45 @@ int get_fq_grid_work(pyiid_ctx *ctx, Layout *L, int n_bins, int k_begin,
     TRY(upload(ctx, &W->d_direct_order, direct));
     TRY(upload(ctx, &W->d_skip, skip));
   }
-  L->fq_grid.insert(L->fq_grid.begin(), std::move(W));
-  while (L->fq_grid.size() > 4) {
-    free_fq_grid(L->fq_grid.back().get());
+  W->on = skip;
+  L->fq_grid.push_back(std::move(W));
+  return PYIID_OK;
+}
+
+// The grid path's share of a layout (n_cfgs == 0: none of it).
+int get_fq_grid_work(pyiid_ctx *ctx, Layout *L, int n_bins, int k_begin,
+                     FqGridWork **out) {
+  // (64 as the normalisations: a captured graph that those outlive keeps its
+  // plans too)
+  const std::pair<int, int> bins(n_bins, k_begin);
+  for (auto it = L->fq_plans.begin(); it != L->fq_plans.end(); ++it)
+    if (it->first == bins) {
+      std::rotate(L->fq_plans.begin(), it, it + 1);
+      *out = L->fq_plans[0].second;
+      return PYIID_OK;
+    }
+  std::vector<int> on = fq_grid_configs(L, n_bins, k_begin);
+  std::vector<unsigned char> skip(L->n_configs, 0);
+  for (int c : on) skip[c] = 1;
+  auto found = std::find_if(L->fq_grid.begin(), L->fq_grid.end(),
+                            [&](auto &W) { return W->on == skip; });
+  if (found == L->fq_grid.end()) {
+    TRY(build_fq_grid_work(ctx, L, on, skip));
+    found = L->fq_grid.end() - 1;
+  }
+  std::rotate(L->fq_grid.begin(), found, found + 1);
+  *out = L->fq_grid[0].get();
+  while (L->fq_grid.size() > 64) {
+    FqGridWork *W = L->fq_grid.back().get();
+    L->fq_plans.erase(
+        std::remove_if(L->fq_plans.begin(), L->fq_plans.end(),
+                       [&](auto &p) { return p.second == W; }),
+        L->fq_plans.end());
+    free_fq_grid(W);
     L->fq_grid.pop_back();
   }
-  *out = L->fq_grid[0].get();
+  L->fq_plans.insert(L->fq_plans.begin(), {bins, *out});
+  if (L->fq_plans.size() > 64) L->fq_plans.pop_back();
   return PYIID_OK;
 }
 

@@ -340,3 +340,44 @@ def test_default_workspace_limit_bounds_a_large_gradient(D, ctx):
     got = g[torch.as_tensor(rows, device=g.device)].cpu().numpy()
     for i in range(len(rows)):
         assert rel(got[i, :, kb:], want[i, :, kb:]) <= TOL_G
+
+
+def test_many_ranges_of_bins_allocate_nothing_once_warm(D, ctx):
+    """A batch of grid and direct configurations and a gradient, each at 20
+    bin counts: warm calls make no allocation (all are captured in one graph),
+    and a replay equals the eager calls."""
+    import torch
+    sizes = [500, 3, 60, 450, 800]
+    parts = [particle(n, 60 + n, 2) for n in sizes]
+    pos = torch.as_tensor(np.concatenate([p for p, _ in parts]), device='cuda')
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    _, sp = np.unique(np.concatenate([z for _, z in parts]),
+                      return_inverse=True)
+    sp = sp.reshape(-1).astype(np.int32)
+    counts = list(range(400, 420))
+    # (a context holds one form-factor table, so all of these are alike)
+    tabs = {nb: np.full((2, nb), 2.0, np.float32) for nb in counts}
+    n1 = sizes[0]
+
+    def calls(out):
+        for nb in counts:
+            f, f1, g1 = out[nb]
+            D.batch_fq(pos, sp, off, tabs[nb], 0.05, nb % 3, out=f)
+            D.fq_grad(pos[:n1], sp[:n1], tabs[nb], 0.05, nb % 3, out_fq=f1,
+                      out_grad=g1)
+
+    def buffers():
+        return {nb: (torch.empty((len(sizes), nb), device='cuda'),
+                     torch.empty(nb, device='cuda'),
+                     torch.empty((n1, 3, nb), device='cuda'))
+                for nb in counts}
+
+    want, got = buffers(), buffers()
+    calls(want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        calls(got)
+    graph.replay()
+    torch.cuda.synchronize()
+    for nb in counts:
+        assert all(torch.equal(a, b) for a, b in zip(want[nb], got[nb])), nb
