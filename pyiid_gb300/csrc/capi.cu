@@ -214,6 +214,7 @@ struct DevBuf {
 // kernels.
 struct FqGridWork {
   std::vector<unsigned char> on;  // [n_configs]
+  void *d_base = nullptr;         // of the arrays below
   int n_segs = 0, total = 0, n_keys = 0, n_cfgs = 0;  // n_cfgs 0: no work
   int n_wide = 0;    // the last of them take the transform in FP64
   int n_direct = 0;  // work items of the other configurations
@@ -234,6 +235,7 @@ struct GradGridWork {
   };
   std::vector<Part> parts;
   int units = 0, staged = 0;       // units of the largest part
+  void *d_base = nullptr;          // of the arrays below
   GradBlock *d_blocks = nullptr;   // [part][n_species][n_species]
   KeyCols *d_key_cols = nullptr;   // [part] columns of each species pair
   int *d_key_spair = nullptr;      // [part][n_spairs]
@@ -287,6 +289,7 @@ struct Layout {
 // polynomials and what its spectrum takes off each bin.
 struct PhaseGrid {
   int n_bins = 0, m = 0;
+  void *d_base = nullptr;       // of the arrays below
   float *d_taps = nullptr;      // [kTaps][kTapCoef]
   double *d_inv_phi = nullptr;  // [n_bins]
   // gradient grids only: (P, R) of each bin, e^{-2 pi i n / m} for n < m
@@ -441,33 +444,31 @@ int upload(pyiid_ctx *ctx, T **dst, const std::vector<T> &src) {
   return PYIID_OK;
 }
 
-void free_fq_grid(FqGridWork *W) {
-  cudaFree(W->d_segs);
-  cudaFree(W->d_seg_begin);
-  cudaFree(W->d_key_cols);
-  cudaFree(W->d_key_spair);
-  cudaFree(W->d_cfg_keys);
-  cudaFree(W->d_direct_order);
-  cudaFree(W->d_skip);
-}
-
-void free_grad_grid(GradGridWork *W) {
-  cudaFree(W->d_blocks);
-  cudaFree(W->d_key_cols);
-  cudaFree(W->d_key_spair);
-  cudaFree(W->d_cfg_keys);
-}
-
-void free_phase_grid(PhaseGrid *G) {
-  cudaFree(G->d_taps);
-  cudaFree(G->d_inv_phi);
-  cudaFree(G->d_pr);
-  cudaFree(G->d_tw);
-}
+// Host arrays that go to the device in one allocation and one copy.
+struct HostPack {
+  std::vector<unsigned char> bytes;
+  std::vector<std::pair<void **, size_t>> parts;
+  template <class T>
+  void add(T **dst, const std::vector<T> &src) {
+    const size_t at = (bytes.size() + 255) & ~(size_t)255;
+    bytes.resize(at + src.size() * sizeof(T));
+    if (!src.empty())
+      std::memcpy(bytes.data() + at, src.data(), src.size() * sizeof(T));
+    parts.push_back({(void **)dst, at});
+  }
+  int upload(pyiid_ctx *ctx, void **base) {
+    bytes.resize(bytes.size() + 1);  // (a part at the end may be empty)
+    CUDA_TRY(ctx, cudaMalloc(base, bytes.size()));
+    CUDA_TRY(ctx, cudaMemcpy(*base, bytes.data(), bytes.size(),
+                             cudaMemcpyHostToDevice));
+    for (auto &p : parts) *p.first = (char *)*base + p.second;
+    return PYIID_OK;
+  }
+};
 
 void free_layout(Layout *L) {
-  for (auto &W : L->fq_grid) free_fq_grid(W.get());
-  for (auto &W : L->grad_grid) free_grad_grid(W.get());
+  for (auto &W : L->fq_grid) cudaFree(W->d_base);
+  for (auto &W : L->grad_grid) cudaFree(W->d_base);
   cudaFree(L->d_perm);
   cudaFree(L->d_tiles);
   cudaFree(L->d_cfg_tiles);
@@ -877,6 +878,7 @@ GridScale grid_scale(double qstep, int m) {
 // out of the bins is smallest, found by scanning beta.
 void window_taps(double sigma, float *taps) {
   const double beta = 0.98 * M_PI * kTaps * (1.0 - 1.0 / (2.0 * sigma));
+  const double peak = std::cyl_bessel_i(0.0, beta);
   constexpr int N = kTapCoef;
   for (int p = 0; p < kTaps; ++p) {
     double y[N], x[N];
@@ -884,7 +886,7 @@ void window_taps(double sigma, float *taps) {
       x[i] = std::cos(M_PI * (i + 0.5) / N) / 2;
       const double d = 2.0 * (p - (kTaps - 1) / 2.0 - x[i]) / kTaps;
       y[i] = std::cyl_bessel_i(0.0, beta * std::sqrt(std::max(0.0, 1 - d * d))) /
-             std::cyl_bessel_i(0.0, beta);
+             peak;
     }
     // Newton's divided differences, then expanded in powers of t
     for (int j = 1; j < N; ++j)
@@ -898,12 +900,18 @@ void window_taps(double sigma, float *taps) {
   }
 }
 
+// (cos, sin) of x turns
+void turn(double x, double *cs) {
+  cs[0] = std::cos(2.0 * M_PI * x);
+  cs[1] = std::sin(2.0 * M_PI * x);
+}
+
 // Spectrum of the window as the kernels evaluate it (the float polynomials,
-// integrated exactly enough by 16 Gauss points per tap): phi_k = integral
+// integrated to 1e-14 by 10 Gauss points per tap): phi_k = integral
 // phi(x) cos(theta_k x) dx, theta_k = 2 pi k / m, and dphi_k = d phi/d theta.
 void window_spectrum(const float *taps, int m, int n_bins, double *phi,
                      double *dphi) {
-  constexpr int G = 16;
+  constexpr int G = 10;
   double gx[G], gw[G];
   for (int i = 0; i < G; ++i) {  // Gauss-Legendre nodes by Newton
     double z = std::cos(M_PI * (i + 0.75) / (G + 0.5)), dp = 0;
@@ -922,7 +930,7 @@ void window_spectrum(const float *taps, int m, int n_bins, double *phi,
     gx[i] = z / 2;
     gw[i] = 1.0 / ((1 - z * z) * dp * dp);
   }
-  std::vector<double> xs, ws;
+  std::vector<double> xs, ws, wx;
   for (int p = 0; p < kTaps; ++p)
     for (int i = 0; i < G; ++i) {
       double f = 0;
@@ -930,16 +938,37 @@ void window_spectrum(const float *taps, int m, int n_bins, double *phi,
         f = f * gx[i] + (double)taps[p * kTapCoef + j];
       xs.push_back(p - (kTaps - 1) / 2.0 - gx[i]);
       ws.push_back(f * gw[i]);
+      wx.push_back(ws.back() * xs.back());
     }
+  // e^{i theta_k x}, one rotation from k to k + 1 and afresh every 64th: the
+  // first call at a bin count waits for this (1,300 bins: 0.15 ms; 1.3 with a
+  // sine and a cosine each time)
+  const int n = (int)xs.size();
+  std::vector<double> c(n), sn(n), cr(n), sr(n);
+  for (int i = 0; i < n; ++i) {
+    double e[2];
+    turn(xs[i] / m, e);
+    cr[i] = e[0];
+    sr[i] = e[1];
+  }
   for (int k = 0; k < n_bins; ++k) {
-    const double th = 2.0 * M_PI * k / m;
+    if (k % 64 == 0)
+      for (int i = 0; i < n; ++i) {
+        double e[2];
+        turn(k * xs[i] / m, e);
+        c[i] = e[0];
+        sn[i] = e[1];
+      }
     double s = 0, d = 0;
-    for (size_t i = 0; i < xs.size(); ++i) {
-      s += ws[i] * std::cos(th * xs[i]);
-      d -= ws[i] * xs[i] * std::sin(th * xs[i]);
+    for (int i = 0; i < n; ++i) {
+      s += ws[i] * c[i];
+      d -= wx[i] * sn[i];
+      const double t = c[i] * cr[i] - sn[i] * sr[i];
+      sn[i] = c[i] * sr[i] + sn[i] * cr[i];
+      c[i] = t;
     }
     phi[k] = s;
-    if (dphi) dphi[k] = d;
+    dphi[k] = d;
   }
 }
 
@@ -968,20 +997,32 @@ int get_phase_grid(pyiid_ctx *ctx, int n_bins, int m, bool with_grad,
                         (float)((1.0 + th * dphi[k] / phi[k]) / phi[k]));
     phi[k] = 1.0 / phi[k];
   }
-  TRY(upload(ctx, &G->d_taps, taps));
-  TRY(upload(ctx, &G->d_inv_phi, phi));
+  HostPack pack;
+  pack.add(&G->d_taps, taps);
+  pack.add(&G->d_inv_phi, phi);
   if (with_grad) {
     std::vector<float2> tw(m);
+    double step[2], c = 1.0, s = 0.0;
+    turn(1.0 / m, step);
     for (int n = 0; n < m; ++n) {
-      const double x = 2.0 * M_PI * n / m;
-      tw[n] = make_float2((float)std::cos(x), (float)-std::sin(x));
+      if (n % 64 == 0) {
+        double e[2];
+        turn((double)n / m, e);
+        c = e[0];
+        s = e[1];
+      }
+      tw[n] = make_float2((float)c, (float)-s);
+      const double t = c * step[0] - s * step[1];
+      s = c * step[1] + s * step[0];
+      c = t;
     }
-    TRY(upload(ctx, &G->d_pr, pr));
-    TRY(upload(ctx, &G->d_tw, tw));
+    pack.add(&G->d_pr, pr);
+    pack.add(&G->d_tw, tw);
   }
+  TRY(pack.upload(ctx, &G->d_base));
   ctx->grids.insert(ctx->grids.begin(), std::move(G));
   while (ctx->grids.size() > 128) {
-    free_phase_grid(ctx->grids.back().get());
+    cudaFree(ctx->grids.back()->d_base);
     ctx->grids.pop_back();
   }
   *out = ctx->grids[0].get();
@@ -1107,13 +1148,15 @@ int build_fq_grid_work(pyiid_ctx *ctx, Layout *L, std::vector<int> on,
     for (int i : L->item_order)
       if (!skip[L->items[i].w / L->n_spairs]) direct.push_back(i);
     W->n_direct = (int)direct.size();
-    TRY(upload(ctx, &W->d_segs, segs));
-    TRY(upload(ctx, &W->d_seg_begin, begin));
-    TRY(upload(ctx, &W->d_key_cols, cols));
-    TRY(upload(ctx, &W->d_key_spair, key_spair));
-    TRY(upload(ctx, &W->d_cfg_keys, cfg_keys));
-    TRY(upload(ctx, &W->d_direct_order, direct));
-    TRY(upload(ctx, &W->d_skip, skip));
+    HostPack pack;
+    pack.add(&W->d_segs, segs);
+    pack.add(&W->d_seg_begin, begin);
+    pack.add(&W->d_key_cols, cols);
+    pack.add(&W->d_key_spair, key_spair);
+    pack.add(&W->d_cfg_keys, cfg_keys);
+    pack.add(&W->d_direct_order, direct);
+    pack.add(&W->d_skip, skip);
+    TRY(pack.upload(ctx, &W->d_base));
   }
   W->on = skip;
   L->fq_grid.push_back(std::move(W));
@@ -1149,7 +1192,7 @@ int get_fq_grid_work(pyiid_ctx *ctx, Layout *L, int n_bins, int k_begin,
         std::remove_if(L->fq_plans.begin(), L->fq_plans.end(),
                        [&](auto &p) { return p.second == W; }),
         L->fq_plans.end());
-    free_fq_grid(W);
+    cudaFree(W->d_base);
     L->fq_grid.pop_back();
   }
   L->fq_plans.insert(L->fq_plans.begin(), {bins, *out});
@@ -1616,11 +1659,13 @@ int get_grad_grid_work(pyiid_ctx *ctx, Layout *L, int n_parts,
     W->parts.push_back(GradGridWork::Part{lo, hi - lo, total});
     W->units = std::max(W->units, units);
   }
-  TRY(upload(ctx, &W->d_blocks, blocks));
-  TRY(upload(ctx, &W->d_key_cols, keys));
-  TRY(upload(ctx, &W->d_key_spair, spair));
-  TRY(upload(ctx, &W->d_cfg_keys,
-             std::vector<int4>{make_int4(0, 0, (int)keys.size(), 0)}));
+  HostPack pack;
+  pack.add(&W->d_blocks, blocks);
+  pack.add(&W->d_key_cols, keys);
+  pack.add(&W->d_key_spair, spair);
+  pack.add(&W->d_cfg_keys,
+           std::vector<int4>{make_int4(0, 0, (int)keys.size(), 0)});
+  TRY(pack.upload(ctx, &W->d_base));
   L->grad_grid.push_back(std::move(W));
   *out = L->grad_grid.back().get();
   return PYIID_OK;
@@ -1862,7 +1907,7 @@ int pyiid_destroy(pyiid_ctx *ctx) {
   for (auto &L : ctx->layouts) free_layout(L.get());
   for (auto &T : ctx->tmats) free_tmatrix(T.get());
   for (auto &N : ctx->nas) cudaFree(N->d_na);
-  for (auto &G : ctx->grids) free_phase_grid(G.get());
+  for (auto &G : ctx->grids) cudaFree(G->d_base);
   cudaFree(ctx->d_status);
   delete ctx;
   return PYIID_OK;
