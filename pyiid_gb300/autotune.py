@@ -82,9 +82,31 @@ def _time(fn, reps):
     return float(np.median(ts))
 
 
+def _fastest(ctx, kern, fn, reps):
+    """Time ``fn()`` under every variant of ``kern`` and select the fastest:
+    (variant, {variant: median ms}, True).  A call that does not run the
+    kernels the variant shapes (F(Q) and gradients on the phase grid, graph
+    replays) is timed once and leaves the selection as it was: (variant,
+    {variant: median ms}, False)."""
+    current = ctx.get_variant(kern)
+    before = ctx.variant_launches(kern)
+    ms = {current: _time(fn, reps)}
+    if ctx.variant_launches(kern) == before:
+        return current, ms, False
+    for idx, _ in variants(kern):
+        if idx != current:
+            ctx.set_variant(kern, idx)
+            ms[idx] = _time(fn, reps)
+    best = min(ms, key=ms.get)
+    ctx.set_variant(kern, best)
+    return best, ms, True
+
+
 def tune(positions, species, scatter, qbin, k_begin=0,
          kernels=('fq', 'grad_fq'), reps=3, save=True):
     """Time all variants of ``kernels`` on this problem, select the fastest.
+    A kernel that the problem does not run (its call takes the phase grid)
+    keeps its variant, and the cache what it holds.
 
     Returns {kernel: {'best': index, 'ms': {index: median ms}}}.
     """
@@ -103,14 +125,13 @@ def tune(positions, species, scatter, qbin, k_begin=0,
         else:
             fn = lambda: debye.grad_fq(pos, species, tab, qbin, k_begin,  # noqa: E731
                                        out=gout)
-        ms = {}
-        for idx, _ in variants(kern):
-            ctx.set_variant(kern, idx)
-            ms[idx] = _time(fn, reps)
-        best = min(ms, key=ms.get)
-        ctx.set_variant(kern, best)
+        best, ms, timed = _fastest(ctx, kern, fn, reps)
         result[kern] = {'best': best, 'ms': ms}
-        cache[_key(kern, n, k - k_begin, tab.shape[0])] = best
+        key = _key(kern, n, k - k_begin, tab.shape[0])
+        if timed:
+            cache[key] = best
+        else:  # (other sizes of the bucket may have been timed)
+            cache.setdefault(key, best)
     if save:
         _save_cache(cache)
     return result
@@ -120,18 +141,14 @@ def tune_call(fn, kernels=('fq', 'adjoint'), reps=3, device=None):
     """Time ``fn()`` (any workload built on the pair kernels, e.g. a batched
     PDFPotential.evaluate or batch_fq call) under every variant of
     ``kernels`` in turn, keeping the fastest of each (the kernels are tuned
-    one after the other, the others at their current variant).
+    one after the other, the others at their current variant).  A kernel that
+    ``fn`` does not run keeps its variant.
 
     Returns {kernel: {'best': index, 'ms': {index: median ms}}}."""
     ctx = context(device)
     result = {}
     for kern in kernels:
-        ms = {}
-        for idx, _ in variants(kern):
-            ctx.set_variant(kern, idx)
-            ms[idx] = _time(fn, reps)
-        best = min(ms, key=ms.get)
-        ctx.set_variant(kern, best)
+        best, ms, _ = _fastest(ctx, kern, fn, reps)
         result[kern] = {'best': best, 'ms': ms}
     return result
 

@@ -61,3 +61,75 @@ def test_unreadable_cache_is_empty(tune):
     with open(tune.cache_path(), 'w') as f:
         f.write('{not json')
     assert tune._load_cache() == {}
+
+
+class CountingCtx:
+    """A context whose calls run the kernels of ``runs`` only."""
+
+    def __init__(self, runs):
+        self.runs, self.var, self.count = runs, {'fq': 5, 'grad_fq': 2}, {}
+        self.set = []
+
+    def get_variant(self, k):
+        return self.var[k]
+
+    def set_variant(self, k, v):
+        self.set.append((k, v))
+        self.var[k] = v
+
+    def variant_launches(self, k):
+        return self.count.get(k, 0)
+
+    def call(self):
+        for k in self.runs:
+            self.count[k] = self.count.get(k, 0) + 1
+
+
+def test_a_kernel_that_does_not_run_keeps_its_variant(tune, monkeypatch):
+    """tune_call times the variants of what the call runs; a kernel that it
+    does not run is neither changed nor chosen by noise."""
+    ctx = CountingCtx({'fq'})
+    monkeypatch.setattr(tune, 'context', lambda device=None: ctx)
+    monkeypatch.setattr(tune, 'variants',
+                        lambda k: [(i, {}) for i in range(8)])
+
+    def timed(fn, reps):
+        fn()
+        return 1.0 if ctx.var['fq'] == 3 else 2.0 - 0.1 * ctx.var['grad_fq']
+    monkeypatch.setattr(tune, '_time', timed)
+    r = tune.tune_call(ctx.call, kernels=('grad_fq', 'fq'))
+    assert r['fq']['best'] == 3 and sorted(r['fq']['ms']) == list(range(8))
+    assert r['grad_fq']['best'] == 2 and list(r['grad_fq']['ms']) == [2]
+    assert ctx.var == {'fq': 3, 'grad_fq': 2}
+    assert all(k == 'fq' for k, _ in ctx.set)
+
+
+def test_tune_saves_what_it_timed(tune, monkeypatch):
+    """Beside a timed choice, a call on the phase grid leaves the cached
+    variant of its bucket as it is, and the current one where there is none."""
+    import numpy as np
+    import torch
+    ctx = CountingCtx({'fq'})
+    monkeypatch.setattr(tune, 'context', lambda device=None: ctx)
+    monkeypatch.setattr(tune, 'variants',
+                        lambda k: [(i, {}) for i in range(8)])
+    monkeypatch.setattr(tune, '_time',
+                        lambda fn, reps: (fn(), 1.0 + (ctx.var['fq'] != 6))[1])
+    for name in ('fq', 'grad_fq'):
+        monkeypatch.setattr(tune.debye, name, lambda *a, **k: ctx.call())
+    monkeypatch.setattr(tune.debye, 'as_positions',
+                        lambda x: torch.as_tensor(x))
+    empty = torch.empty
+    monkeypatch.setattr(tune.torch, 'empty',
+                        lambda *a, **k: empty(1))
+    tab = np.ones((1, 300), np.float32)
+    args = (np.zeros((200, 3), np.float32), np.zeros(200, np.int32), tab, 0.05)
+    key = tune._key('grad_fq', 200, 300, 1)
+    tune.tune(*args, kernels=('fq',))
+    ctx.var['grad_fq'] = 4
+    ctx.runs = set()
+    tune.tune(*args, kernels=('grad_fq',))
+    assert tune._load_cache()[key] == 4
+    ctx.var['grad_fq'] = 1
+    tune.tune(*args, kernels=('grad_fq',))
+    assert tune._load_cache() == {tune._key('fq', 200, 300, 1): 6, key: 4}
