@@ -283,6 +283,8 @@ __global__ void __launch_bounds__(kAdjBlock)
     o[bl * 3 + 1] = jy;
     o[bl * 3 + 2] = jz;
   }
+  // (an atom against itself counts nothing, whatever its place: 0 x NaN)
+  if (ti.y == 1 && it.y == it.x) gx = gy = gz = 0.f;
   sred[warp][lane][0] = gx;
   sred[warp][lane][1] = gy;
   sred[warp][lane][2] = gz;

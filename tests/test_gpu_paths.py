@@ -406,3 +406,29 @@ def test_first_call_at_a_bin_count(D, ctx):
         times.append(time.perf_counter() - t)
         assert ran == 0
     assert np.median(times) <= 0.75e-3, times
+
+
+@pytest.mark.parametrize('bad', [np.nan, np.inf])
+def test_pair_force_of_a_lone_atom_without_a_place(D, ctx, bad):
+    """A one-atom configuration has no pairs: its gradient is 0 wherever it
+    is, and the other configurations' are untouched."""
+    import torch
+    e = O.update_experiment({'rstep': 0.02, 'rmax': 20.0})
+    qb, rg = O.pdf_qbin(e), O.r_grid(e)
+    nb = int(np.floor(e['qmax'] / qb))
+    sizes = [300, 1, 65, 1, 280]
+    pos = np.concatenate([particle(n, n)[0] for n in sizes])
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    sp, tab, _ = species_tables([79] * len(pos), qb, nb)
+    gobs = torch.as_tensor(O.pdf_fft(
+        O.fq(S.fcc_nearest(4.0, 50).astype(np.float32),
+             np.repeat(tab, 50, 0), qb), e['rstep'], qb, rg, e['qmin']))
+    grads = []
+    for x in (0.0, bad):
+        pos[[300, 366], 1] = x
+        ran, out = launched(ctx, 'adjoint', lambda: D.batch_potential_grad(
+            pos, sp, off, tab, qb, e['rstep'], rg, e['qmin'], gobs))
+        assert ran == 0
+        grads.append(out['grad'].cpu().numpy())
+    assert np.all(grads[1][[300, 366]] == 0)
+    assert np.array_equal(grads[0], grads[1])
