@@ -477,21 +477,28 @@ __global__ void __launch_bounds__(32 * kSpreadWarps)
     c = end;
   }
   if (lane == 0) sspill[warp] = spilled;
-  if (finish_rows(out, wi, works ? cur : -1, alone, splan))
-    spill(cur, true);
-  else if (splan[0] >= 0)
+  if (finish_rows(out, wi, works ? cur : -1, alone, splan)) {
+    if (spilled) {
+      spill(cur, true);
+    } else {  // (in line: small batches would wait for the function's code)
+      float *row = out.warp_row(wi + cur);
+      for (int i = lane; i < words; i += 32) row[i] = sum_copies(hist4, i);
+      if (lane == 0) out.flag[wi + cur] = 1;
+    }
+  } else if (splan[0] >= 0)
     for (int i = threadIdx.x; i < words; i += blockDim.x) {
       float s = 0.f, c = 0.f;
       for (int w = 0; w < splan[1]; ++w) {
+        const float x = sum_copies(
+            smem4 + w * (kSpreadStage / 16 + 2 * words) + kSpreadStage / 16, i);
         if (sspill[w]) {
           const int wj = blockIdx.x * plan.per_cta + w;
           pair_add(out.warp_row(wj + splan[0])[i], s, c);
           pair_add(out.low_row(wj)[i], s, c);
+          pair_add(x, s, c);
+        } else {
+          s += x;
         }
-        pair_add(sum_copies(smem4 + w * (kSpreadStage / 16 + 2 * words) +
-                                kSpreadStage / 16,
-                            i),
-                 s, c);
       }
       out.cta_row(blockIdx.x)[i] = s + c;
     }
