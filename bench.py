@@ -470,8 +470,8 @@ def run_gpu_sharded(args, rank, world, local):
 # the pairs): unordered pairs of F(Q) and of the force table (64 x 1,000 atoms),
 # ordered pairs of the gradient (2,001 atoms; counted without F, so low for the
 # pass that sums F beside it)
-GRID_INST_PER_PAIR = {'fq_spread_kernel': 4.95, 'adjoint_grid_kernel': 3.87,
-                      'grad_spread_kernel': 16.4}
+GRID_INST_PER_PAIR = {'fq_spread_kernel': 5.04, 'adjoint_grid_kernel': 3.88,
+                      'grad_spread_kernel': 16.2}
 
 
 def grid_roofline(torch, counted, ms, sm_mhz=2070.0):

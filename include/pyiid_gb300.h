@@ -92,7 +92,9 @@ int64_t pyiid_launch_count(const pyiid_ctx *ctx);
  * fq[k] = 2 * nan_to_num( S_k / na_k ),  k in [k_begin, n_bins)
  *   S_k  = sum_{a>b} f_a(Q_k) f_b(Q_k) sin(Q_k r_ab) / r_ab
  *   na_k = n_atoms * mean_{a>b} f_a(Q_k) f_b(Q_k)
- * Pair sums are accumulated in FP32 (compensated) per tile and reduced in FP64.
+ * Pair sums are accumulated in FP32 (compensated) per tile and reduced in FP64,
+ * or, where that is faster, spread on a grid of phases (FP32 cells, sums in
+ * float pairs, FP64 per bin): the same to about 2e-7 of F.
  *
  * Replaces wrap_fq of cpu_wrappers/flat_multi_cpu_wrap.py:22-60 (same value as
  * cpu_wrappers/flat_serial_cpu_wrap.py:13-69, cpu_wrappers/nxn_cpu_wrap.py:9-69
@@ -107,8 +109,7 @@ int pyiid_fq(pyiid_ctx *ctx, const float *positions, const int32_t *species,
              int n_atoms, const float *scatter, int n_species, int n_bins,
              double qbin, int k_begin, float *fq);
 
-/* F(Q) of many configurations in one pass (one pair-sum launch over the
- * work items of every configuration, then one finishing launch).
+/* F(Q) of many configurations in one pass (the same few launches for all).
  * Configuration b owns atoms offsets[b] .. offsets[b+1]-1 of the packed
  * positions/species; all share one Q grid and one species table.
  *   positions : device float [total_atoms][3]

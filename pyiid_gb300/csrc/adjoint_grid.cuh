@@ -9,7 +9,7 @@
 //   B(u) = sum_k W_k sin(k theta),  theta = dq r = 2 pi u / M,
 // s_ab = (c B'(u) - B(u)/r) / r^2 with c = du/dr: one function of one
 // variable for all pairs of a key.  adjoint_grid_table_kernel tabulates it,
-// adjoint_grid_kernel reads it once per ordered pair.
+// adjoint_grid_kernel reads it once per unordered pair.
 #pragma once
 
 #include "debye_kernels.cuh"

@@ -1307,9 +1307,9 @@ int check_common(pyiid_ctx *ctx, int n_configs, const int32_t *offsets,
   return PYIID_OK;
 }
 
-// Sums the partial histograms of n_keys keys, at most about
-// `most` of each: about four of them per thread row.  Many rows over few cells take
-// CTAs of eight cells, so that there are enough of those.
+// Sums the partial histograms of n_keys keys, at most about `most` of each:
+// about four of them per thread row.  Many rows over few cells take CTAs of
+// eight cells, so that there are enough of those.
 int launch_grid_reduce(pyiid_ctx *ctx, const HistRows &rows,
                        const KeyCols *d_key_cols, const int *ext, int n_cfgs,
                        PlanShape shape, int total, int m, int n_keys,
@@ -1802,7 +1802,7 @@ int run_potential(pyiid_ctx *ctx, const double *gobs, const double *gcalc,
 }
 
 // G(r) rows of n_configs F(Q) rows.  Eight configurations share the reads of
-// T where there are as many and their partial sums fit 48 KB (1,536 bins).
+// T where there are as many and their partial sums fit 32 KB (1,024 bins).
 int run_pdf(pyiid_ctx *ctx, const float *fq, const TMatrix *T, int n_bins,
             int n_r, int n_configs, double *gr) {
   TRY(set_attrs(ctx));

@@ -227,13 +227,13 @@ __device__ __forceinline__ bool finish_rows(const HistRows &out, int wi,
 // the window are polynomials of degree 7 in the pair's position within its
 // cell, evaluated together by packed FMAs (coefficients in registers): 19
 // instructions per eight pairs.  Bound by instruction issue and the latency
-// of its dependent chains (0.60 issued per cycle and scheduler): two columns
+// of its dependent chains (0.59 issued per cycle and scheduler): two columns
 // go side by side, and as many warps run as have room for a histogram, 8 per
-// SM at 650 cells.  158 instructions per 32 pairs; four slots of one tap per
+// SM at 650 cells.  161 instructions per 32 pairs; four slots of one tap per
 // lane, at half the memory per warp, took 248.
-// 64 x 1,000 atoms at 330 bins: 224 us (fq_pair3_kernel 1,451); 256 alloys of
+// 64 x 1,000 atoms at 330 bins: 223 us (fq_pair3_kernel 1,451); 256 alloys of
 // 55 to 2,000 atoms at 500 bins 1.22 ms (11.5); 10,007 atoms at 1,500 bins
-// 0.49 ms (9.5).
+// 0.47 ms (9.5).
 constexpr int kSpreadSlots = 8;
 constexpr int kSpreadCols = 2;
 constexpr PlanShape kFqPlan{4 * kSpreadSlots, 8};
@@ -774,8 +774,12 @@ __global__ void __launch_bounds__(32 * kFqDftWarps, 3)
 // by n cells are common to all blocks of a bin, so what FP32 rounds off them
 // multiplies every 33rd cell's sum, which sees the small-angle peak of F (its
 // height grows with the atoms) at the bins near multiples of M / 33.
+// Above 1e8 pairs, where the direct kernels' error is passed (error of F at
+// 20,000 atoms 2.0e-7 in FP32, 6.3e-8 so, direct 1.5e-7; at 14,000 1.2e-7 in
+// FP32, direct 1.8e-7).
 // One key at a time; warps share the blocks, each centre one rotation by
-// kFqDftWarps blocks from the one before.  FP64 bound.
+// kFqDftWarps blocks from the one before.  FP64 bound: 38 us at 1,500 bins,
+// of 1.4 ms and more.
 __host__ __device__ constexpr int fq_wide_smem(int m) {
   return fq_dft_blocks(m) * (kFqDftReach + 1) * 4 * (int)sizeof(double);
 }

@@ -242,8 +242,9 @@ static __device__ __noinline__ bool grad_spread_rest(
 // the 8 cells x (x, y, z, F) of a pair are 32 consecutive words.  What a warp
 // waits for is the chain read - add - write, so four pairs go together when
 // no two of them are within 8 cells (found for all groups of four by three
-// shuffles), one by one otherwise.  Bound by the shared-memory pipe (83 %
-// busy; 16.4 instructions per ordered pair fill 64 % of the issue slots).
+// shuffles), one by one otherwise.  Bound by the shared-memory pipe (82 %
+// busy; 16.2 instructions per ordered pair fill 64 % of the issue slots, both
+// counted at the 2,001 atoms below).
 // 2,001 atoms, 4.0 M ordered pairs, without F: 90 us; 20,000 atoms with F,
 // 400 M pairs: 9.8 ms (gradfq2_kernel 2,056 us, fqgrad2_kernel 205 ms, whose
 // work grows with the bins too).
